@@ -47,9 +47,6 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
-# nominal FP32 FFMA rate of one B200: 148 SMs x 128 FP32 lanes x 2 flops at
-# the 1965 MHz maximum SM clock (no measured figure exists for the SIMT pipes)
-FP32_SIMT_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 
 
 def peaks():
@@ -573,10 +570,8 @@ def run_recall_extension(dev, steps, warmup, replicates=4096, ticks=200, plain_s
                      "tick_tflops": tflops, "tick_frac": tflops / pk["bf16_tflops"]},
         "fp32_engine": {"value": value32, "unit": "replicate-ticks/s", "ms_per_step": ms32,
                         "us_per_tick": ms32 * 1e3 / T, "tflops": tflops32, "gpu_launches_per_step": launches32,
-                        "contraction_us_per_launch": k_ms32 * 1e3, "contraction_tflops": k_tflops32,
-                        "kernel": "recall_fp32_kernel (SIMT FFMA, W in fp32)",
-                        "fp32_simt_peak_tflops": FP32_SIMT_PEAK_TFLOPS,
-                        "frac_of_fp32_simt_peak": k_tflops32 / FP32_SIMT_PEAK_TFLOPS},
+                        "contraction_us_per_launch": k_ms32 * 1e3, "contraction_dense_equivalent_tflops": k_tflops32,
+                        "kernel": "recall_events_kernel (FP32 additions of the spiking sources' weights)"},
         "speedup_bf16_vs_fp32_engine": value / value32,
         "plain_fp32": {"value": plain_rate, "unit": "replicate-ticks/s", "replicates_timed": plain_sample,
                        "ms_per_replicate": statistics.mean(plain_ms),

@@ -20,11 +20,11 @@
  *   warps 2..5  epilogue, one replicate row per thread (TMEM lane = row):
  *               tcgen05.ld of the accumulator and the epsc update.
  *
- * FP32 (recall_fp32_kernel): the same contraction on the FP32 pipes with W
- * kept in FP32 -- a register-tiled SIMT product (CTA tile 128 x 128, 8 x 8
- * outputs per thread, K stages of 16 double-buffered in shared memory) with
- * the same epilogue expression.  It exists to measure the tensor-core form
- * against the same engine at full precision.
+ * FP32: W kept in FP32, the spikes as bits.  recall_events_kernel adds the
+ * weights of the sources that spiked, in ascending order; where most sources
+ * can spike, or a weight is not finite, recall_fp32_kernel multiplies densely
+ * (CTA tile 128 x 128, 8 x 8 outputs per thread, K stages of 16
+ * double-buffered in shared memory), to the same bits.
  *
  * Every mbarrier wait is bounded (1 s of %globaltimer); a wait that runs out
  * sets an error bit and the CTA leaves its loops, waits (bounded) for its own
@@ -61,7 +61,8 @@ struct Params {
   float* dsup_cur;
   const float* epsc_prev;
   float* epsc_cur;
-  uint16_t* s_out; /* BF16 [R][N] spikes of this tick */
+  uint16_t* s_out; /* BF16 [R][N] spikes of this tick (BF16 contraction) */
+  uint32_t* s_bits; /* the same as bits [R][N/32] (FP32 contraction) */
   uint8_t* counts; /* [R][N] */
   int count_on;
   const float* bj;
@@ -198,7 +199,7 @@ __device__ __forceinline__ float dsup_mcu0(const Params& p, int row, uint32_t se
    lane to lane; one Philox call per four MCUs and stream.  Its own kernel,
    run beside the contraction on a second stream: a CTA of the contraction
    leaves room on its SM for three of its CTAs. */
-template <int M>
+template <int M, bool kBits>
 __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
   constexpr int Q = M / 4;
   const int lane = threadIdx.x & 31;
@@ -214,7 +215,8 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
     const bool bad = r >= p.R || row + c0 + Q > n || ((row + c0) & 3) != 0 || (c0 + Q) > p.N ||
                      (reinterpret_cast<uintptr_t>(p.dsup_prev) & 15) || (reinterpret_cast<uintptr_t>(p.dsup_cur) & 15) ||
                      (reinterpret_cast<uintptr_t>(p.epsc_prev) & 15) || (reinterpret_cast<uintptr_t>(p.bj) & 15) ||
-                     (reinterpret_cast<uintptr_t>(p.s_out) & 15) || (reinterpret_cast<uintptr_t>(p.counts) & 15);
+                     (kBits ? reinterpret_cast<uintptr_t>(p.s_bits) & 15 : reinterpret_cast<uintptr_t>(p.s_out) & 15) ||
+                     (reinterpret_cast<uintptr_t>(p.counts) & 15);
     /* the warp leaves together: the shuffles below take all 32 lanes */
     if (__any_sync(0xffffffffu, bad)) {
       if (bad && atomicOr(p.err, kErrAlign) == 0) p.err[1] = tid;
@@ -287,14 +289,28 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
 #pragma unroll
   for (int m = 0; m < Q; m += 4)
     *reinterpret_cast<float4*>(p.dsup_cur + row + c0 + m) = make_float4(d[m], d[m + 1], d[m + 2], d[m + 3]);
-  /* BF16 1.0 = 0x3F80; four MCUs per 8-byte store (Q is a multiple of 4) */
+  if (kBits) {
+    /* row + c0 is a multiple of Q, so a quarter's bits are whole bytes, or
+       half a byte at Q = 4, where two lanes share one */
+    uint8_t* o = reinterpret_cast<uint8_t*>(p.s_bits) + ((row + c0) >> 3);
+    if (Q == 16) {
+      *reinterpret_cast<uint16_t*>(o) = (uint16_t)bits;
+    } else if (Q == 8) {
+      *o = (uint8_t)bits;
+    } else {
+      const uint32_t hi = __shfl_down_sync(0xffffffffu, bits, 1);
+      if ((q & 1) == 0) *o = (uint8_t)(bits | (hi << 4));
+    }
+  } else {
+    /* BF16 1.0 = 0x3F80; four MCUs per 8-byte store (Q is a multiple of 4) */
 #pragma unroll
-  for (int m = 0; m < Q; m += 4) {
-    uint32_t w[2];
+    for (int m = 0; m < Q; m += 4) {
+      uint32_t w[2];
 #pragma unroll
-    for (int k = 0; k < 2; k++)
-      w[k] = (((bits >> (m + 2 * k)) & 1u) ? 0x3F80u : 0u) | ((((bits >> (m + 2 * k + 1)) & 1u) ? 0x3F80u : 0u) << 16);
-    *reinterpret_cast<uint2*>(p.s_out + row + c0 + m) = make_uint2(w[0], w[1]);
+      for (int k = 0; k < 2; k++)
+        w[k] = (((bits >> (m + 2 * k)) & 1u) ? 0x3F80u : 0u) | ((((bits >> (m + 2 * k + 1)) & 1u) ? 0x3F80u : 0u) << 16);
+      *reinterpret_cast<uint2*>(p.s_out + row + c0 + m) = make_uint2(w[0], w[1]);
+    }
   }
   if (p.count_on) {
 #pragma unroll
@@ -469,8 +485,9 @@ constexpr int kF32BM = 128, kF32BN = 128, kF32BK = 16, kF32Threads = 256;
 
 /* FP32 SIMT contraction with the epsc epilogue of recall_tick_kernel:
    epsc(t)[r][j] = epsc(t-1)[r][j] * (1 - kepsc) + sum_i S(t-3)[r][i] * W[i][j]
-   with W in FP32 ([source i][destination j], row-major) and S the BF16 0/1
-   spike ring (its value is exact: the bits shifted into an FP32 word).
+   with W in FP32 ([source i][destination j], row-major) and S the 0/1 spike
+   bits.  The dense form: it multiplies every weight, so it is taken only where
+   recall_events_kernel is not (see bcpnn_recall_run).
 
    One CTA per 128 x 128 output tile (blockIdx.x = M-tile * (N/128) + N-tile);
    thread (ty, tx) = (tid / 16, tid % 16) owns rows {ty*4 .. +3, 64 + ty*4 ..
@@ -479,7 +496,7 @@ constexpr int kF32BM = 128, kF32BN = 128, kF32BK = 16, kF32Threads = 256;
    memory, two buffers, the next stage's global loads held in registers while
    the current one is multiplied, one barrier per stage. */
 __global__ void __launch_bounds__(kF32Threads, 2)
-    recall_fp32_kernel(const uint16_t* __restrict__ s, const float* __restrict__ w, Params p) {
+    recall_fp32_kernel(const uint32_t* __restrict__ s, const float* __restrict__ w, Params p) {
   __shared__ __align__(16) float As[2][kF32BK][kF32BM];
   __shared__ __align__(16) float Bs[2][kF32BK][kF32BN];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -497,14 +514,14 @@ __global__ void __launch_bounds__(kF32Threads, 2)
       return;
     }
   }
-  /* S stage: row a_row, eight BF16 at a_k (one 16-byte load); W stage: row
-     b_k, eight floats at b_n (two 16-byte loads) */
+  /* S stage: row a_row, eight spike bits at a_k (one byte); W stage: row b_k,
+     eight floats at b_n (two 16-byte loads) */
   const int a_row = tid & 127, a_k = (tid >> 7) * 8;
   const int b_k = tid >> 4, b_n = (tid & 15) * 8;
-  const uint16_t* ag = s + (size_t)(m0 + a_row) * p.N + a_k;
+  const uint8_t* ag = reinterpret_cast<const uint8_t*>(s) + ((size_t)(m0 + a_row) * p.N + a_k) / 8;
   const float* bg = w + (size_t)b_k * p.N + n0 + b_n;
   const size_t b_step = (size_t)kF32BK * p.N;
-  uint4 ra = __ldg(reinterpret_cast<const uint4*>(ag));
+  uint32_t ra = __ldg(ag);
   float4 rb0 = __ldg(reinterpret_cast<const float4*>(bg));
   float4 rb1 = __ldg(reinterpret_cast<const float4*>(bg + 4));
   float acc[8][8];
@@ -514,12 +531,8 @@ __global__ void __launch_bounds__(kF32Threads, 2)
     for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
 
   auto stage = [&](int buf) {
-    const uint32_t u[4] = {ra.x, ra.y, ra.z, ra.w};
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      As[buf][a_k + 2 * j][a_row] = __uint_as_float(u[j] << 16);
-      As[buf][a_k + 2 * j + 1][a_row] = __uint_as_float(u[j] & 0xFFFF0000u);
-    }
+    for (int j = 0; j < 8; j++) As[buf][a_k + j][a_row] = (ra >> j) & 1u ? 1.0f : 0.0f;
     *reinterpret_cast<float4*>(&Bs[buf][b_k][b_n]) = rb0;
     *reinterpret_cast<float4*>(&Bs[buf][b_k][b_n + 4]) = rb1;
   };
@@ -529,7 +542,7 @@ __global__ void __launch_bounds__(kF32Threads, 2)
   for (int kt = 0; kt < kTiles; kt++) {
     const int buf = kt & 1;
     if (kt + 1 < kTiles) {
-      ra = __ldg(reinterpret_cast<const uint4*>(ag + (size_t)(kt + 1) * kF32BK));
+      ra = __ldg(ag + (size_t)(kt + 1) * (kF32BK / 8));
       const float* b = bg + (size_t)(kt + 1) * b_step;
       rb0 = __ldg(reinterpret_cast<const float4*>(b));
       rb1 = __ldg(reinterpret_cast<const float4*>(b + 4));
@@ -569,6 +582,368 @@ __global__ void __launch_bounds__(kF32Threads, 2)
   }
 }
 
+/* ---- FP32 contraction by events ------------------------------------------
+
+   Each output adds the rows of W of the sources that spiked, in ascending
+   source order from 0:
+     epsc(t)[r][j] = epsc(t-1)[r][j] * (1 - kepsc) + (((W[i0][j] + W[i1][j]) + W[i2][j]) + ...)
+   The multiply-adds of recall_fp32_kernel do the same additions in the same
+   order, and fma(0, w, acc) = acc for a finite w, so both give the same bits;
+   at the 1 spike in 50 sources of a recall the dense form does 50 times the
+   work.
+
+   Bound by the shared-memory reads of W: 4 bytes per spike and destination
+   (128 bytes per SM and cycle).  A CTA (one per SM) takes a run of (column
+   tile of 64, replicate) pairs, the same number in every CTA; 15 warps hold
+   up to 24 replicates each, two columns per lane, in registers (48
+   accumulators a lane), so a chunk of W serves 360 replicates once it is in
+   shared memory.  W comes in chunks of 384 sources x 64 columns (TMA, two
+   buffers, issued by a warp of its own); a warp reads a row of a chunk as 256
+   contiguous bytes, without bank conflicts, for any spike pattern.  The
+   spikes of a replicate and chunk come as a list of 16-bit source numbers
+   (recall_lists_kernel), padded to a multiple of four with the number of a
+   row of zeros (the sum is never -0, so adding +0 leaves it as it is), read
+   four at a time with all lanes on the same replicate.  The replicates are
+   walked in groups of eight whose accumulators rotate through the registers:
+   one unrolled body for all 24 replicates is more code than the instruction
+   caches hold.  A replicate with more than kEvCap spikes in a chunk is listed
+   from its bits by the warp that needs it (walk_bits).
+
+   At N = R = 4096, M = 64 and 20 Hz noise (2.2 % of the sources spike): 345 us
+   a launch, 2815 us dense.  8.2 us are added per 0.1 % of density, of which
+   the weights' reads are 8.0 at 128 bytes per SM and cycle; 184 us remain
+   without spikes: per replicate and chunk the count, the loop and the padding,
+   per pass the epilogue.  W's chunks alone would take 88 us and come in
+   beside.  24 replicates in 15 warps were the best of 8 x 31, 16 x 19, 16 x
+   23, 24 x 15 and 32 x 15; eight list entries per step were slower than four
+   (435 us). */
+constexpr int kEvCols = 64, kEvRows = 384, kEvBox = 192, kEvWarps = 15, kEvThreads = (kEvWarps + 1) * 32;
+constexpr int kEvReps = 24;          /* replicates per warp and pass */
+constexpr int kEvGroup = 8;          /* replicates of one unrolled body */
+constexpr int kEvCap = 32;           /* listed spikes per replicate and chunk */
+constexpr int kEvListWords = kEvCap / 2;
+/* the expected share of sources spiking above which the dense kernel is the
+   faster one: 2777 us by events at 0.2 (2815 us dense), 3169 us at 0.24 */
+constexpr float kEvMaxDensity = 0.2f;
+constexpr int kEvWords = kEvRows / 32;
+constexpr uint32_t kEvRowBytes = kEvCols * 4;
+constexpr uint32_t kEvChunkBytes = kEvRows * kEvRowBytes;
+constexpr uint32_t kEvBufBytes = kEvChunkBytes + kEvRowBytes; /* and the row of zeros */
+constexpr uint32_t kEvScratch = (kEvRows + 8) * 2; /* a warp's list of one replicate (walk_bits) */
+/* the warps' lists, their scratch lists, their counts */
+constexpr uint32_t kEvListBytes = kEvWarps * (kEvReps * (kEvListWords * 4 + 1) + kEvScratch);
+constexpr size_t kEvSmemBytes = 2 * kEvBufBytes + kEvListBytes + 4 * sizeof(uint64_t);
+static_assert(kEvReps % kEvGroup == 0 && kEvGroup == 8, "a group's counts are one 8-byte read");
+static_assert(kEvReps * kEvListWords % 128 == 0, "a warp's lists are whole 16-byte words per lane");
+static_assert(kEvScratch % 8 == 0 && kEvListBytes % 8 == 0 && kEvBufBytes % 128 == 0, "shared memory alignment");
+static_assert(kEvWords % 4 == 0 && kEvWords <= 16, "walk_bits gives a word to each of at most 16 lanes");
+static_assert(kEvSmemBytes <= 232448, "shared memory of one CTA");
+
+/* byte offset, in a chunk of 256-byte rows, of the lane's columns of the row
+   of a 16-bit list entry; lane8 = 8 * lane is the low byte */
+__device__ __forceinline__ uint32_t ev_row0(uint32_t two, uint32_t lane8) { return __byte_perm(two, lane8, 0x7104); }
+__device__ __forceinline__ uint32_t ev_row1(uint32_t two, uint32_t lane8) { return __byte_perm(two, lane8, 0x7324); }
+
+/* two IEEE additions in one instruction, as a 64-bit register pair */
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long c;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
+}
+
+__device__ __forceinline__ unsigned long long lds64(uint32_t a) {
+  unsigned long long v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+  return v;
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+
+/* the spike lists of one tick, [chunk][replicate][kEvCap], and their counts,
+   [chunk][replicate]: one thread per list; the sources of the chunk that
+   spiked, ascending, padded with row kEvRows (count: kEvCap + 1 if more) */
+__global__ void __launch_bounds__(256) recall_lists_kernel(const uint32_t* __restrict__ bits, uint4* __restrict__ lists,
+                                                           uint8_t* __restrict__ counts, int R, int N) {
+  __shared__ uint16_t buf[256][kEvCap + 2]; /* 17 words a row: no bank conflicts */
+  const int W32 = N / 32;
+  const long long n = (long long)R * ((N + kEvRows - 1) / kEvRows);
+  const long long x = (long long)blockIdx.x * 256 + threadIdx.x;
+  uint16_t* mine = buf[threadIdx.x];
+  if (x < n) {
+    const int c = (int)(x / R), r = (int)(x - (long long)c * R);
+    const uint32_t* b = bits + (size_t)r * W32 + c * kEvWords;
+    const int nw = min(kEvWords, W32 - c * kEvWords);
+    int cnt = 0;
+    for (int v = 0; v < nw; v++) {
+      uint32_t w = __ldg(b + v);
+      while (w) {
+        const int k = __ffs(w) - 1;
+        w &= w - 1;
+        if (cnt < kEvCap) mine[cnt] = (uint16_t)(v * 32 + k);
+        cnt++;
+      }
+    }
+    for (int k = cnt; k < kEvCap; k++) mine[k] = (uint16_t)kEvRows;
+    counts[x] = (uint8_t)(cnt <= kEvCap ? cnt : kEvCap + 1);
+  }
+  __syncthreads();
+  /* the block's lists are contiguous */
+  uint32_t* out = reinterpret_cast<uint32_t*>(lists) + (size_t)blockIdx.x * 256 * kEvListWords;
+  const long long left = n - (long long)blockIdx.x * 256;
+  const int words = (int)(left < 256 ? left : 256) * kEvListWords;
+  for (int k = threadIdx.x; k < words; k += 256)
+    out[k] = reinterpret_cast<const uint32_t*>(buf[k / kEvListWords])[k % kEvListWords];
+}
+
+/* a replicate with more than kEvCap spikes in a chunk: its nw words of bits
+   (global memory) listed in the warp's scratch (kEvRows + 4 entries at byte
+   address l), padded to a multiple of four with row kEvRows, and their rows
+   added to acc as from a list of its own */
+__device__ __noinline__ unsigned long long walk_bits(unsigned long long acc, const uint32_t* words, int nw, uint32_t l,
+                                                     uint32_t w0, uint32_t lane8) {
+  const int lane = (int)lane8 >> 3;
+  uint32_t w = lane < nw ? __ldg(words + lane) : 0u;
+  int at = __popc(w);
+  const int own = at;
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += y;
+  }
+  const int n = __shfl_sync(0xffffffffu, at, 15); /* kEvWords <= 16 lanes hold words */
+  uint32_t d = l + 2 * (uint32_t)(at - own);
+  while (w) {
+    const int b = __ffs(w) - 1;
+    w &= w - 1;
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(d), "h"((unsigned short)(lane * 32 + b)) : "memory");
+    d += 2;
+  }
+  if (lane < 4)
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(l + 2 * (uint32_t)(n + lane)), "h"((unsigned short)kEvRows) : "memory");
+  __syncwarp();
+#pragma unroll 1
+  for (const uint32_t end = l + 2 * (uint32_t)n; l < end; l += 8) {
+    const unsigned long long x = lds64(l);
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
+    const unsigned long long v0 = lds64(w0 + ev_row0(x0, lane8)), v1 = lds64(w0 + ev_row1(x0, lane8));
+    const unsigned long long v2 = lds64(w0 + ev_row0(x1, lane8)), v3 = lds64(w0 + ev_row1(x1, lane8));
+    acc = add2(add2(add2(add2(acc, v0), v1), v2), v3);
+  }
+  __syncwarp();
+  return acc;
+}
+
+/* the passes of one CTA: (column tile, replicates [a, e)) for its run of pairs */
+struct EvPass {
+  long long pair, end;
+  int R, tile, a, e, seg_r0, seg_len, npass, k;
+  __device__ __forceinline__ void init(long long p0, long long p1, int R_) {
+    pair = p0;
+    end = p1;
+    R = R_;
+    npass = k = 0;
+  }
+  __device__ __forceinline__ bool next() {
+    if (k == npass) {
+      if (pair >= end) return false;
+      tile = (int)(pair / R);
+      seg_r0 = (int)(pair - (long long)tile * R);
+      const long long left = end - pair;
+      seg_len = left < R - seg_r0 ? (int)left : R - seg_r0;
+      npass = (seg_len + kEvWarps * kEvReps - 1) / (kEvWarps * kEvReps);
+      pair += seg_len;
+      k = 0;
+    }
+    a = seg_r0 + (int)((long long)seg_len * k / npass);
+    e = seg_r0 + (int)((long long)seg_len * (k + 1) / npass);
+    k++;
+    return true;
+  }
+};
+
+__global__ void __launch_bounds__(kEvThreads, 1)
+    recall_events_kernel(const __grid_constant__ CUtensorMap map_w, const uint32_t* __restrict__ bits,
+                         const uint4* __restrict__ lists, const uint8_t* __restrict__ counts, Params p) {
+  extern __shared__ __align__(128) uint8_t ev_smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(ev_smem + 2 * kEvBufBytes + kEvListBytes);
+  uint64_t* empty = full + 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int N = p.N, W32 = N / 32, n_chunks = (N + kEvRows - 1) / kEvRows;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], kEvWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 2 * kEvCols)
+    reinterpret_cast<float*>(ev_smem + (threadIdx.x / kEvCols) * kEvBufBytes + kEvChunkBytes)[threadIdx.x % kEvCols] = 0.0f;
+  __syncthreads();
+  /* self-check: whole column tiles, alignment of the ring and of every vector access */
+  const bool ok0 = N % kEvCols == 0 && W32 % 4 == 0 && (smem_u32(ev_smem) & 127u) == 0 &&
+                   (reinterpret_cast<uintptr_t>(lists) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.epsc_prev) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(p.epsc_cur) & 15) == 0;
+  if (!ok0) {
+    if (threadIdx.x == 0 && atomicOr(p.err, kErrAlign) == 0) p.err[1] = -1 - (int)blockIdx.x;
+    return;
+  }
+  const long long T = (long long)(N / kEvCols) * p.R;
+  EvPass ps;
+  ps.init(T * blockIdx.x / gridDim.x, T * (blockIdx.x + 1) / gridDim.x, p.R);
+  uint32_t it = 0; /* chunks so far: buffer it & 1, phase (it >> 1) & 1 */
+
+  if (warp == kEvWarps) {
+    if (lane == 0) {
+      bool ok = true;
+      while (ok && ps.next()) {
+        for (int c = 0; c < n_chunks; c++, it++) {
+          const uint32_t s = it & 1;
+          if (!mbar_wait(&empty[s], ((it >> 1) & 1) ^ 1, p.err)) {
+            ok = false;
+            break;
+          }
+          uint8_t* dst = ev_smem + s * kEvBufBytes;
+          const int row = c * kEvRows;
+          const bool two = row + kEvBox < N; /* no box starts past the last row */
+          mbar_expect_tx(&full[s], two ? kEvChunkBytes : kEvChunkBytes / 2);
+          tma_load_2d(dst, &map_w, &full[s], ps.tile * kEvCols, row);
+          if (two) tma_load_2d(dst + kEvBox * kEvRowBytes, &map_w, &full[s], ps.tile * kEvCols, row + kEvBox);
+        }
+      }
+      /* leave no copy in flight */
+      for (uint32_t j = (it > 2 ? it - 2 : 0); j < it; j++) {
+        const unsigned long long t0 = gtimer();
+        while (!mbar_try_wait(&full[j & 1], (j >> 1) & 1) && gtimer() - t0 < kWaitNs) {
+        }
+      }
+    }
+    return;
+  }
+
+  uint8_t* const my_lists = ev_smem + 2 * kEvBufBytes + warp * (kEvReps * kEvListWords * 4);
+  uint8_t* const my_scratch = ev_smem + 2 * kEvBufBytes + kEvWarps * kEvReps * kEvListWords * 4 + warp * kEvScratch;
+  uint8_t* const my_counts =
+      ev_smem + 2 * kEvBufBytes + kEvWarps * (kEvReps * kEvListWords * 4 + kEvScratch) + warp * kEvReps;
+  const uint32_t scratch_a = smem_u32(my_scratch);
+  const uint32_t lists_a = smem_u32(my_lists), counts_a = smem_u32(my_counts), lane8 = (uint32_t)lane * 8;
+  while (ps.next()) {
+    const int q = (ps.e - ps.a + kEvWarps - 1) / kEvWarps;
+    const int r0 = ps.a + warp * q;
+    const int nr = max(0, min(q, ps.e - r0)); /* this warp's replicates */
+    unsigned long long acc[kEvReps]; /* two columns each */
+#pragma unroll
+    for (int i = 0; i < kEvReps; i++) acc[i] = 0ull;
+    /* the warp's lists of a chunk, contiguous: a few 16-byte words per lane, one chunk ahead */
+    constexpr int kListLoads = kEvReps * (kEvListWords / 4) / 32;
+    uint4 b[kListLoads];
+    uint8_t bc = 0; /* lists of no replicate: count 0 */
+    auto fetch = [&](int c) {
+      const uint4* src = lists + ((size_t)c * p.R + r0) * (kEvListWords / 4);
+#pragma unroll
+      for (int v = 0; v < kListLoads; v++)
+        if (lane + 32 * v < nr * (kEvListWords / 4)) b[v] = __ldg(src + lane + 32 * v);
+      if (lane < nr) bc = __ldg(counts + (size_t)c * p.R + r0 + lane);
+    };
+    fetch(0);
+    for (int c = 0; c < n_chunks; c++, it++) {
+#pragma unroll
+      for (int v = 0; v < kListLoads; v++)
+        if (lane + 32 * v < nr * (kEvListWords / 4)) *reinterpret_cast<uint4*>(my_lists + (lane + 32 * v) * 16) = b[v];
+      if (lane < kEvReps) my_counts[lane] = bc;
+      __syncwarp();
+      if (c + 1 < n_chunks) fetch(c + 1);
+      const uint32_t s = it & 1;
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (it >> 1) & 1, p.err) ? 1 : 0) != 0;
+      if (!ok) return;
+      const uint32_t w0 = smem_u32(ev_smem) + s * kEvBufBytes;
+      uint32_t l = lists_a;
+      /* groups of replicates: after each, the accumulators rotate by one group */
+#pragma unroll 1
+      for (int g = 0; g < kEvReps; g += kEvGroup) {
+        const unsigned long long cnts = lds64(counts_a + g);
+        unsigned long long xn = lds64(l);
+#pragma unroll
+        for (int i = 0; i < kEvGroup; i++, l += kEvListWords * 4) {
+          const uint32_t cnt = (uint32_t)(cnts >> (8 * i)) & 0xffu;
+          unsigned long long x = xn;
+          if (i + 1 < kEvGroup) xn = lds64(l + kEvListWords * 4);
+          if (cnt <= kEvCap) {
+            unsigned long long a = acc[i];
+            const uint32_t end = l + 2 * cnt;
+            uint32_t e = l;
+#pragma unroll 1
+            while (e < end) {
+              const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
+              const unsigned long long v0 = lds64(w0 + ev_row0(x0, lane8)), v1 = lds64(w0 + ev_row1(x0, lane8));
+              const unsigned long long v2 = lds64(w0 + ev_row0(x1, lane8)), v3 = lds64(w0 + ev_row1(x1, lane8));
+              e += 8;
+              x = lds64(e);
+              a = add2(add2(add2(add2(a, v0), v1), v2), v3);
+            }
+            acc[i] = a;
+          } else {
+            const int w = c * kEvWords;
+            acc[i] = walk_bits(acc[i], bits + (size_t)(r0 + g + i) * W32 + w, min(kEvWords, W32 - w), scratch_a, w0,
+                               lane8);
+          }
+        }
+        unsigned long long t[kEvGroup];
+#pragma unroll
+        for (int i = 0; i < kEvGroup; i++) t[i] = acc[i];
+#pragma unroll
+        for (int i = 0; i < kEvReps - kEvGroup; i++) acc[i] = acc[i + kEvGroup];
+#pragma unroll
+        for (int i = 0; i < kEvGroup; i++) acc[kEvReps - kEvGroup + i] = t[i];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
+    /* epilogue: 256 contiguous bytes per replicate row and warp, four rows' loads at a time */
+    const size_t col = (size_t)ps.tile * kEvCols + 2 * lane;
+#pragma unroll
+    for (int i0 = 0; i0 < kEvReps; i0 += 4) {
+      if (i0 >= nr) break;
+      float2 ev[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (i0 + i < nr) ev[i] = *reinterpret_cast<const float2*>(p.epsc_prev + (size_t)(r0 + i0 + i) * N + col);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (i0 + i < nr) {
+          float2 o;
+          o.x = ev[i].x * p.one_m_kepsc + __uint_as_float((uint32_t)acc[i0 + i]);
+          o.y = ev[i].y * p.one_m_kepsc + __uint_as_float((uint32_t)(acc[i0 + i] >> 32));
+          *reinterpret_cast<float2*>(p.epsc_cur + (size_t)(r0 + i0 + i) * N + col) = o;
+        }
+    }
+  }
+}
+
+/* sets *flag when a weight is infinite or NaN: 0 * w is then not 0, and only
+   the dense contraction gives what the products give */
+__global__ void nonfinite_kernel(const float* w, size_t n, int* flag) {
+  bool bad = false;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    bad |= !(fabsf(w[i]) <= 3.402823466e38f);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
+}
+
+/* one row of spikes to every replicate's row of bits */
+__global__ void broadcast_bits_kernel(uint32_t* s, int R, int N, const int8_t* row) {
+  const int W32 = N / 32;
+  const size_t n = (size_t)R * W32;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int8_t* x = row + (i % W32) * 32;
+    uint32_t w = 0;
+    for (int k = 0; k < 32; k++) w |= (x[k] ? 1u : 0u) << k;
+    s[i] = w;
+  }
+}
+
 __global__ void broadcast_spikes_kernel(uint16_t* s, int R, int N, const int8_t* row) {
   size_t n = (size_t)R * N;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -593,7 +968,8 @@ struct bcpnn_recall {
   cudaEvent_t ev_pop = nullptr, ev_gemm = nullptr;
   float* dsup[2] = {nullptr, nullptr};
   float* epsc[2] = {nullptr, nullptr};
-  uint16_t* s[4] = {nullptr, nullptr, nullptr, nullptr}; /* spike ring, by tick mod 4 */
+  uint16_t* s[4] = {nullptr, nullptr, nullptr, nullptr}; /* spike ring, by tick mod 4 (BF16 contraction) */
+  uint32_t* sb[4] = {nullptr, nullptr, nullptr, nullptr}; /* the same as bits [R][N/32] (FP32 contraction) */
   uint16_t* wt = nullptr; /* W^T BF16 [N][N] (BF16 contraction) */
   float* wf = nullptr;    /* W FP32 [N][N], [source][destination] (FP32 contraction) */
   uint8_t* counts = nullptr;
@@ -607,6 +983,9 @@ struct bcpnn_recall {
   int counted = 0;   /* counted ticks since the counters were cleared */
   CUtensorMap map_s[4];
   CUtensorMap map_w;
+  uint4* lists[2] = {nullptr, nullptr}; /* spike lists of a tick, by tick parity (recall_lists_kernel) */
+  uint8_t* list_cnt[2] = {nullptr, nullptr};
+  bool finite_w = false; /* FP32 contraction: every loaded weight is finite */
   uint64_t launches = 0;
   int sms = 148;
   /* in-place timing of the contraction launches (bcpnn_recall_timing) */
@@ -636,7 +1015,9 @@ typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int encode_map(bcpnn_recall* r, CUtensorMap* map, void* base, int rows, int cols, int box_rows) {
+/* tensor map over a row-major [rows][cols] matrix: BF16 in 128-byte swizzled
+   boxes of kTileK columns, or FP32 (f32) in plain boxes of kEvCols columns */
+int encode_map(bcpnn_recall* r, CUtensorMap* map, void* base, int rows, int cols, int box_rows, bool f32 = false) {
   static EncodeTiled fn = nullptr;
   if (!fn) {
     cudaDriverEntryPointQueryResult q;
@@ -646,11 +1027,12 @@ int encode_map(bcpnn_recall* r, CUtensorMap* map, void* base, int rows, int cols
     fn = (EncodeTiled)p;
   }
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kTileK, (cuuint32_t)box_rows};
+  cuuint64_t strides[1] = {(cuuint64_t)cols * (f32 ? 4 : 2)};
+  cuuint32_t box[2] = {(cuuint32_t)(f32 ? kEvCols : kTileK), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult e = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+  CUresult e = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  f32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (e != CUDA_SUCCESS) return fail(r, BCPNN_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)e));
   return BCPNN_OK;
@@ -726,22 +1108,31 @@ int bcpnn_recall_create(const bcpnn_recall_desc* d, bcpnn_recall** out) {
   int rc = BCPNN_OK;
   for (int i = 0; i < 2 && !rc; i++) rc = dalloc(r, &r->dsup[i], RN);
   for (int i = 0; i < 2 && !rc; i++) rc = dalloc(r, &r->epsc[i], RN);
-  for (int i = 0; i < 4 && !rc; i++) rc = dalloc(r, &r->s[i], RN);
+  for (int i = 0; i < 4 && !rc; i++) rc = fp32 ? dalloc(r, &r->sb[i], RN / 32) : dalloc(r, &r->s[i], RN);
   if (!rc && !fp32) rc = dalloc(r, &r->wt, (size_t)N * N);
   if (!rc && fp32) rc = dalloc(r, &r->wf, (size_t)N * N);
   if (!rc) rc = dalloc(r, &r->counts, RN);
   if (!rc) rc = dalloc(r, &r->bj, (size_t)N);
   if (!rc) rc = dalloc(r, &r->lgidx, (size_t)R * H);
   if (!rc) rc = dalloc(r, &r->wmask, (size_t)R * H);
-  if (!rc) rc = dalloc(r, &r->err, 2);
+  if (!rc) rc = dalloc(r, &r->err, 4);
   if (rc) return bad(rc);
-  if (cudaMemset(r->err, 0, 2 * sizeof(int)) != cudaSuccess || cudaMemset(r->counts, 0, RN) != cudaSuccess)
+  if (cudaMemset(r->err, 0, 4 * sizeof(int)) != cudaSuccess || cudaMemset(r->counts, 0, RN) != cudaSuccess)
     return bad(BCPNN_ERR_CUDA);
   if (!fp32) {
     for (int i = 0; i < 4 && !rc; i++) rc = encode_map(r, &r->map_s[i], r->s[i], R, (int)N, kTileM);
     if (!rc) rc = encode_map(r, &r->map_w, r->wt, (int)N, (int)N, kTileN);
     if (rc) return bad(rc);
     if (cudaFuncSetAttribute(recall_tick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) !=
+        cudaSuccess)
+      return bad(BCPNN_ERR_CUDA);
+  } else {
+    if ((rc = encode_map(r, &r->map_w, r->wf, (int)N, (int)N, kEvBox, true))) return bad(rc);
+    for (int i = 0; i < 2; i++)
+      if ((rc = dalloc(r, &r->lists[i], (size_t)R * ((N + kEvRows - 1) / kEvRows) * (kEvListWords / 4))) ||
+          (rc = dalloc(r, &r->list_cnt[i], (size_t)R * ((N + kEvRows - 1) / kEvRows))))
+        return bad(rc);
+    if (cudaFuncSetAttribute(recall_events_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEvSmemBytes) !=
         cudaSuccess)
       return bad(BCPNN_ERR_CUDA);
   }
@@ -778,6 +1169,15 @@ int bcpnn_recall_load(bcpnn_recall* r, const float* w, const float* bj, const fl
   if (r->wf) {
     /* FP32 contraction: W as given, [source][destination] */
     RCU(cudaMemcpy(r->wf, w, (size_t)N * N * 4, cudaMemcpyHostToDevice));
+    int* flag = r->err + 2;
+    int bad = 0;
+    RCU(cudaMemsetAsync(flag, 0, sizeof(int), r->stream));
+    nonfinite_kernel<<<592, 256, 0, r->stream>>>(r->wf, (size_t)N * N, flag);
+    RCU(cudaGetLastError());
+    RCU(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, r->stream));
+    RCU(cudaStreamSynchronize(r->stream));
+    r->finite_w = bad == 0;
+    r->launches++;
   } else {
     /* W^T in BF16: row j = destination MCU, K-contiguous over source MCUs */
     std::vector<uint16_t> wt((size_t)N * N);
@@ -810,8 +1210,12 @@ int bcpnn_recall_load(bcpnn_recall* r, const float* w, const float* bj, const fl
   if (e == cudaSuccess) e = cudaMemcpy(row_s + N, spikes_tm2, (size_t)N, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(row_s + 2 * N, spikes_tm1, (size_t)N, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    for (int k = 0; k < 3; k++)
-      broadcast_spikes_kernel<<<592, 256, 0, r->stream>>>(r->s[mod4(k - 3)], R, N, row_s + (size_t)k * N);
+    for (int k = 0; k < 3; k++) {
+      if (r->wf)
+        broadcast_bits_kernel<<<592, 256, 0, r->stream>>>(r->sb[mod4(k - 3)], R, N, row_s + (size_t)k * N);
+      else
+        broadcast_spikes_kernel<<<592, 256, 0, r->stream>>>(r->s[mod4(k - 3)], R, N, row_s + (size_t)k * N);
+    }
     e = cudaStreamSynchronize(r->stream);
   }
   cudaFree(row_f);
@@ -881,6 +1285,18 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   const int grid = n_tiles < r->sms ? n_tiles : r->sms;
   const int f32_tiles = (r->N / kF32BN) * (d.replicates / kF32BM);
   const int pop_blocks = (int)((size_t)d.replicates * d.hcu_num * 4 / 256);
+  void (*pop)(Params) = nullptr;
+  if (d.mcu_num == 16) pop = r->wf ? recall_pop_kernel<16, true> : recall_pop_kernel<16, false>;
+  if (d.mcu_num == 32) pop = r->wf ? recall_pop_kernel<32, true> : recall_pop_kernel<32, false>;
+  if (d.mcu_num == 64) pop = r->wf ? recall_pop_kernel<64, true> : recall_pop_kernel<64, false>;
+  /* FP32: the contraction by events unless a weight is not finite, or so many
+     MCUs can spike (an HCU's activities sum to at most 1) that the dense form
+     is the faster one */
+  const bool events = r->wf && r->finite_w && p.maxfqdt / (float)d.mcu_num + p.pr <= kEvMaxDensity;
+  const long long ev_pairs = (long long)(r->N / kEvCols) * d.replicates;
+  const int ev_grid = (int)(ev_pairs / kEvWarps < r->sms ? ev_pairs / kEvWarps : r->sms);
+  const int list_blocks =
+      (int)(((long long)d.replicates * ((r->N + kEvRows - 1) / kEvRows) + 255) / 256);
   /* Tick kk: the population update needs epsc(kk-1) and dsup(kk-1); the
      contraction needs S(kk-3) and epsc(kk-1).  So both wait only for tick
      kk-1 and run side by side: pop(kk) after gemm(kk-1) (it also must not
@@ -893,6 +1309,10 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
       r->tev.push_back(e);
     }
   }
+  if (events && n_ticks > 0) /* later ticks' lists are made beside the contraction of the tick before */
+    recall_lists_kernel<<<list_blocks, 256, 0, r->stream>>>(r->sb[mod4(r->kk - 3)], r->lists[r->kk & 1],
+                                                             r->list_cnt[r->kk & 1], d.replicates, r->N);
+  RCU(cudaGetLastError());
   RCU(cudaEventRecord(r->ev_gemm, r->stream));
   RCU(cudaStreamWaitEvent(r->pop_stream, r->ev_gemm, 0));
   for (int i = 0; i < n_ticks; i++) {
@@ -903,15 +1323,20 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
     p.epsc_prev = r->epsc[prev];
     p.epsc_cur = r->epsc[cur];
     p.s_out = r->s[mod4(kk)];
+    p.s_bits = r->sb[mod4(kk)];
     p.simstep = first + i;
     p.count_on = (first + i >= count_first && first + i <= count_last) ? 1 : 0;
-    if (d.mcu_num == 16) recall_pop_kernel<16><<<pop_blocks, 256, 0, r->pop_stream>>>(p);
-    if (d.mcu_num == 32) recall_pop_kernel<32><<<pop_blocks, 256, 0, r->pop_stream>>>(p);
-    if (d.mcu_num == 64) recall_pop_kernel<64><<<pop_blocks, 256, 0, r->pop_stream>>>(p);
+    pop<<<pop_blocks, 256, 0, r->pop_stream>>>(p);
+    if (events && i + 1 < n_ticks)
+      recall_lists_kernel<<<list_blocks, 256, 0, r->pop_stream>>>(r->sb[mod4(kk - 2)], r->lists[cur ^ 1],
+                                                                   r->list_cnt[cur ^ 1], d.replicates, r->N);
     RCU(cudaGetLastError());
     if (r->timing) RCU(cudaEventRecord(r->tev[2 * i], r->stream));
-    if (r->wf)
-      recall_fp32_kernel<<<f32_tiles, kF32Threads, 0, r->stream>>>(r->s[mod4(kk - 3)], r->wf, p);
+    if (events)
+      recall_events_kernel<<<ev_grid, kEvThreads, kEvSmemBytes, r->stream>>>(r->map_w, r->sb[mod4(kk - 3)], r->lists[cur],
+                                                                           r->list_cnt[cur], p);
+    else if (r->wf)
+      recall_fp32_kernel<<<f32_tiles, kF32Threads, 0, r->stream>>>(r->sb[mod4(kk - 3)], r->wf, p);
     else
       recall_tick_kernel<<<grid, kThreads, kSmemBytes, r->stream>>>(r->map_s[mod4(kk - 3)], r->map_w, p);
     RCU(cudaGetLastError());
@@ -925,7 +1350,7 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   }
   r->kk += n_ticks;
   r->counted += counted;
-  r->launches += 2 * (uint64_t)n_ticks;
+  r->launches += (events ? 3 : 2) * (uint64_t)n_ticks;
   int rc = check_err(r); /* synchronises the stream: every timing event has completed */
   if (rc == BCPNN_OK && r->timing) {
     for (int i = 0; i < n_ticks; i++) {
@@ -946,6 +1371,11 @@ static int resolve_rows(bcpnn_recall* r, const char* name, int32_t row0, int32_t
   std::string s(name);
   const long long last = r->kk - 1; /* last tick run */
   *kind = 0;
+  auto spikes = [&](long long tick) {
+    *base = r->wf ? (void*)r->sb[mod4(tick)] : (void*)r->s[mod4(tick)];
+    *elem = 2;
+    *kind = r->wf ? 2 : 1;
+  };
   if (s == "dsup") {
     *base = r->dsup[(int)(last & 1) & 1];
     *elem = 4;
@@ -956,17 +1386,11 @@ static int resolve_rows(bcpnn_recall* r, const char* name, int32_t row0, int32_t
     *base = r->counts;
     *elem = 1;
   } else if (s == "spike" || s == "spike_tm1") {
-    *base = r->s[mod4(last)];
-    *elem = 2;
-    *kind = 1;
+    spikes(last);
   } else if (s == "spike_tm2") {
-    *base = r->s[mod4(last - 1)];
-    *elem = 2;
-    *kind = 1;
+    spikes(last - 1);
   } else if (s == "spike_tm3") {
-    *base = r->s[mod4(last - 2)];
-    *elem = 2;
-    *kind = 1;
+    spikes(last - 2);
   } else {
     return fail(r, BCPNN_ERR_NOT_FOUND, "unknown recall array " + s);
   }
@@ -984,7 +1408,14 @@ int bcpnn_recall_read(bcpnn_recall* r, const char* name, int32_t row0, int32_t n
   if (rc) return rc;
   RCU(cudaSetDevice(r->d.device));
   const size_t off = (size_t)row0 * r->N * elem, n = (size_t)n_rows * r->N;
-  if (kind == 1) {
+  if (kind == 2) {
+    /* N is a multiple of 32: whole words per row */
+    std::vector<uint32_t> tmp(n / 32);
+    RCU(cudaMemcpyAsync(tmp.data(), (uint32_t*)base + (size_t)row0 * r->N / 32, n / 8, cudaMemcpyDeviceToHost, r->stream));
+    RCU(cudaStreamSynchronize(r->stream));
+    int8_t* o = (int8_t*)host;
+    for (size_t i = 0; i < n; i++) o[i] = (int8_t)((tmp[i / 32] >> (i % 32)) & 1u);
+  } else if (kind == 1) {
     std::vector<uint16_t> tmp(n);
     RCU(cudaMemcpyAsync(tmp.data(), (uint8_t*)base + off, n * 2, cudaMemcpyDeviceToHost, r->stream));
     RCU(cudaStreamSynchronize(r->stream));
@@ -1008,7 +1439,13 @@ int bcpnn_recall_write(bcpnn_recall* r, const char* name, int32_t row0, int32_t 
   if (rc) return rc;
   RCU(cudaSetDevice(r->d.device));
   const size_t off = (size_t)row0 * r->N * elem, n = (size_t)n_rows * r->N;
-  if (kind == 1) {
+  if (kind == 2) {
+    std::vector<uint32_t> tmp(n / 32, 0u);
+    const int8_t* in = (const int8_t*)host;
+    for (size_t i = 0; i < n; i++) tmp[i / 32] |= (in[i] ? 1u : 0u) << (i % 32);
+    RCU(cudaMemcpyAsync((uint32_t*)base + (size_t)row0 * r->N / 32, tmp.data(), n / 8, cudaMemcpyHostToDevice, r->stream));
+    RCU(cudaStreamSynchronize(r->stream));
+  } else if (kind == 1) {
     std::vector<uint16_t> tmp(n);
     const int8_t* in = (const int8_t*)host;
     for (size_t i = 0; i < n; i++) tmp[i] = in[i] ? 0x3F80u : 0u;

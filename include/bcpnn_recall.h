@@ -28,7 +28,8 @@
  * Limits: N = H*M a multiple of 256, M dividing 256 (HCUs never straddle a
  * 256-column tile), R a multiple of 128, one population.  sm_100a only.
  * desc.contraction selects an FP32 form of the contraction (W kept in FP32,
- * SIMT multiply-adds) with everything else unchanged.
+ * the weights of the spiking sources added in ascending source order) with
+ * everything else unchanged.
  */
 #ifndef BCPNN_RECALL_H
 #define BCPNN_RECALL_H
@@ -59,8 +60,8 @@ typedef struct bcpnn_recall_desc {
 /* The form of the support contraction S(t-3) . W:
    BCPNN_RECALL_BF16  W rounded once to BF16, tcgen05 tensor-core MMA with
                       FP32 accumulation in tensor memory;
-   BCPNN_RECALL_FP32  W kept in FP32, FP32 fused multiply-adds on the SIMT
-                      pipes (the same engine at full precision, for measuring
+   BCPNN_RECALL_FP32  W kept in FP32, FP32 additions in ascending source order
+                      from 0 (the same engine at full precision, for measuring
                       the BF16 form against).
    Both accumulate in FP32 in an order of their own, not gsbn's row order, and
    share the population kernel and the epsc epilogue. */
