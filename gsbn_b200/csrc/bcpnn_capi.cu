@@ -31,6 +31,11 @@
 #include "bcpnn_tick.cuh"
 #undef BCPNN_TICK_THREADS
 #undef BCPNN_TICK_NS
+#define BCPNN_TICK_THREADS 128
+#define BCPNN_TICK_NS t128
+#include "bcpnn_tick.cuh"
+#undef BCPNN_TICK_THREADS
+#undef BCPNN_TICK_NS
 #include "bcpnn_multi.cuh"
 #include "bcpnn_numerics.h"
 
@@ -384,14 +389,9 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
     cudaLaunchCooperativeKernel(net->tick_fn, dim3(net->total_hcu), dim3(net->threads), args, smem, net->stream);
   } else {
     for (int it = 0; it < n_ticks; ++it) {
-      if (net->threads == 256 && net->fp64)
-        t256::tick_kernel<1, 0><<<net->total_hcu, 256, smem, net->stream>>>(net->d_net, net->d_rp, it, 1, net->bar);
-      else if (net->threads == 256)
-        t256::tick_kernel<0, 0><<<net->total_hcu, 256, smem, net->stream>>>(net->d_net, net->d_rp, it, 1, net->bar);
-      else if (net->fp64)
-        t512::tick_kernel<1, 0><<<net->total_hcu, 512, smem, net->stream>>>(net->d_net, net->d_rp, it, 1, net->bar);
-      else
-        t512::tick_kernel<0, 0><<<net->total_hcu, 512, smem, net->stream>>>(net->d_net, net->d_rp, it, 1, net->bar);
+      int one = 1;
+      void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&it, (void*)&one, (void*)&net->bar};
+      cudaLaunchKernel(net->tick_fn0, dim3(net->total_hcu), dim3(net->threads), args, smem, net->stream);
     }
   }
 }
@@ -411,6 +411,48 @@ int capture_graph(bcpnn_net* net, int n_ticks, bool with_all, cudaGraphExec_t* o
   cudaGraphDestroy(g);
   CU(ie);
   return BCPNN_OK;
+}
+
+/* The tick kernel's instances by CTA size: 512, 256 or 128 threads. */
+struct TickForm {
+  int threads;
+  const void* fn[2][2]; /* [fp64][deferred columns] */
+  size_t (*smem)(int M, int n_in, const int* C);
+};
+
+#define TICK_FORM(T)                                                                                          \
+  {T,                                                                                                         \
+   {{(const void*)t##T::tick_kernel<0, 0>, (const void*)t##T::tick_kernel<0, 1>},                             \
+    {(const void*)t##T::tick_kernel<1, 0>, (const void*)t##T::tick_kernel<1, 1>}},                            \
+   t##T::tick_smem_bytes_for}
+const TickForm kTickForms[] = {TICK_FORM(512), TICK_FORM(256), TICK_FORM(128)};
+#undef TICK_FORM
+
+/* dynamic shared memory of a form for the network's largest population */
+size_t form_smem(const bcpnn_net* net, const TickForm& f) {
+  size_t smem = 0;
+  for (const PopHost& P : net->pops) {
+    int C[kMaxIn] = {0};
+    for (size_t q = 0; q < P.in_proj.size(); ++q) C[q] = net->projs[P.in_proj[q]].C;
+    smem = std::max(smem, f.smem(P.M, (int)P.in_proj.size(), C));
+  }
+  return smem;
+}
+
+/* raise the dynamic shared memory limit of both instances of a form.  The
+   limit is an attribute of the kernel, shared by every network of the process:
+   only ever raised, per device, so that a network created later with a smaller
+   need does not lower it under an earlier one */
+bool raise_smem(const TickForm& f, bool fp64, int dev, size_t smem) {
+  static std::mutex mu;
+  static size_t raised[2][3][kMaxDevices] = {{{0}}};
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& r = raised[fp64 ? 1 : 0][&f - kTickForms][dev];
+  if (smem <= r) return true;
+  for (const void* fn : f.fn[fp64 ? 1 : 0])
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+  r = smem;
+  return true;
 }
 
 /* name -> (kind, pointer, count, element type) resolution */
@@ -570,17 +612,9 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
   net->device = desc->device;
   net->max_ticks = desc->max_ticks_per_run;
   net->exchange = desc->exchange_spikes != 0;
-  net->threads = desc->tick_threads == 256 ? 256 : 512;
   net->fp64 = desc->fp64_tables != 0;
   net->multi = desc->update_variant == 1;
   net->ring_len = desc->spike_buffer_size > 0 ? desc->spike_buffer_size : 1;
-  if (net->threads == 256) {
-    net->tick_fn = net->fp64 ? (const void*)t256::tick_kernel<1, 1> : (const void*)t256::tick_kernel<0, 1>;
-    net->tick_fn0 = net->fp64 ? (const void*)t256::tick_kernel<1, 0> : (const void*)t256::tick_kernel<0, 0>;
-  } else {
-    net->tick_fn = net->fp64 ? (const void*)t512::tick_kernel<1, 1> : (const void*)t512::tick_kernel<0, 1>;
-    net->tick_fn0 = net->fp64 ? (const void*)t512::tick_kernel<1, 0> : (const void*)t512::tick_kernel<0, 0>;
-  }
   {
     const char* e = std::getenv("GSBN_DIRECT_LAUNCH");
     net->direct = e && e[0] == '1';
@@ -831,49 +865,53 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
     net->err = "copy of network descriptor failed";
     return bail(BCPNN_ERR_CUDA);
   }
-  /* shared memory of the resident tick kernel: the largest population */
-  size_t smem = 0;
-  for (const PopHost& P : net->pops) {
-    int C[kMaxIn] = {0};
-    for (size_t q = 0; q < P.in_proj.size(); ++q) C[q] = net->projs[P.in_proj[q]].C;
-    smem = std::max(smem, net->threads == 256 ? t256::tick_smem_bytes_for(P.M, (int)P.in_proj.size(), C)
-                                              : t512::tick_smem_bytes_for(P.M, (int)P.in_proj.size(), C));
-  }
-  int smem_max = 0;
-  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, net->device);
-  if (smem + 1024 > (size_t)smem_max) {
-    net->err = "network too large for the resident tick kernel: " + std::to_string(smem) +
-               " bytes of shared memory per HCU";
-    return bail(BCPNN_ERR_INVALID);
-  }
-  net->tick_smem = smem;
-  /* the limit is an attribute of the kernel, shared by every network of the
-     process: only ever raise it, per device, so that a network created later
-     with a smaller need does not lower it under an earlier one */
+  /* The tick kernel's CTA size, and whether every CTA of the grid (one per
+     HCU) is resident at once, which the persistent launch needs.  A given
+     tick_threads stays; the default is the largest size whose grid is
+     resident: 512 threads up to one HCU per SM, 256 up to two, 128 up to four.
+     256 HCUs x 50 MCUs, C = 1000: 13.9 us per tick with 256 threads, 39.8 with
+     512 in one launch per tick; 310 x 20, C = 400: 14.4 with 128, 45.5 with 512
+     in one launch per tick; up to 148 HCUs the larger CTA is the faster one
+     (100 x 100: 9.9 with 512, 13.7 with 256). */
   {
-    static std::mutex mu;
-    static size_t raised[4][kMaxDevices] = {{0}};
-    std::lock_guard<std::mutex> lock(mu);
-    const int dev = net->device, v = (net->threads == 256 ? 1 : 0) + (net->fp64 ? 2 : 0);
-    if (dev < 0 || dev >= kMaxDevices) { net->err = "device ordinal out of range"; return bail(BCPNN_ERR_INVALID); }
-    if (smem > raised[v][dev]) {
-      if (cudaFuncSetAttribute(net->tick_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-          cudaFuncSetAttribute(net->tick_fn0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (net->device < 0 || net->device >= kMaxDevices) {
+      net->err = "device ordinal out of range";
+      return bail(BCPNN_ERR_INVALID);
+    }
+    int smem_max = 0, coop = 0, sms = 0;
+    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, net->device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, net->device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->device);
+    const char* e = std::getenv("GSBN_PER_TICK");
+    const bool forced = e && e[0] == '1';
+    const int f64 = net->fp64 ? 1 : 0;
+    const TickForm* form = nullptr;
+    for (const TickForm& f : kTickForms) {
+      if (desc->tick_threads ? f.threads != desc->tick_threads : net->max_m > f.threads) continue;
+      const size_t smem = form_smem(net, f);
+      if (smem + 1024 > (size_t)smem_max) {
+        if (form) break; /* a larger size fits */
+        net->err = "network too large for the resident tick kernel: " + std::to_string(smem) +
+                   " bytes of shared memory per HCU";
+        return bail(BCPNN_ERR_INVALID);
+      }
+      if (!raise_smem(f, net->fp64, net->device, smem)) {
         net->err = "cannot raise the shared memory limit of tick_kernel";
         return bail(BCPNN_ERR_CUDA);
       }
-      raised[v][dev] = smem;
+      int per_sm = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f.fn[f64][1], f.threads, smem);
+      const bool resident = (long long)per_sm * sms >= net->total_hcu;
+      if (!form || resident) {
+        form = &f;
+        net->threads = f.threads;
+        net->tick_smem = smem;
+        net->persistent = !forced && coop && resident && !net->multi;
+      }
+      if (resident || net->multi || forced) break;
     }
-  }
-  /* persistent path: every CTA of the grid must be resident at once */
-  {
-    int coop = 0, sms = 0, per_sm = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, net->device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, net->tick_fn, net->threads, smem);
-    const char* e = std::getenv("GSBN_PER_TICK");
-    bool forced = e && e[0] == '1';
-    net->persistent = !forced && coop && (long long)per_sm * sms >= net->total_hcu && !net->multi;
+    net->tick_fn0 = form->fn[f64][0];
+    net->tick_fn = form->fn[f64][1];
     if ((rc = dalloc(net, &net->bar, 4 + (size_t)net->total_hcu))) return bail(rc);
   }
   /* ProcUpdMulti: shared memory of its projection kernel (largest M, C) */

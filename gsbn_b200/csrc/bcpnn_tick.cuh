@@ -31,9 +31,10 @@
 #include "bcpnn_device.cuh"
 
 /* This header is compiled once per CTA size: the includer defines
-   BCPNN_TICK_THREADS (512 or 256) and BCPNN_TICK_NS, the namespace the
-   variant lives in.  512 threads suit large HCUs (one CTA per SM); 256
-   threads let two CTAs share an SM, for batches of small HCUs. */
+   BCPNN_TICK_THREADS (512, 256 or 128) and BCPNN_TICK_NS, the namespace the
+   variant lives in.  512 threads suit networks of up to one HCU per SM; 256
+   (128) threads let two (four) CTAs share an SM, so that networks of more HCUs
+   keep the persistent launch. */
 #ifndef BCPNN_TICK_THREADS
 #define BCPNN_TICK_THREADS 512
 #define BCPNN_TICK_NS t512
@@ -45,7 +46,7 @@ namespace BCPNN_TICK_NS {
 constexpr int kBlock = BCPNN_TICK_THREADS;
 constexpr int kWarps = kBlock / 32;
 constexpr int kRowChunkCells = kBlock; /* row cells staged per chunk (one per thread) */
-constexpr int kMinBlocks = kBlock <= 256 ? 2 : 1;
+constexpr int kMinBlocks = 512 / kBlock; /* 128 registers a thread at every size */
 
 /* The CTA is split in two warp groups that run concurrently inside a tick:
    group A (warps 0-7): support, softmax, spikes, j-traces, active rows;
@@ -429,6 +430,7 @@ __global__ void barrier_probe_kernel(unsigned int* bar, int* err, unsigned long 
    first, as in gsbn (rows, then columns). */
 constexpr int kCellsPerUnit = kColUnit / kGroup;          /* cells of one unit per thread */
 constexpr int kHelpUnits = kCellsPerUnit >= 2 ? 1 : 2;    /* units per pass */
+constexpr int kHelpCells = kCellsPerUnit < 2 ? 1 : 2;     /* cells of a unit per thread at a time */
 
 template <int kF64>
 __device__ __forceinline__ void help_columns(const NetDev* __restrict__ net, const RunParams* __restrict__ rp,
@@ -452,10 +454,6 @@ __device__ __forceinline__ void help_columns(const NetDev* __restrict__ net, con
       for (int u = 0; u < kHelpUnits; ++u)
         if (u0 + u * G < n) d[u] = __ldcg(ring + (beg + u0 + (unsigned)u * G) % cap);
     }
-    size_t index[kHelpUnits][kCellsPerUnit];
-    int tv[kHelpUnits][kCellsPerUnit];
-    float4 cv[kHelpUnits][kCellsPerUnit];
-    bool ok[kHelpUnits][kCellsPerUnit];
     const ProjDev* Jp[kHelpUnits];
     const TabRef* Tp[kHelpUnits];
 #pragma unroll
@@ -474,64 +472,75 @@ __device__ __forceinline__ void help_columns(const NetDev* __restrict__ net, con
           Tp[u] = &rp->tabs[d[u].y];
         }
       }
-#pragma unroll
-      for (int c = 0; c < kCellsPerUnit; ++c) {
-        const int r = c * kGroup + gtid;
-        ok[u][c] = false;
-        if (valid && r < (d[u].w >> 16)) {
-          const ProjDev& J = *Jp[u];
-          const int row = d[u].z + r;
-          index[u][c] = (size_t)row * J.M + (d[u].w & 0xffff);
-          ok[u][c] = J.ii[row] >= 0;
-          tv[u][c] = __ldcg(J.tij + index[u][c]);
-          cv[u][c] = __ldcg(J.cell + index[u][c]);
-        }
-      }
     }
-    PROBE(3); /* B slot 19 */
-    float4 tA[kHelpUnits][kCellsPerUnit], tB[kHelpUnits][kCellsPerUnit];
-    double2 tR0[kHelpUnits][kCellsPerUnit], tR1[kHelpUnits][kCellsPerUnit];
+#pragma unroll 1
+    for (int c0 = 0; c0 < kCellsPerUnit; c0 += kHelpCells) {
+      size_t index[kHelpUnits][kHelpCells];
+      int tv[kHelpUnits][kHelpCells];
+      float4 cv[kHelpUnits][kHelpCells];
+      bool ok[kHelpUnits][kHelpCells];
 #pragma unroll
-    for (int u = 0; u < kHelpUnits; ++u)
+      for (int u = 0; u < kHelpUnits; ++u) {
+        const bool valid = u0 + u * G < n;
 #pragma unroll
-      for (int c = 0; c < kCellsPerUnit; ++c) {
-        if (!ok[u][c]) continue;
-        const TabRef& T = *Tp[u];
-        const int pdt = simstep - tv[u][c];
-        if (pdt > 0 && pdt < T.len) {
-          tA[u][c] = T.tab[(size_t)pdt * 4 + 0];
-          tB[u][c] = T.tab[(size_t)pdt * 4 + 1];
-          tR0[u][c] = T.rtab[(size_t)pdt * 4 + 0];
-          tR1[u][c] = T.rtab[(size_t)pdt * 4 + 1];
-        }
-      }
-#pragma unroll
-    for (int u = 0; u < kHelpUnits; ++u)
-#pragma unroll
-      for (int c = 0; c < kCellsPerUnit; ++c) {
-        if (!ok[u][c]) continue;
-        const ProjDev& J = *Jp[u];
-        const int pdt = simstep - tv[u][c];
-        float4 c4 = cv[u][c];
-        if (pdt <= 0) {
-          c4.w += J.kftj;
-        } else {
-          float4 A = tA[u][c], B = tB[u][c];
-          double2 R0 = tR0[u][c], R1 = tR1[u][c];
-          if (pdt >= Tp[u]->len) {
-            const Coef k = make_coef(J.taupdt * prn, J.ke, J.kzi, J.kzj, kF64);
-            if (kF64)
-              table_pair(k.kp, k.ke, k.kzi, k.kzj, pdt, 0, A, B, 1);
-            else
-              cell_factors(k.kp, k.ke, k.kzi, k.kzj, pdt, A, B);
-            recip_part(A, B, 0, R0, R1);
+        for (int c = 0; c < kHelpCells; ++c) {
+          const int r = (c0 + c) * kGroup + gtid;
+          ok[u][c] = false;
+          if (valid && r < (d[u].w >> 16)) {
+            const ProjDev& J = *Jp[u];
+            const int row = d[u].z + r;
+            index[u][c] = (size_t)row * J.M + (d[u].w & 0xffff);
+            ok[u][c] = J.ii[row] >= 0;
+            tv[u][c] = __ldcg(J.tij + index[u][c]);
+            cv[u][c] = __ldcg(J.cell + index[u][c]);
           }
-          c4 = cell_step_nl(c4, Tp[u], A, B, R0, R1);
-          c4.w = c4.w + J.kftj;
         }
-        J.cell[index[u][c]] = c4;
-        J.tij[index[u][c]] = simstep;
       }
+      PROBE(3); /* B slot 19 */
+      float4 tA[kHelpUnits][kHelpCells], tB[kHelpUnits][kHelpCells];
+      double2 tR0[kHelpUnits][kHelpCells], tR1[kHelpUnits][kHelpCells];
+#pragma unroll
+      for (int u = 0; u < kHelpUnits; ++u)
+#pragma unroll
+        for (int c = 0; c < kHelpCells; ++c) {
+          if (!ok[u][c]) continue;
+          const TabRef& T = *Tp[u];
+          const int pdt = simstep - tv[u][c];
+          if (pdt > 0 && pdt < T.len) {
+            tA[u][c] = T.tab[(size_t)pdt * 4 + 0];
+            tB[u][c] = T.tab[(size_t)pdt * 4 + 1];
+            tR0[u][c] = T.rtab[(size_t)pdt * 4 + 0];
+            tR1[u][c] = T.rtab[(size_t)pdt * 4 + 1];
+          }
+        }
+#pragma unroll
+      for (int u = 0; u < kHelpUnits; ++u)
+#pragma unroll
+        for (int c = 0; c < kHelpCells; ++c) {
+          if (!ok[u][c]) continue;
+          const ProjDev& J = *Jp[u];
+          const int pdt = simstep - tv[u][c];
+          float4 c4 = cv[u][c];
+          if (pdt <= 0) {
+            c4.w += J.kftj;
+          } else {
+            float4 A = tA[u][c], B = tB[u][c];
+            double2 R0 = tR0[u][c], R1 = tR1[u][c];
+            if (pdt >= Tp[u]->len) {
+              const Coef k = make_coef(J.taupdt * prn, J.ke, J.kzi, J.kzj, kF64);
+              if (kF64)
+                table_pair(k.kp, k.ke, k.kzi, k.kzj, pdt, 0, A, B, 1);
+              else
+                cell_factors(k.kp, k.ke, k.kzi, k.kzj, pdt, A, B);
+              recip_part(A, B, 0, R0, R1);
+            }
+            c4 = cell_step_nl(c4, Tp[u], A, B, R0, R1);
+            c4.w = c4.w + J.kftj;
+          }
+          J.cell[index[u][c]] = c4;
+          J.tij[index[u][c]] = simstep;
+        }
+    }
     PROBE(4); /* B slot 20 */
     group_sync(bar_id);
     PROBE(5); /* B slot 21 */

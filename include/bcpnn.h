@@ -89,8 +89,9 @@ typedef struct bcpnn_net_desc {
   int32_t exchange_spikes;   /* 1: ProcExchangeSpike runs every tick          */
   int32_t device;            /* CUDA device ordinal                           */
   int32_t max_ticks_per_run; /* capacity of the per-run spike log             */
-  int32_t tick_threads;      /* CTA size of the tick kernel: 512 (0 = default)
-                                or 256 (two CTAs per SM, HCUs of <= 256 MCUs) */
+  int32_t tick_threads;      /* CTA size of the tick kernel: 512, or 256 (two CTAs
+                                per SM, HCUs of <= 256 MCUs); 0: by the number
+                                of HCUs, the same results */
   int32_t fp64_tables;       /* 0: gsbn's closed-form trace decay in float (bit
                                 parity with the reference CPU path); 1: per
                                 elapsed-tick propagators expm(d A) built in FP64
