@@ -36,6 +36,7 @@
 #include "bcpnn_tick.cuh"
 #undef BCPNN_TICK_THREADS
 #undef BCPNN_TICK_NS
+#include "bcpnn_flow.cuh"
 #include "bcpnn_multi.cuh"
 #include "bcpnn_numerics.h"
 
@@ -133,6 +134,9 @@ struct bcpnn_net {
   int ring_len = 1;         /* its spike buffer size */
   const void* tick_fn = nullptr;  /* the tick kernel variant of the persistent launch */
   const void* tick_fn0 = nullptr; /* the same size and decay form with in-CTA columns */
+  const void* flow_fn = nullptr;  /* the dataflow kernel (bcpnn_flow.cuh), where the network fits it */
+  size_t flow_smem = 0;
+  flow::Args flow_args{};
   unsigned int* bar = nullptr; /* persistent kernel: [0] grid barrier arrivals, [1..2] column units by
                                   tick parity, [4 + cta] column units done for each CTA */
   int4* col_ring = nullptr;    /* deferred column units (NetDev::col_ring) */
@@ -341,6 +345,14 @@ int reset_state(bcpnn_net* net) {
   return BCPNN_OK;
 }
 
+/* external spike replay is tick_kernel's */
+bool use_flow(const bcpnn_net* net) {
+  if (!net->flow_fn) return false;
+  for (const PopDev& D : net->hp)
+    if (D.ext) return false;
+  return true;
+}
+
 /* the work of one run, queued on the network's stream */
 void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
   for (const PopHost& P : net->pops)
@@ -382,7 +394,11 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
     }
     return;
   }
-  if (net->persistent) {
+  if (use_flow(net)) {
+    int n = n_ticks;
+    void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&net->flow_args, (void*)&n};
+    cudaLaunchCooperativeKernel(net->flow_fn, dim3(net->total_hcu), dim3(net->threads), args, net->flow_smem, net->stream);
+  } else if (net->persistent) {
     cudaMemsetAsync(net->bar, 0, (4 + (size_t)net->total_hcu) * sizeof(unsigned int), net->stream);
     int it0 = 0, n = n_ticks;
     void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&it0, (void*)&n, (void*)&net->bar};
@@ -453,6 +469,75 @@ bool raise_smem(const TickForm& f, bool fp64, int dev, size_t smem) {
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
   r = smem;
   return true;
+}
+
+/* The dataflow kernel's instances: CTA size and warps of population update
+   (one MCU per thread), the fewest that hold the network's largest HCU. */
+struct FlowForm {
+  int threads, pop_warps, queue_warps;
+  const void* fn;
+};
+#define FLOW_FORM(T, P, Q) {T, P, Q, (const void*)flow::flow_kernel<T, P, Q>}
+const FlowForm kFlowForms[] = {FLOW_FORM(512, 1, 2), FLOW_FORM(512, 2, 2), FLOW_FORM(512, 4, 2),
+                               FLOW_FORM(256, 1, 1), FLOW_FORM(256, 2, 1), FLOW_FORM(256, 4, 1)};
+#undef FLOW_FORM
+
+/* choose the dataflow kernel for a persistent network; leaves flow_fn null
+   where the network does not fit it */
+int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
+#ifndef BCPNN_PHASE_PROBE /* the probe build measures tick_kernel */
+  if (net->max_m > flow::kMaxM) return BCPNN_OK;
+  std::vector<int> word0;
+  int n_words = 0;
+  for (const PopHost& P : net->pops) {
+    word0.push_back(n_words);
+    n_words += P.H * ((P.M + 31) / 32);
+    if (n_words > flow::kMaxWords) return BCPNN_OK;
+  }
+  for (const FlowForm& f : kFlowForms) {
+    if (f.threads != net->threads || f.pop_warps * 32 < net->max_m) continue;
+    size_t smem = 0;
+    for (const PopHost& P : net->pops) {
+      int C[kMaxIn] = {0};
+      for (size_t q = 0; q < P.in_proj.size(); ++q) C[q] = net->projs[P.in_proj[q]].C;
+      for (int c : C)
+        if (c > 0xfffe) return BCPNN_OK; /* slot numbers in 16 bits */
+      smem = std::max(smem, flow::smem_bytes(P.M, (int)P.in_proj.size(), C, n_words, f.threads, f.queue_warps));
+    }
+    if (smem + 8192 > smem_max) return BCPNN_OK;
+    static std::mutex mu;
+    static size_t raised[sizeof(kFlowForms) / sizeof(kFlowForms[0])][kMaxDevices] = {{0}};
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      size_t& r = raised[&f - kFlowForms][net->device];
+      if (smem > r) {
+        CU(cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        r = smem;
+      }
+    }
+    int per_sm = 0;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f.fn, f.threads, smem));
+    if ((long long)per_sm * sms < net->total_hcu) return BCPNN_OK;
+    int rc;
+    int* d_word0 = nullptr;
+    unsigned long long *words = nullptr, *seeds = nullptr;
+    const size_t nw = (size_t)flow::kWordTicks * n_words, ns = (size_t)flow::kSeedTicks * net->pops.size();
+    if ((rc = dalloc(net, &d_word0, word0.size())) || (rc = dalloc(net, &words, nw)) || (rc = dalloc(net, &seeds, ns)))
+      return rc;
+    CU(cudaMemcpyAsync(d_word0, word0.data(), word0.size() * sizeof(int), cudaMemcpyHostToDevice, net->stream));
+    CU(cudaMemsetAsync(words, 0, nw * sizeof(*words), net->stream));
+    CU(cudaMemsetAsync(seeds, 0, ns * sizeof(*seeds), net->stream));
+    CU(cudaStreamSynchronize(net->stream));
+    net->flow_args.words = words;
+    net->flow_args.seeds = seeds;
+    net->flow_args.word0 = d_word0;
+    net->flow_args.n_words = n_words;
+    net->flow_smem = smem;
+    net->flow_fn = f.fn;
+    return BCPNN_OK;
+  }
+#endif
+  return BCPNN_OK;
 }
 
 /* name -> (kind, pointer, count, element type) resolution */
@@ -913,6 +998,7 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
     net->tick_fn0 = form->fn[f64][0];
     net->tick_fn = form->fn[f64][1];
     if ((rc = dalloc(net, &net->bar, 4 + (size_t)net->total_hcu))) return bail(rc);
+    if (net->persistent && (rc = setup_flow(net, sms, (size_t)smem_max))) return bail(rc);
   }
   /* ProcUpdMulti: shared memory of its projection kernel (largest M, C) */
   if (net->multi) {

@@ -1,0 +1,842 @@
+/*
+ * bcpnn_flow.cuh -- the tick of the plain FP32 path as a dataflow inside and
+ * between CTAs: one CTA per (population, destination HCU), persistent over a
+ * run, without a grid-wide barrier.  HCUs of at most 128 MCUs; the others, and
+ * external spike replay, take tick_kernel (bcpnn_tick.cuh).
+ *
+ * What a tick t of HCU h needs (ProcUpdLazy.cpp:88-124):
+ *   P(t)  population update  Pop.cpp:229-323: epsc(t-1), bj(t-1), and the
+ *         softmax seed of the tick, the new dsup of the population's MCU 0
+ *         (Pop.cpp:270), which HCU 0 computes first thing in its P(t);
+ *   W(t)  rows  Proj.cpp:365-479, 667-720: the active rows listed by Q(t-1),
+ *         pj(t), and the columns of t-1 (same cells); it gives epsc(t).  It
+ *         does not need the spikes of t: zj alone takes them (Proj.cpp:349);
+ *         columns  Proj.cpp:481-536, 722-760: the spikes of t, after its rows;
+ *   Q(t)  delay queue  Proj.cpp:621-630, 645-664: the spikes of t-1 of every
+ *         source HCU; it lists the active rows of t+1.
+ * So three groups of warps run side by side and meet at shared-memory
+ * mbarriers: E(t) (W -> P, Q: epsc(t), and the lists of t are free), S(t) (P ->
+ * W: spikes of t, pj(t+1)), L(t+1) (Q -> W: the active rows of t+1).  A CTA
+ * whose HCU spikes does its whole columns itself while its next population
+ * update runs; only its rows of t+1 wait, and through them its P(t+2).
+ *
+ * Between CTAs a spike word carries its own flag: 32 spikes and the tick's tag
+ * in 64 bits, one relaxed store, polled by every CTA's Q.  Q waits for the
+ * words of all HCUs of the network, its sources or not, which bounds how far
+ * CTAs run apart: P(t) needs Q(t-2), so a CTA that publishes t has seen every
+ * word of t-3, and a CTA that published t-3 has read the words of t-6 and the
+ * seed of t-3.  Words are kept for 8 ticks and seeds for 4.
+ *
+ * Bound by the longest cycle of dependences: P(t) -> columns(t) -> rows(t+1) ->
+ * P(t+2) takes two ticks, E(t-1) -> P(t) one.  Per tick, against tick_kernel with
+ * its grid barrier and its columns spread over the grid: 10 x 10 2.88 us (7.4),
+ * 50 x 50 3.77 (8.8), 100 x 100 with C = 1000 6.18 (9.9), 256 x 50 with C = 1000
+ * 10.4 (13.8), 296 x 20 with C = 400 6.2 (11.3).  The decays and their exact
+ * division are those of bcpnn_device.cuh, so every value is bit-identical to
+ * tick_kernel's and to the oracle's.
+ *
+ * Every wait is bounded (kBarrierNs): it sets kErrBarrier and the CTA's abort
+ * flag, the groups leave their tick loops together, and the state is not
+ * written back.
+ */
+#ifndef BCPNN_FLOW_CUH
+#define BCPNN_FLOW_CUH
+
+#include "bcpnn_device.cuh"
+
+namespace bcpnn {
+namespace flow {
+
+constexpr int kMaxM = 128;        /* one MCU per thread of up to four warps */
+constexpr int kWordTicks = 8, kSeedTicks = 4;
+constexpr int kMaxWords = 2047;   /* word and bit of a source MCU in 16 bits, 0xffff: none */
+constexpr unsigned long long kWaitNs = 2000000000ull;
+
+struct Args {
+  unsigned long long* words; /* [kWordTicks][n_words]: tag << 32 | 32 spikes */
+  unsigned long long* seeds; /* [n_pops][kSeedTicks]: tag << 32 | float bits */
+  const int* word0;          /* [n_pops] first word of a population */
+  int n_words;
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+/* An event of every tick: four mbarriers by tick, so that a group which is up to
+   three ticks behind the one that signals still finds its tick's phase (a phase
+   is told by its parity; no group falls more than two behind). */
+constexpr int kEventTicks = 4;
+
+__device__ __forceinline__ void mb_init(unsigned long long* ev) {
+  for (int k = 0; k < kEventTicks; ++k)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(ev + k)) : "memory");
+}
+
+__device__ __forceinline__ void mb_arrive(unsigned long long* ev, int k) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(ev + k % kEventTicks)) : "memory");
+}
+
+__device__ __forceinline__ bool mb_try(unsigned long long* b, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_addr(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+/* wait for the event of tick k >= 0; false when another group gave up, or after kWaitNs */
+__device__ __forceinline__ bool mb_wait(unsigned long long* ev, int k, volatile int* abort_flag, int* err) {
+  unsigned long long* const b = ev + k % kEventTicks;
+  const uint32_t parity = (uint32_t)(k / kEventTicks) & 1u;
+  if (mb_try(b, parity)) return true;
+  const unsigned long long t0 = now_ns();
+  while (!mb_try(b, parity)) {
+    if (*abort_flag) return false;
+    if (now_ns() - t0 > kWaitNs) {
+      atomicOr(err, kErrBarrier);
+      *abort_flag = 1;
+      return false;
+    }
+  }
+  return true;
+}
+
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void st_word(unsigned long long* p, uint32_t tag, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)tag << 32) | v) : "memory");
+}
+
+/* poll *p for the tag; false when a group or another CTA gave up, or after kWaitNs */
+__device__ __forceinline__ bool poll_word(const unsigned long long* p, uint32_t tag, uint32_t& v, volatile int* abort_flag,
+                                          int* err) {
+  unsigned long long w = ld_word(p);
+  if ((uint32_t)(w >> 32) != tag) {
+    const unsigned long long t0 = now_ns();
+    do {
+      if (*abort_flag || *(volatile int*)err) {
+        *abort_flag = 1;
+        return false;
+      }
+      if (now_ns() - t0 > kWaitNs) {
+        atomicOr(err, kErrBarrier);
+        *abort_flag = 1;
+        return false;
+      }
+      w = ld_word(p);
+    } while ((uint32_t)(w >> 32) != tag);
+  }
+  v = (uint32_t)w;
+  return true;
+}
+
+/* barrier of one group of n threads; bar_any also gives the OR of a flag */
+__device__ __forceinline__ void bar(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+__device__ __forceinline__ bool bar_any(int id, int n, bool flag) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(id), "r"(n), "r"((uint32_t)flag)
+      : "memory");
+  return r != 0;
+}
+
+/* shared-memory layout of a CTA, in 4-byte words */
+struct Layout {
+  int act;                 /* [M rounded up to 4] */
+  int bits;                /* [n_words] the previous tick's spikes of the network */
+  int pi;                  /* [rows of a chunk] */
+  int w;                   /* [chunk cells] */
+  int skip;                /* bytes [chunk cells] */
+  int q[kMaxIn];           /* blocks of the incoming projections */
+  int total;
+};
+
+/* slots per queue warp, a multiple of 32 */
+__host__ __device__ inline int queue_part(int C, int qw) { return ((C + qw - 1) / qw + 31) & ~31; }
+
+/* a projection's block: pj ej zj bj [M], epsc [2][M], pjn [2][M]; qi [C]; then 16-bit list [2][qw * part], src [C]; bytes
+   di [C] */
+__host__ __device__ inline int block_words(int M, int C, int qw) {
+  return 8 * M + C + (2 * qw * queue_part(C, qw) + C + 1) / 2 + (C + 3) / 4;
+}
+
+__host__ __device__ inline int chunk_rows(int M, int cells) { return cells / M < 1 ? 1 : cells / M; }
+
+__host__ __device__ inline void layout(int M, int n_in, const int* C, int n_words, int cells, int qw, Layout& L) {
+  int o = 0;
+  L.act = o; o += (M + 3) & ~3;
+  L.bits = o; o += (n_words + 3) & ~3;
+  const int rows = chunk_rows(M, cells);
+  const int n = rows * M > cells ? rows * M : cells;
+  L.pi = o; o += rows;
+  L.w = o; o += n;
+  L.skip = o; o += (n + 3) / 4;
+  for (int k = 0; k < kMaxIn; ++k) {
+    L.q[k] = o;
+    if (k < n_in) o += block_words(M, C[k], qw);
+  }
+  L.total = o;
+}
+
+struct Block {
+  float *pj, *ej, *zj, *bj, *epsc, *pjn;
+  uint32_t* qi;
+  uint16_t *list, *src;
+  uint8_t* di;
+};
+
+template <int kQW>
+__device__ __forceinline__ Block block(float* sm, const Layout& L, int k, int M, int C) {
+  Block b;
+  float* f = sm + L.q[k];
+  b.pj = f;
+  b.ej = f + M;
+  b.zj = f + 2 * M;
+  b.bj = f + 3 * M;
+  b.epsc = f + 4 * M;
+  b.pjn = f + 6 * M;
+  b.qi = (uint32_t*)(f + 8 * M);
+  b.list = (uint16_t*)(b.qi + C);
+  b.src = b.list + 2 * kQW * queue_part(C, kQW);
+  b.di = (uint8_t*)((uint32_t*)b.list + (2 * kQW * queue_part(C, kQW) + C + 1) / 2);
+  return b;
+}
+
+constexpr int kBarP = 1, kBarW = 2, kBarQ = 3;
+/* delay byte: delay in bits 0-4; bit 5: the source population is not published, and bits 6 and 7 are its constant flags
+   by tick parity; else bit 6 is the source's spike before the launch */
+constexpr int kUnfed = 32;
+
+/* kThreads: 512 (one CTA per SM) or 256 (two); kPW warps of population update (M <= 32 kPW), kQW of delay queue, the
+   others rows and columns */
+template <int kThreads, int kPW, int kQW>
+__global__ void __launch_bounds__(kThreads, 512 / kThreads)
+    flow_kernel(const NetDev* __restrict__ net_g, const RunParams* __restrict__ rp_g, Args fa, int n_ticks) {
+  constexpr int kP = kPW * 32, kQ = kQW * 32, kW = kThreads - kP - kQ;
+  constexpr int kCells = kThreads; /* row cells of one chunk */
+  extern __shared__ __align__(16) float sm[];
+  __shared__ NetDev s_net;
+  __shared__ RunParams s_rp;
+  __shared__ PopDev s_pop;
+  __shared__ ProjDev s_proj[kMaxIn];
+  __shared__ TabRef s_tab[kMaxIn];
+  __shared__ int s_inp[kMaxIn], s_srcM[kMaxIn], s_src0[kMaxIn], s_fed[kMaxIn];
+  __shared__ Layout s_L;
+  __shared__ unsigned long long s_E[kEventTicks], s_S[kEventTicks], s_Lst[kEventTicks];
+  __shared__ int s_abort;
+  __shared__ int s_nl[kMaxIn][2][kQW]; /* list lengths by tick parity */
+  __shared__ uint32_t s_spk[2][kPW];   /* spikes of this HCU by tick parity */
+  __shared__ float s_red[kPW];
+  __shared__ float s_seed;
+  __shared__ unsigned long long s_rows, s_cols;
+
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    s_net = *net_g;
+    s_rp = *rp_g;
+    s_abort = 0;
+    s_rows = s_cols = 0;
+    mb_init(s_E);
+    mb_init(s_S);
+    mb_init(s_Lst);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const NetDev* __restrict__ net = &s_net;
+  const RunParams* __restrict__ rp = &s_rp;
+  const int P = net->cta_pop[blockIdx.x], h = net->cta_hcu[blockIdx.x];
+  if (tid == 0) s_pop = net->pops[P];
+  __syncthreads();
+  const PopDev& pop = s_pop;
+  const int M = pop.M, n = pop.n, n_in = pop.n_in;
+  if (tid < kMaxIn && tid < n_in) {
+    const int p = pop.in_proj[tid];
+    s_inp[tid] = p;
+    s_proj[tid] = net->projs[p];
+    s_tab[tid] = rp->tabs[p];
+    const PopDev& src = net->pops[s_proj[tid].src];
+    s_srcM[tid] = src.M;
+    s_src0[tid] = fa.word0[s_proj[tid].src];
+    int fed = 0;
+    for (int k = 0; k < src.n_out; ++k) fed |= src.out_proj[k] == p;
+    s_fed[tid] = fed;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int c[kMaxIn];
+#pragma unroll
+    for (int k = 0; k < kMaxIn; ++k) c[k] = k < n_in ? s_proj[k].C : 0;
+    layout(M, n_in, c, fa.n_words, kCells, kQW, s_L);
+  }
+  __syncthreads();
+  const Layout& L = s_L;
+  float* s_act = sm + L.act;
+  uint32_t* s_bits = (uint32_t*)(sm + L.bits);
+
+  /* ---- load the state the previous tick left ---- */
+  const int cur0 = rp->k0 & 1, prev0 = cur0 ^ 1;
+  const float prn = rp->prn;
+  for (int k = 0; k < n_in; ++k) {
+    const ProjDev& J = s_proj[k];
+    Block B = block<kQW>(sm, L, k, M, J.C);
+    const size_t eoff = (size_t)J.proj_in_pop * n;
+    const float kp = J.taupdt * prn;
+    for (int j = tid; j < M; j += kThreads) {
+      const int idx = h * M + j;
+      const float pj = J.pj[idx], ej = J.ej[idx];
+      B.pj[j] = pj;
+      B.ej[j] = ej;
+      B.zj[j] = J.zj[idx];
+      B.bj[j] = pop.bj[prev0][eoff + idx];
+      B.epsc[prev0 * M + j] = pop.epsc[prev0][eoff + idx];
+      B.pjn[cur0 * M + j] = pj + (ej - pj) * kp;
+    }
+    for (int s = tid; s < J.C; s += kThreads) {
+      const int r = h * J.C + s, ii = J.ii[r];
+      uint32_t src = 0xffffu, di = 0;
+      if (ii >= J.Ns) atomicOr(net->err, kErrIndex);
+      if (ii >= 0 && ii < J.Ns) {
+        const int hs = ii / s_srcM[k], ms = ii - hs * s_srcM[k];
+        src = (uint32_t)(s_src0[k] + hs * ((s_srcM[k] + 31) >> 5) + (ms >> 5)) << 5 | (uint32_t)(ms & 31);
+        di = (uint32_t)J.di[r] & 31u;
+        if (s_fed[k]) di |= J.si[prev0][ii] > 0 ? 64u : 0u;
+        else di |= kUnfed | (J.si[0][ii] > 0 ? 64u : 0u) | (J.si[1][ii] > 0 ? 128u : 0u);
+      }
+      B.src[s] = (uint16_t)src;
+      B.di[s] = (uint8_t)di;
+      B.qi[s] = (uint32_t)J.qi[r];
+    }
+    /* the listed rows, ascending, by queue warp: the first part's are the first n0 */
+    const int part = queue_part(J.C, kQW), cnt = J.list_cnt[h];
+    const int* rows = J.list + h * J.C;
+    int n0 = cnt;
+    if (kQW > 1) {
+      int lo = 0, hi = cnt; /* first entry of the second part */
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rows[mid] - h * J.C < part) lo = mid + 1;
+        else hi = mid;
+      }
+      n0 = lo;
+    }
+    if (tid < kQW) s_nl[k][cur0][tid] = tid == 0 ? n0 : cnt - n0;
+    for (int e = tid; e < cnt; e += kThreads)
+      B.list[cur0 * kQW * part + (e < n0 ? e : part + e - n0)] = (uint16_t)(rows[e] - h * J.C);
+  }
+  if (tid < ((M + 3) & ~3) - M) s_act[M + tid] = 0.0f; /* read by the serial sum */
+  __syncthreads();
+
+  if (tid < kP) {
+    /* ================= P: population update, j-traces ================= */
+    const int j = tid, warp = tid >> 5, lane = tid & 31;
+    const bool active = j < M;
+    const int idx = h * M + (active ? j : 0);
+    float dsup = pop.dsup[prev0][idx], act = pop.act[idx];
+    int cnt = pop.counter[idx];
+    bool spk = false;
+    const float lg = rp->lginp[pop.mcu_start + idx], wm = rp->wmask[pop.hcu_start + h];
+    const int wph = (M + 31) >> 5;
+    const float pr = net->poisson_hz * net->dt;
+    bool bad = false;
+    for (int it = 0; it < n_ticks; ++it) {
+      const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1, prev = cur ^ 1;
+      const uint32_t tag = rp->serial0 + (uint32_t)it;
+      /* what depends on tick and MCU only, before the wait */
+      const float u = bx_uniform01(pop.rng_seed, pop.rng_pop, (uint32_t)simstep, (uint32_t)idx);
+      bool extra = false;
+      if (net->poisson_hz > 0.0f)
+        extra = bx_uniform01_poisson(pop.rng_seed, pop.rng_pop, (uint32_t)simstep, (uint32_t)idx) < pr;
+      float noise = 0.0f;
+      if (pop.snoise != 0.0f)
+        noise = pop.snoise * dev_normal01(pop.rng_seed, pop.rng_pop, (uint32_t)simstep, (uint32_t)idx);
+      float sup = pop.lgbias + pop.igain * lg + noise;
+      if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
+      float wsup = 0.0f;
+      for (int k = 0; k < n_in; ++k) {
+        const Block B = block<kQW>(sm, L, k, M, s_proj[k].C);
+        if (active) wsup += B.bj[j] + B.epsc[prev * M + j];
+      }
+      sup += (pop.wgain * wm) * wsup;
+      const float d = dsup + (sup - dsup) * pop.taumdt;
+      /* the softmax seed (Pop.cpp:270) */
+      unsigned long long* const slot = fa.seeds + P * kSeedTicks + (tag & (kSeedTicks - 1));
+      float seed = 0.0f;
+      if (h == 0) {
+        if (tid == 0) {
+          st_word(slot, tag, __float_as_uint(d));
+          s_seed = d;
+        }
+      } else if (lane == 0) {
+        if (it == 0) {
+          float ws = 0.0f;
+          int offset = 0;
+          for (int m = 0; m < pop.dim_proj; m++) {
+            ws += __ldcg(pop.bj[prev] + offset) + __ldcg(pop.epsc[prev] + offset);
+            offset += n;
+          }
+          float nz = 0.0f;
+          if (pop.snoise != 0.0f) nz = pop.snoise * dev_normal01(pop.rng_seed, pop.rng_pop, (uint32_t)simstep, 0u);
+          float sp = pop.lgbias + pop.igain * rp->lginp[pop.mcu_start] + nz;
+          sp += (pop.wgain * rp->wmask[pop.hcu_start]) * ws;
+          const float d0 = __ldcg(pop.dsup[prev]);
+          seed = d0 + (sp - d0) * pop.taumdt;
+        } else if (!bad) {
+          uint32_t v = 0;
+          bad = !poll_word(slot, tag, v, &s_abort, net->err);
+          seed = __uint_as_float(v);
+        }
+      }
+      /* pj of the next tick (Proj.cpp:340: it takes ej and pj only); its buffer is free, the rows that read it are done */
+      for (int k = 0; k < n_in; ++k) {
+        const ProjDev& J = s_proj[k];
+        const Block B = block<kQW>(sm, L, k, M, J.C);
+        if (active) {
+          const float pj = B.pjn[cur * M + j];
+          float ej = B.ej[j];
+          ej += (B.zj[j] - ej) * J.ke;
+          B.pj[j] = pj;
+          B.ej[j] = ej;
+          B.pjn[prev * M + j] = pj + (ej - pj) * (J.taupdt * prn);
+        }
+      }
+      /* the maximum: of the HCU's MCUs, then against the seed, which a NaN never replaces and which stays if it is NaN */
+      float mx = __int_as_float(0xff800000);
+      if (active && d > mx) mx = d;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float w = __shfl_xor_sync(0xffffffffu, mx, o);
+        mx = (w > mx) ? w : mx;
+      }
+      seed = __shfl_sync(0xffffffffu, seed, 0);
+      if (kPW > 1) {
+        if (lane == 0) s_red[warp] = mx;
+        bar(kBarP, kP);
+        if (h == 0) seed = s_seed;
+        float m = seed;
+#pragma unroll
+        for (int w = 0; w < kPW; ++w) m = (s_red[w] > m) ? s_red[w] : m;
+        mx = m;
+      } else {
+        if (h == 0) seed = __shfl_sync(0xffffffffu, d, 0);
+        mx = (mx > seed) ? mx : seed;
+      }
+      const float maxact = bx_expf(pop.wtagain * mx);
+      float a = bx_expf(pop.wtagain * (d - mx));
+      if (maxact < 1.0f) a *= maxact;
+      if (active) s_act[j] = a;
+      if (kPW > 1) bar(kBarP, kP);
+      else __syncwarp();
+      /* serial, in MCU order (Pop.cpp:281-293), by every thread; the padding adds +0 to a sum that is never -0 */
+      float vsum = 0.0f;
+      {
+        const float4* v = (const float4*)s_act;
+        float4 x = v[0];
+        for (int m = 4; m < M; m += 4) {
+          const float4 y = v[m >> 2];
+          vsum += x.x;
+          vsum += x.y;
+          vsum += x.z;
+          vsum += x.w;
+          x = y;
+        }
+        vsum += x.x;
+        vsum += x.y;
+        vsum += x.z;
+        vsum += x.w;
+      }
+      if (vsum > 1.0f) a /= vsum;
+      spk = active && ((u < a * pop.maxfqdt) || extra);
+      const uint32_t word = __ballot_sync(0xffffffffu, spk);
+      if (lane == 0 && warp < wph) {
+        st_word(fa.words + (size_t)(tag & (kWordTicks - 1)) * fa.n_words + fa.word0[P] + h * wph + warp, tag, word);
+        s_spk[cur][warp] = word;
+      }
+      if (kPW > 1) {
+        bad = bar_any(kBarP, kP, bad);
+      } else {
+        bad = __any_sync(0xffffffffu, bad);
+        __syncwarp();
+      }
+      if (tid == 0) mb_arrive(s_S, it); /* the group's writes happen before: barrier above */
+      /* in the shadow of the rows and columns: state, traces, bias, records */
+      dsup = d;
+      act = a;
+      cnt += spk ? 1 : 0;
+      if (spk) {
+        atomicOr(&pop.spk_log[(size_t)it * pop.log_words + (idx >> 5)], 1u << (idx & 31));
+        if (idx == 9)
+          for (int k = 0; k < n_in; ++k) atomicOr(&net->ss_log[(size_t)it * net->n_projs + s_inp[k]], 2u);
+      }
+      for (int k = 0; k < n_in; ++k) {
+        const ProjDev& J = s_proj[k];
+        const Block B = block<kQW>(sm, L, k, M, J.C);
+        if (active) {
+          float zj = B.zj[j];
+          zj *= (1 - J.kzj);
+          if (spk) zj += J.kftj;
+          B.zj[j] = zj;
+          if (J.taupdt * prn != 0.0f) B.bj[j] = J.bgain * bx_logf(B.pj[j] + J.eps);
+        }
+      }
+      if (bad) break;
+    }
+    bar(0, kThreads);
+    if (!s_abort && active) {
+      const int last = (rp->k0 + n_ticks - 1) & 1;
+      pop.dsup[last][idx] = dsup;
+      pop.act[idx] = act;
+      pop.counter[idx] = cnt;
+      pop.spike[idx] = spk ? 1 : 0;
+      for (int k = 0; k < pop.n_out; ++k) net->projs[pop.out_proj[k]].si[last][idx] = spk ? 1 : 0;
+    }
+  } else if (tid < kP + kQ) {
+    /* ================= Q: spike words, delay queue ================= */
+    const int qt = tid - kP, warp = qt >> 5, lane = qt & 31;
+    bool bad = false;
+    for (int it = 0; it < n_ticks; ++it) {
+      const int cur = (rp->k0 + it) & 1, prev = cur ^ 1, nxt = prev;
+      if (it > 0) {
+        const uint32_t tag = rp->serial0 + (uint32_t)(it - 1);
+        const unsigned long long* w = fa.words + (size_t)(tag & (kWordTicks - 1)) * fa.n_words;
+        for (int x0 = 0; x0 < fa.n_words; x0 += 4 * kQ) {
+          /* four words' loads at once; the late ones are polled */
+          unsigned long long v[4];
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const int x = x0 + y * kQ + qt;
+            if (x < fa.n_words) v[y] = ld_word(w + x);
+          }
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const int x = x0 + y * kQ + qt;
+            if (x < fa.n_words) {
+              uint32_t b = (uint32_t)v[y];
+              if ((uint32_t)(v[y] >> 32) != tag && !bad) bad = !poll_word(w + x, tag, b, &s_abort, net->err);
+              s_bits[x] = b;
+            }
+          }
+        }
+        /* the lists written below were read by the rows of it - 1 */
+        if (!bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
+      }
+      if (kQW > 1) bar(kBarQ, kQ);
+      else __syncwarp();
+      for (int k = 0; k < n_in; ++k) {
+        const ProjDev& J = s_proj[k];
+        const int C = J.C;
+        const Block B = block<kQW>(sm, L, k, M, C);
+        const int part = queue_part(C, kQW);
+        uint16_t* out = B.list + (nxt * kQW + warp) * part;
+        const int s1 = min(C, (warp + 1) * part);
+        int total = 0;
+        for (int s0 = warp * part; s0 < s1; s0 += 128) {
+          uint32_t src[4], di[4], qv[4];
+          bool on[4];
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const int s = s0 + y * 32 + lane;
+            src[y] = 0xffffu;
+            if (s < s1) {
+              src[y] = B.src[s];
+              di[y] = B.di[s];
+              qv[y] = B.qi[s];
+            }
+          }
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const int s = s0 + y * 32 + lane;
+            on[y] = false;
+            if (src[y] != 0xffffu) {
+              bool sp;
+              if (di[y] & kUnfed) sp = (di[y] >> (6 + prev)) & 1u;
+              else if (it == 0) sp = (di[y] >> 6) & 1u;
+              else sp = (s_bits[src[y] >> 5] >> (src[y] & 31u)) & 1u;
+              on[y] = qv[y] & 1u;
+              uint32_t q = (uint32_t)((int)qv[y] >> 1);
+              if (sp) q |= 1u << ((di[y] & 31u) - 1u);
+              B.qi[s] = q;
+            }
+          }
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const unsigned m = __ballot_sync(0xffffffffu, on[y]);
+            if (on[y]) out[total + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(s0 + y * 32 + lane);
+            total += __popc(m);
+          }
+        }
+        if (lane == 0) s_nl[k][nxt][warp] = total;
+      }
+      if (kQW > 1) {
+        bad = bar_any(kBarQ, kQ, bad);
+      } else {
+        bad = __any_sync(0xffffffffu, bad);
+        __syncwarp();
+      }
+      if (qt == 0) mb_arrive(s_Lst, it);
+      if (bad) break;
+    }
+    bar(0, kThreads);
+  } else {
+    /* ================= W: rows, columns ================= */
+    const int wt = tid - kP - kQ;
+    float* s_pi = sm + L.pi;
+    float* s_w = sm + L.w;
+    int8_t* s_skip = (int8_t*)(sm + L.skip);
+    const int rch = chunk_rows(M, kCells);
+    bool bad = false;
+    for (int it = 0; it < n_ticks; ++it) {
+      const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1, prev = cur ^ 1;
+      if (it > 0) {
+        if (!bad) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err);
+        /* together: a list that is not there is not read.  Also: the columns of it - 1 are in place */
+        bad = bar_any(kBarW, kW, bad);
+        if (bad) break;
+      }
+      for (int k = 0; k < n_in; ++k) {
+        const ProjDev& J = s_proj[k];
+        const int C = J.C;
+        const Block B = block<kQW>(sm, L, k, M, C);
+        const TabRef& T = s_tab[k];
+        const int tlen = T.len;
+        const float kp = J.taupdt * prn;
+        for (int j = wt; j < M; j += kW) B.epsc[cur * M + j] = B.epsc[prev * M + j] * (1 - J.kepsc);
+        const int part = queue_part(C, kQW);
+        const uint16_t* l0 = B.list + cur * kQW * part;
+        const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
+        auto row_of = [&](int e) { return h * C + (int)(e < n0 ? l0[e] : l0[part + e - n0]); };
+        for (int base = 0; base < nrow; base += rch) {
+          const int nr = min(rch, nrow - base);
+          /* row traces (threads from the top of the group) beside the cells (from the bottom) */
+          for (int t = kW - 1 - wt; t < nr; t += kW) {
+            const int r = row_of(base + t);
+            if (r == 9) atomicOr(&net->ss_log[(size_t)it * net->n_projs + s_inp[k]], 1u);
+            const int pdt = simstep - J.ti[r];
+            const float4 tr = make_float4(J.pi[r], J.ei[r], J.zi[r], 0.0f);
+            if (pdt <= 0) {
+              J.zi[r] = tr.z + J.kfti;
+              J.ti[r] = simstep;
+              s_pi[t] = tr.x;
+            } else {
+              float4 A, Bt;
+              double2 R0, R1;
+              if (pdt < tlen) {
+                A = T.tab[(size_t)pdt * 4 + 2];
+                Bt = T.tab[(size_t)pdt * 4 + 3];
+                R0 = T.rtab[(size_t)pdt * 4 + 2];
+                R1 = T.rtab[(size_t)pdt * 4 + 3];
+              } else {
+                load_entry(T.tab, tlen, T.k, pdt, 2, A, Bt);
+                recip_part(A, Bt, 2, R0, R1);
+              }
+              const float4 rt = row_step_nl(tr, &T, A, Bt, R0, R1);
+              J.pi[r] = rt.x;
+              J.ei[r] = rt.y;
+              J.zi[r] = rt.z + J.kfti;
+              J.ti[r] = simstep;
+              s_pi[t] = rt.x;
+            }
+          }
+          for (int c = wt; c < nr * M; c += kW) {
+            const int rr = c / M, j = c - rr * M;
+            const size_t index = (size_t)row_of(base + rr) * M + j;
+            const int pdt = simstep - J.tij[index];
+            float4 q = J.cell[index];
+            const float wv = kp == 0.0f ? J.wij[index] : 0.0f;
+            if (pdt <= 0) {
+              q.z += J.kfti;
+              J.cell[index] = q;
+              J.tij[index] = simstep;
+              s_skip[c] = 1;
+            } else {
+              float4 A, Bt;
+              double2 R0, R1;
+              if (pdt < tlen) {
+                A = T.tab[(size_t)pdt * 4 + 0];
+                Bt = T.tab[(size_t)pdt * 4 + 1];
+                R0 = T.rtab[(size_t)pdt * 4 + 0];
+                R1 = T.rtab[(size_t)pdt * 4 + 1];
+              } else {
+                load_entry(T.tab, tlen, T.k, pdt, 0, A, Bt);
+                recip_part(A, Bt, 0, R0, R1);
+              }
+              q = cell_step_nl(q, &T, A, Bt, R0, R1);
+              q.z = q.z + J.kfti;
+              J.cell[index] = q;
+              J.tij[index] = simstep;
+              s_w[c] = kp == 0.0f ? wv : q.x;
+              s_skip[c] = 0;
+            }
+          }
+          bar(kBarW, kW);
+          /* weights, Proj.cpp:458-462; without plasticity they stay */
+          if (kp != 0.0f) {
+            for (int c = wt; c < nr * M; c += kW) {
+              if (s_skip[c]) continue;
+              const int rr = c / M, j = c - rr * M;
+              const float w = J.wgain * bx_logf((s_w[c] + J.eps2) / ((s_pi[rr] + J.eps) * (B.pjn[cur * M + j] + J.eps)));
+              J.wij[(size_t)row_of(base + rr) * M + j] = w;
+              s_w[c] = w;
+            }
+            bar(kBarW, kW);
+          }
+          for (int j = wt; j < M; j += kW) {
+            float e = B.epsc[cur * M + j];
+            for (int rr = 0; rr < nr; ++rr)
+              if (!s_skip[rr * M + j]) e += s_w[rr * M + j];
+            B.epsc[cur * M + j] = e;
+          }
+          if (base + rch < nrow || k + 1 < n_in) bar(kBarW, kW);
+        }
+        if (wt == 0) s_rows += (unsigned long long)nrow * M;
+      }
+      bar(kBarW, kW);
+      if (wt == 0) mb_arrive(s_E, it);
+      /* columns of this tick's spikes */
+      bad = !mb_wait(s_S, it, &s_abort, net->err);
+      if (!bad) {
+        uint32_t sp[kPW];
+        int nspk = 0;
+#pragma unroll
+        for (int w = 0; w < kPW; ++w) {
+          sp[w] = w * 32 < M ? s_spk[cur][w] : 0u;
+          nspk += __popc(sp[w]);
+        }
+        for (int k = 0; k < n_in && nspk > 0; ++k) {
+          const ProjDev& J = s_proj[k];
+          const int C = J.C;
+          const Block B = block<kQW>(sm, L, k, M, C);
+          const TabRef& T = s_tab[k];
+          const int tlen = T.len;
+          for (int i = 0; i < nspk; ++i) {
+            /* the i-th spiking MCU */
+            int left = i, j = 0;
+            uint32_t m = 0;
+#pragma unroll
+            for (int w = 0; w < kPW; ++w) {
+              const int c = __popc(sp[w]);
+              if (left >= 0 && left < c) {
+                m = sp[w];
+                for (; left > 0; --left) m &= m - 1;
+                j = w * 32 + __ffs(m) - 1;
+                left = -1;
+              } else if (left >= 0) {
+                left -= c;
+              }
+            }
+            for (int s0 = 0; s0 < C; s0 += kColU * kW) {
+              size_t index[kColU];
+              int tv[kColU];
+              float4 cv[kColU];
+              bool ok[kColU];
+#pragma unroll
+              for (int u = 0; u < kColU; ++u) {
+                const int s = s0 + u * kW + wt;
+                ok[u] = s < C && B.src[s < C ? s : 0] != 0xffffu;
+                index[u] = (size_t)(h * C + s) * M + j;
+                if (ok[u]) {
+                  tv[u] = J.tij[index[u]];
+                  cv[u] = J.cell[index[u]];
+                }
+              }
+              float4 tA[kColU], tB[kColU];
+              double2 tR0[kColU], tR1[kColU];
+#pragma unroll
+              for (int u = 0; u < kColU; ++u) {
+                const int pdt = simstep - tv[u];
+                if (ok[u] && pdt > 0 && pdt < tlen) {
+                  tA[u] = T.tab[(size_t)pdt * 4 + 0];
+                  tB[u] = T.tab[(size_t)pdt * 4 + 1];
+                  tR0[u] = T.rtab[(size_t)pdt * 4 + 0];
+                  tR1[u] = T.rtab[(size_t)pdt * 4 + 1];
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < kColU; ++u) {
+                if (!ok[u]) continue;
+                const int pdt = simstep - tv[u];
+                float4 q = cv[u];
+                if (pdt <= 0) {
+                  q.w += J.kftj;
+                } else {
+                  float4 A = tA[u], Bt = tB[u];
+                  double2 R0 = tR0[u], R1 = tR1[u];
+                  if (pdt >= tlen) {
+                    load_entry(T.tab, tlen, T.k, pdt, 0, A, Bt);
+                    recip_part(A, Bt, 0, R0, R1);
+                  }
+                  q = cell_step_nl(q, &T, A, Bt, R0, R1);
+                  q.w = q.w + J.kftj;
+                }
+                J.cell[index[u]] = q;
+                J.tij[index[u]] = simstep;
+              }
+            }
+          }
+          if (wt == 0) s_cols += (unsigned long long)nspk * C;
+        }
+      }
+    }
+    bar(0, kThreads);
+  }
+
+  /* ---- the state back to the buffers of the last tick.  Q has seen every
+     CTA's words of the tick before the last, so no CTA still reads what the
+     launch began with (its first softmax seed, the spikes before it) ---- */
+  if (s_abort) return;
+  if (tid == 0) {
+    if (s_rows) atomicAdd(&net->counters[0], s_rows);
+    if (s_cols) atomicAdd(&net->counters[1], s_cols);
+  }
+  const int last = (rp->k0 + n_ticks - 1) & 1, next = last ^ 1;
+  for (int k = 0; k < n_in; ++k) {
+    const ProjDev& J = s_proj[k];
+    const Block B = block<kQW>(sm, L, k, M, J.C);
+    const size_t eoff = (size_t)J.proj_in_pop * n;
+    for (int j = tid; j < M; j += kThreads) {
+      const int idx = h * M + j;
+      J.pj[idx] = B.pj[j];
+      J.ej[idx] = B.ej[j];
+      J.zj[idx] = B.zj[j];
+      pop.epsc[last][eoff + idx] = B.epsc[last * M + j];
+      pop.bj[last][eoff + idx] = B.bj[j];
+    }
+    for (int s = tid; s < J.C; s += kThreads)
+      if (B.src[s] != 0xffffu) J.qi[h * J.C + s] = (int)B.qi[s];
+    const int part = queue_part(J.C, kQW), n0 = s_nl[k][next][0];
+    const int cnt = kQW > 1 ? n0 + s_nl[k][next][kQW - 1] : n0;
+    const uint16_t* l = B.list + next * kQW * part;
+    for (int e = tid; e < cnt; e += kThreads) J.list[h * J.C + e] = h * J.C + (int)(e < n0 ? l[e] : l[part + e - n0]);
+    if (tid == 0) J.list_cnt[h] = cnt;
+  }
+}
+
+/* dynamic shared memory, in bytes, for the network's populations; kQW queue warps, `cells` per chunk */
+inline size_t smem_bytes(int M, int n_in, const int* C, int n_words, int cells, int qw) {
+  Layout L;
+  layout(M, n_in, C, n_words, cells, qw, L);
+  return (size_t)L.total * 4;
+}
+
+}  // namespace flow
+}  // namespace bcpnn
+
+#endif /* BCPNN_FLOW_CUH */
