@@ -14,9 +14,13 @@
  *         columns  Proj.cpp:481-536, 722-760: the spikes of t, after its rows;
  *   Q(t)  delay queue  Proj.cpp:621-630, 645-664: the spikes of t-1 of every
  *         source HCU; it lists the active rows of t+1.
- * So three groups of warps run side by side and meet at shared-memory
- * mbarriers: E(t) (W -> P, Q: epsc(t), and the lists of t are free), S(t) (P ->
- * W: spikes of t, pj(t+1)), L(t+1) (Q -> W: the active rows of t+1).  A CTA
+ * The row traces (Proj.cpp:397-416) belong to the rows alone, so a warp of its
+ * own, R(t), does those of the listed rows beside the decays of their cells.
+ * The four groups run side by side and meet at shared-memory mbarriers: E(t) (W
+ * -> P, Q: epsc(t), and the lists of t are free), S(t) (P -> W: spikes of t,
+ * pj(t+1)), L(t+1) (Q -> W, R: the active rows of t+1), T(t) (R -> W: their new
+ * pi).  A cell's thread goes from its decay to its weight without a barrier; one
+ * barrier before the ordered sum is the only one of the rows.  A CTA
  * whose HCU spikes does its whole columns itself while its next population
  * update runs; only its rows of t+1 wait, and through them its P(t+2).
  *
@@ -29,9 +33,10 @@
  *
  * Bound by the longest cycle of dependences: P(t) -> columns(t) -> rows(t+1) ->
  * P(t+2) takes two ticks, E(t-1) -> P(t) one.  Per tick, against tick_kernel with
- * its grid barrier and its columns spread over the grid: 10 x 10 2.88 us (7.4),
- * 50 x 50 3.77 (8.8), 100 x 100 with C = 1000 6.18 (9.9), 256 x 50 with C = 1000
- * 10.4 (13.8), 296 x 20 with C = 400 6.2 (11.3).  The decays and their exact
+ * its grid barrier and its columns spread over the grid: 10 x 10 2.4 us (7.4),
+ * 50 x 50 2.9 (8.8), 100 x 100 with C = 1000 4.5 (9.9), 256 x 50 with C = 1000
+ * 7.8 (13.8), 296 x 20 with C = 400 4.7 (11.3).  With the row traces in W and two
+ * more barriers before the sum, decays as calls: 2.8, 3.7, 6.0, 9.7 and 5.7.  The decays and their exact
  * division are those of bcpnn_device.cuh, so every value is bit-identical to
  * tick_kernel's and to the oracle's.
  *
@@ -72,9 +77,9 @@ __device__ __forceinline__ unsigned long long now_ns() {
    is told by its parity; no group falls more than two behind). */
 constexpr int kEventTicks = 4;
 
-__device__ __forceinline__ void mb_init(unsigned long long* ev) {
+__device__ __forceinline__ void mb_init(unsigned long long* ev, int arrivals) {
   for (int k = 0; k < kEventTicks; ++k)
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(ev + k)) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(ev + k)), "r"(arrivals) : "memory");
 }
 
 __device__ __forceinline__ void mb_arrive(unsigned long long* ev, int k) {
@@ -159,13 +164,38 @@ __device__ __forceinline__ bool bar_any(int id, int n, bool flag) {
   return r != 0;
 }
 
+/* one decay of a cell (row traces) on the float closed-form path, in line; the
+   exact fallback and the FP64-built propagators out of line */
+__device__ __forceinline__ float4 cell_step(float4 c, const TabRef& T, float4 A, float4 B, double2 R0, double2 R1) {
+  float4 f = c;
+  if (!T.k.fp64 && cell_decay_fast(f, T.k, T.rk, A, B, R0, R1)) return f;
+  return cell_step_nl(c, &T, A, B, R0, R1);
+}
+
+__device__ __forceinline__ float4 row_step(float4 r, const TabRef& T, float4 A, float4 B, double2 R0, double2 R1) {
+  float4 f = r;
+  if (!T.k.fp64 && row_decay_fast(f, T.k, T.rk, A, B, R0, R1)) return f;
+  return row_step_nl(r, &T, A, B, R0, R1);
+}
+
+/* part 0 (cells) or 2 (rows) of the table entry of pdt > 0 elapsed ticks */
+__device__ __forceinline__ void entry(const TabRef& T, int pdt, int part, float4& A, float4& B, double2& R0, double2& R1) {
+  if (pdt < T.len) {
+    A = T.tab[(size_t)pdt * 4 + part];
+    B = T.tab[(size_t)pdt * 4 + part + 1];
+    R0 = T.rtab[(size_t)pdt * 4 + part];
+    R1 = T.rtab[(size_t)pdt * 4 + part + 1];
+  } else {
+    load_entry(T.tab, T.len, T.k, pdt, part, A, B);
+    recip_part(A, B, part, R0, R1);
+  }
+}
+
 /* shared-memory layout of a CTA, in 4-byte words */
 struct Layout {
   int act;                 /* [M rounded up to 4] */
   int bits;                /* [n_words] the previous tick's spikes of the network */
-  int pi;                  /* [rows of a chunk] */
-  int w;                   /* [chunk cells] */
-  int skip;                /* bytes [chunk cells] */
+  int w;                   /* [chunk cells] weights to add */
   int q[kMaxIn];           /* blocks of the incoming projections */
   int total;
 };
@@ -173,10 +203,10 @@ struct Layout {
 /* slots per queue warp, a multiple of 32 */
 __host__ __device__ inline int queue_part(int C, int qw) { return ((C + qw - 1) / qw + 31) & ~31; }
 
-/* a projection's block: pj ej zj bj [M], epsc [2][M], pjn [2][M]; qi [C]; then 16-bit list [2][qw * part], src [C]; bytes
-   di [C] */
+/* a projection's block: pj ej zj bj [M], epsc [2][M], pjn [2][M]; qi [C], pi [2][C] (by list entry); then 16-bit list
+   [2][qw * part], src [C]; bytes di [C] */
 __host__ __device__ inline int block_words(int M, int C, int qw) {
-  return 8 * M + C + (2 * qw * queue_part(C, qw) + C + 1) / 2 + (C + 3) / 4;
+  return 8 * M + 3 * C + (2 * qw * queue_part(C, qw) + C + 1) / 2 + (C + 3) / 4;
 }
 
 __host__ __device__ inline int chunk_rows(int M, int cells) { return cells / M < 1 ? 1 : cells / M; }
@@ -187,9 +217,7 @@ __host__ __device__ inline void layout(int M, int n_in, const int* C, int n_word
   L.bits = o; o += (n_words + 3) & ~3;
   const int rows = chunk_rows(M, cells);
   const int n = rows * M > cells ? rows * M : cells;
-  L.pi = o; o += rows;
   L.w = o; o += n;
-  L.skip = o; o += (n + 3) / 4;
   for (int k = 0; k < kMaxIn; ++k) {
     L.q[k] = o;
     if (k < n_in) o += block_words(M, C[k], qw);
@@ -198,7 +226,7 @@ __host__ __device__ inline void layout(int M, int n_in, const int* C, int n_word
 }
 
 struct Block {
-  float *pj, *ej, *zj, *bj, *epsc, *pjn;
+  float *pj, *ej, *zj, *bj, *epsc, *pjn, *pi;
   uint32_t* qi;
   uint16_t *list, *src;
   uint8_t* di;
@@ -215,7 +243,8 @@ __device__ __forceinline__ Block block(float* sm, const Layout& L, int k, int M,
   b.epsc = f + 4 * M;
   b.pjn = f + 6 * M;
   b.qi = (uint32_t*)(f + 8 * M);
-  b.list = (uint16_t*)(b.qi + C);
+  b.pi = f + 8 * M + C;
+  b.list = (uint16_t*)(b.pi + 2 * C);
   b.src = b.list + 2 * kQW * queue_part(C, kQW);
   b.di = (uint8_t*)((uint32_t*)b.list + (2 * kQW * queue_part(C, kQW) + C + 1) / 2);
   return b;
@@ -226,12 +255,12 @@ constexpr int kBarP = 1, kBarW = 2, kBarQ = 3;
    by tick parity; else bit 6 is the source's spike before the launch */
 constexpr int kUnfed = 32;
 
-/* kThreads: 512 (one CTA per SM) or 256 (two); kPW warps of population update (M <= 32 kPW), kQW of delay queue, the
-   others rows and columns */
+/* kThreads: 512 (one CTA per SM) or 256 (two); kPW warps of population update (M <= 32 kPW), kQW of delay queue, one of
+   row traces, the others rows and columns */
 template <int kThreads, int kPW, int kQW>
 __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     flow_kernel(const NetDev* __restrict__ net_g, const RunParams* __restrict__ rp_g, Args fa, int n_ticks) {
-  constexpr int kP = kPW * 32, kQ = kQW * 32, kW = kThreads - kP - kQ;
+  constexpr int kP = kPW * 32, kQ = kQW * 32, kW = kThreads - kP - kQ - 32;
   constexpr int kCells = kThreads; /* row cells of one chunk */
   extern __shared__ __align__(16) float sm[];
   __shared__ NetDev s_net;
@@ -241,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
   __shared__ TabRef s_tab[kMaxIn];
   __shared__ int s_inp[kMaxIn], s_srcM[kMaxIn], s_src0[kMaxIn], s_fed[kMaxIn];
   __shared__ Layout s_L;
-  __shared__ unsigned long long s_E[kEventTicks], s_S[kEventTicks], s_Lst[kEventTicks];
+  __shared__ unsigned long long s_E[kEventTicks], s_S[kEventTicks], s_Lst[kEventTicks], s_T[kEventTicks];
   __shared__ int s_abort;
   __shared__ int s_nl[kMaxIn][2][kQW]; /* list lengths by tick parity */
   __shared__ uint32_t s_spk[2][kPW];   /* spikes of this HCU by tick parity */
@@ -255,9 +284,10 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     s_rp = *rp_g;
     s_abort = 0;
     s_rows = s_cols = 0;
-    mb_init(s_E);
-    mb_init(s_S);
-    mb_init(s_Lst);
+    mb_init(s_E, kW / 32);
+    mb_init(s_S, 1);
+    mb_init(s_Lst, 1);
+    mb_init(s_T, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -595,12 +625,51 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       if (bad) break;
     }
     bar(0, kThreads);
+  } else if (tid < kP + kQ + 32) {
+    /* ================= R: row traces ================= */
+    const int lane = tid & 31;
+    bool bad = false;
+    for (int it = 0; it < n_ticks; ++it) {
+      const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1;
+      if (it > 0) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err);
+      if (__any_sync(0xffffffffu, bad)) break;
+      for (int k = 0; k < n_in; ++k) {
+        const ProjDev& J = s_proj[k];
+        const Block B = block<kQW>(sm, L, k, M, J.C);
+        const TabRef& T = s_tab[k];
+        const int part = queue_part(J.C, kQW);
+        const uint16_t* l0 = B.list + cur * kQW * part;
+        const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
+        for (int e = lane; e < nrow; e += 32) {
+          const int r = h * J.C + (int)(e < n0 ? l0[e] : l0[part + e - n0]);
+          if (r == 9) atomicOr(&net->ss_log[(size_t)it * net->n_projs + s_inp[k]], 1u);
+          const int pdt = simstep - J.ti[r];
+          const float4 tr = make_float4(J.pi[r], J.ei[r], J.zi[r], 0.0f);
+          float pi = tr.x;
+          if (pdt <= 0) {
+            J.zi[r] = tr.z + J.kfti;
+          } else {
+            float4 A, Bt;
+            double2 R0, R1;
+            entry(T, pdt, 2, A, Bt, R0, R1);
+            const float4 rt = row_step(tr, T, A, Bt, R0, R1);
+            pi = rt.x;
+            J.pi[r] = pi;
+            J.ei[r] = rt.y;
+            J.zi[r] = rt.z + J.kfti;
+          }
+          J.ti[r] = simstep;
+          B.pi[cur * J.C + e] = pi;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mb_arrive(s_T, it);
+    }
+    bar(0, kThreads);
   } else {
     /* ================= W: rows, columns ================= */
-    const int wt = tid - kP - kQ;
-    float* s_pi = sm + L.pi;
+    const int wt = tid - kP - kQ - 32, lane = tid & 31;
     float* s_w = sm + L.w;
-    int8_t* s_skip = (int8_t*)(sm + L.skip);
     const int rch = chunk_rows(M, kCells);
     bool bad = false;
     for (int it = 0; it < n_ticks; ++it) {
@@ -611,107 +680,63 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         bad = bar_any(kBarW, kW, bad);
         if (bad) break;
       }
+      bool traces = false;
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
         const int C = J.C;
         const Block B = block<kQW>(sm, L, k, M, C);
         const TabRef& T = s_tab[k];
-        const int tlen = T.len;
         const float kp = J.taupdt * prn;
-        for (int j = wt; j < M; j += kW) B.epsc[cur * M + j] = B.epsc[prev * M + j] * (1 - J.kepsc);
         const int part = queue_part(C, kQW);
         const uint16_t* l0 = B.list + cur * kQW * part;
         const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
-        auto row_of = [&](int e) { return h * C + (int)(e < n0 ? l0[e] : l0[part + e - n0]); };
+        if (nrow == 0)
+          for (int j = wt; j < M; j += kW) B.epsc[cur * M + j] = B.epsc[prev * M + j] * (1 - J.kepsc);
         for (int base = 0; base < nrow; base += rch) {
           const int nr = min(rch, nrow - base);
-          /* row traces (threads from the top of the group) beside the cells (from the bottom) */
-          for (int t = kW - 1 - wt; t < nr; t += kW) {
-            const int r = row_of(base + t);
-            if (r == 9) atomicOr(&net->ss_log[(size_t)it * net->n_projs + s_inp[k]], 1u);
-            const int pdt = simstep - J.ti[r];
-            const float4 tr = make_float4(J.pi[r], J.ei[r], J.zi[r], 0.0f);
-            if (pdt <= 0) {
-              J.zi[r] = tr.z + J.kfti;
-              J.ti[r] = simstep;
-              s_pi[t] = tr.x;
-            } else {
-              float4 A, Bt;
-              double2 R0, R1;
-              if (pdt < tlen) {
-                A = T.tab[(size_t)pdt * 4 + 2];
-                Bt = T.tab[(size_t)pdt * 4 + 3];
-                R0 = T.rtab[(size_t)pdt * 4 + 2];
-                R1 = T.rtab[(size_t)pdt * 4 + 3];
-              } else {
-                load_entry(T.tab, tlen, T.k, pdt, 2, A, Bt);
-                recip_part(A, Bt, 2, R0, R1);
-              }
-              const float4 rt = row_step_nl(tr, &T, A, Bt, R0, R1);
-              J.pi[r] = rt.x;
-              J.ei[r] = rt.y;
-              J.zi[r] = rt.z + J.kfti;
-              J.ti[r] = simstep;
-              s_pi[t] = rt.x;
-            }
-          }
           for (int c = wt; c < nr * M; c += kW) {
-            const int rr = c / M, j = c - rr * M;
-            const size_t index = (size_t)row_of(base + rr) * M + j;
+            const int rr = c / M, j = c - rr * M, e = base + rr;
+            const size_t index = (size_t)(h * C + (int)(e < n0 ? l0[e] : l0[part + e - n0])) * M + j;
             const int pdt = simstep - J.tij[index];
             float4 q = J.cell[index];
-            const float wv = kp == 0.0f ? J.wij[index] : 0.0f;
+            float w = kp == 0.0f ? J.wij[index] : 0.0f; /* without plasticity the weights stay */
             if (pdt <= 0) {
               q.z += J.kfti;
-              J.cell[index] = q;
-              J.tij[index] = simstep;
-              s_skip[c] = 1;
+              w = -0.0f; /* adds nothing, to any sum */
             } else {
               float4 A, Bt;
               double2 R0, R1;
-              if (pdt < tlen) {
-                A = T.tab[(size_t)pdt * 4 + 0];
-                Bt = T.tab[(size_t)pdt * 4 + 1];
-                R0 = T.rtab[(size_t)pdt * 4 + 0];
-                R1 = T.rtab[(size_t)pdt * 4 + 1];
-              } else {
-                load_entry(T.tab, tlen, T.k, pdt, 0, A, Bt);
-                recip_part(A, Bt, 0, R0, R1);
-              }
-              q = cell_step_nl(q, &T, A, Bt, R0, R1);
+              entry(T, pdt, 0, A, Bt, R0, R1);
+              q = cell_step(q, T, A, Bt, R0, R1);
               q.z = q.z + J.kfti;
-              J.cell[index] = q;
-              J.tij[index] = simstep;
-              s_w[c] = kp == 0.0f ? wv : q.x;
-              s_skip[c] = 0;
+              if (kp != 0.0f) { /* Proj.cpp:458-462 */
+                if (!traces) {
+                  if (!mb_wait(s_T, it, &s_abort, net->err)) bad = true;
+                  traces = true;
+                }
+                w = J.wgain * bx_logf((q.x + J.eps2) / ((B.pi[cur * C + e] + J.eps) * (B.pjn[cur * M + j] + J.eps)));
+                J.wij[index] = w;
+              }
             }
+            J.cell[index] = q;
+            J.tij[index] = simstep;
+            s_w[c] = w;
           }
           bar(kBarW, kW);
-          /* weights, Proj.cpp:458-462; without plasticity they stay */
-          if (kp != 0.0f) {
-            for (int c = wt; c < nr * M; c += kW) {
-              if (s_skip[c]) continue;
-              const int rr = c / M, j = c - rr * M;
-              const float w = J.wgain * bx_logf((s_w[c] + J.eps2) / ((s_pi[rr] + J.eps) * (B.pjn[cur * M + j] + J.eps)));
-              J.wij[(size_t)row_of(base + rr) * M + j] = w;
-              s_w[c] = w;
-            }
-            bar(kBarW, kW);
-          }
+          /* epsc in row order */
           for (int j = wt; j < M; j += kW) {
-            float e = B.epsc[cur * M + j];
-            for (int rr = 0; rr < nr; ++rr)
-              if (!s_skip[rr * M + j]) e += s_w[rr * M + j];
+            float e = base == 0 ? B.epsc[prev * M + j] * (1 - J.kepsc) : B.epsc[cur * M + j];
+            for (int rr = 0; rr < nr; ++rr) e += s_w[rr * M + j];
             B.epsc[cur * M + j] = e;
           }
           if (base + rch < nrow || k + 1 < n_in) bar(kBarW, kW);
         }
         if (wt == 0) s_rows += (unsigned long long)nrow * M;
       }
-      bar(kBarW, kW);
-      if (wt == 0) mb_arrive(s_E, it);
+      __syncwarp();
+      if (lane == 0) mb_arrive(s_E, it);
       /* columns of this tick's spikes */
-      bad = !mb_wait(s_S, it, &s_abort, net->err);
+      if (!bad) bad = !mb_wait(s_S, it, &s_abort, net->err);
       if (!bad) {
         uint32_t sp[kPW];
         int nspk = 0;
@@ -725,72 +750,41 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           const int C = J.C;
           const Block B = block<kQW>(sm, L, k, M, C);
           const TabRef& T = s_tab[k];
-          const int tlen = T.len;
-          for (int i = 0; i < nspk; ++i) {
-            /* the i-th spiking MCU */
-            int left = i, j = 0;
-            uint32_t m = 0;
+#pragma unroll 1
+          for (int w = 0; w < kPW; ++w)
+            for (uint32_t m = s_spk[cur][w]; m && w * 32 < M; m &= m - 1) {
+              const int j = w * 32 + __ffs(m) - 1;
+              float4* const cell = J.cell + (size_t)h * C * M + j;
+              int* const tij = J.tij + (size_t)h * C * M + j;
+              /* kColU cells of a thread at a time, their loads together */
+              for (int s0 = wt; s0 < C; s0 += kColU * kW) {
+                int pdt[kColU];
+                float4 cv[kColU], A[kColU], Bt[kColU];
+                double2 R0[kColU], R1[kColU];
 #pragma unroll
-            for (int w = 0; w < kPW; ++w) {
-              const int c = __popc(sp[w]);
-              if (left >= 0 && left < c) {
-                m = sp[w];
-                for (; left > 0; --left) m &= m - 1;
-                j = w * 32 + __ffs(m) - 1;
-                left = -1;
-              } else if (left >= 0) {
-                left -= c;
-              }
-            }
-            for (int s0 = 0; s0 < C; s0 += kColU * kW) {
-              size_t index[kColU];
-              int tv[kColU];
-              float4 cv[kColU];
-              bool ok[kColU];
-#pragma unroll
-              for (int u = 0; u < kColU; ++u) {
-                const int s = s0 + u * kW + wt;
-                ok[u] = s < C && B.src[s < C ? s : 0] != 0xffffu;
-                index[u] = (size_t)(h * C + s) * M + j;
-                if (ok[u]) {
-                  tv[u] = J.tij[index[u]];
-                  cv[u] = J.cell[index[u]];
-                }
-              }
-              float4 tA[kColU], tB[kColU];
-              double2 tR0[kColU], tR1[kColU];
-#pragma unroll
-              for (int u = 0; u < kColU; ++u) {
-                const int pdt = simstep - tv[u];
-                if (ok[u] && pdt > 0 && pdt < tlen) {
-                  tA[u] = T.tab[(size_t)pdt * 4 + 0];
-                  tB[u] = T.tab[(size_t)pdt * 4 + 1];
-                  tR0[u] = T.rtab[(size_t)pdt * 4 + 0];
-                  tR1[u] = T.rtab[(size_t)pdt * 4 + 1];
-                }
-              }
-#pragma unroll
-              for (int u = 0; u < kColU; ++u) {
-                if (!ok[u]) continue;
-                const int pdt = simstep - tv[u];
-                float4 q = cv[u];
-                if (pdt <= 0) {
-                  q.w += J.kftj;
-                } else {
-                  float4 A = tA[u], Bt = tB[u];
-                  double2 R0 = tR0[u], R1 = tR1[u];
-                  if (pdt >= tlen) {
-                    load_entry(T.tab, tlen, T.k, pdt, 0, A, Bt);
-                    recip_part(A, Bt, 0, R0, R1);
+                for (int u = 0; u < kColU; ++u) {
+                  const int s = s0 + u * kW;
+                  pdt[u] = -1;
+                  if (s < C && B.src[s] != 0xffffu) {
+                    pdt[u] = max(simstep - tij[(size_t)s * M], 0);
+                    cv[u] = cell[(size_t)s * M];
                   }
-                  q = cell_step_nl(q, &T, A, Bt, R0, R1);
-                  q.w = q.w + J.kftj;
                 }
-                J.cell[index[u]] = q;
-                J.tij[index[u]] = simstep;
+#pragma unroll
+                for (int u = 0; u < kColU; ++u)
+                  if (pdt[u] > 0) entry(T, pdt[u], 0, A[u], Bt[u], R0[u], R1[u]);
+#pragma unroll
+                for (int u = 0; u < kColU; ++u) {
+                  if (pdt[u] < 0) continue;
+                  float4 q = cv[u];
+                  if (pdt[u] > 0) q = cell_step(q, T, A[u], Bt[u], R0[u], R1[u]);
+                  q.w += J.kftj;
+                  const size_t at = (size_t)(s0 + u * kW) * M;
+                  cell[at] = q;
+                  tij[at] = simstep;
+                }
               }
             }
-          }
           if (wt == 0) s_cols += (unsigned long long)nspk * C;
         }
       }
