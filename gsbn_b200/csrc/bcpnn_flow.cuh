@@ -33,9 +33,9 @@
  *
  * Bound by the longest cycle of dependences: P(t) -> columns(t) -> rows(t+1) ->
  * P(t+2) takes two ticks, E(t-1) -> P(t) one.  Per tick, against tick_kernel with
- * its grid barrier and its columns spread over the grid: 10 x 10 2.4 us (7.4),
+ * its grid barrier and its columns spread over the grid: 10 x 10 2.2 us (7.4),
  * 50 x 50 2.9 (8.8), 100 x 100 with C = 1000 4.5 (9.9), 256 x 50 with C = 1000
- * 7.8 (13.8), 296 x 20 with C = 400 4.7 (11.3).  With the row traces in W and two
+ * 7.4 (13.8), 296 x 20 with C = 400 3.8 (11.3).  With the row traces in W and two
  * more barriers before the sum, decays as calls: 2.8, 3.7, 6.0, 9.7 and 5.7.  The decays and their exact
  * division are those of bcpnn_device.cuh, so every value is bit-identical to
  * tick_kernel's and to the oracle's.
@@ -178,6 +178,20 @@ __device__ __forceinline__ float4 row_step(float4 r, const TabRef& T, float4 A, 
   return row_step_nl(r, &T, A, B, R0, R1);
 }
 
+/* an entry beyond the table, computed; out of line, it is never needed while
+   the tables cover a run */
+struct Entry {
+  float4 A, B;
+  double2 R0, R1;
+};
+
+__device__ __noinline__ Entry entry_beyond(const TabRef& T, int pdt, int part) {
+  Entry e;
+  load_entry(T.tab, T.len, T.k, pdt, part, e.A, e.B);
+  recip_part(e.A, e.B, part, e.R0, e.R1);
+  return e;
+}
+
 /* part 0 (cells) or 2 (rows) of the table entry of pdt > 0 elapsed ticks */
 __device__ __forceinline__ void entry(const TabRef& T, int pdt, int part, float4& A, float4& B, double2& R0, double2& R1) {
   if (pdt < T.len) {
@@ -186,8 +200,11 @@ __device__ __forceinline__ void entry(const TabRef& T, int pdt, int part, float4
     R0 = T.rtab[(size_t)pdt * 4 + part];
     R1 = T.rtab[(size_t)pdt * 4 + part + 1];
   } else {
-    load_entry(T.tab, T.len, T.k, pdt, part, A, B);
-    recip_part(A, B, part, R0, R1);
+    const Entry e = entry_beyond(T, pdt, part);
+    A = e.A;
+    B = e.B;
+    R0 = e.R0;
+    R1 = e.R1;
   }
 }
 
@@ -255,7 +272,12 @@ constexpr int kBarP = 1, kBarW = 2, kBarQ = 3;
    by tick parity; else bit 6 is the source's spike before the launch */
 constexpr int kUnfed = 32;
 
-/* kThreads: 512 (one CTA per SM) or 256 (two); kPW warps of population update (M <= 32 kPW), kQW of delay queue, one of
+/* The loops of a tick are not unrolled: the four groups run through all of their
+   code every tick, one dependent instruction after the other, and what does not
+   stay in the instruction caches is fetched again each time (296 x 20, C = 400:
+   4.7 -> 3.8 us per tick, 10 x 10: 2.4 -> 2.2).
+
+   kThreads: 512 (one CTA per SM) or 256 (two); kPW warps of population update (M <= 32 kPW), kQW of delay queue, one of
    row traces, the others rows and columns */
 template <int kThreads, int kPW, int kQW>
 __global__ void __launch_bounds__(kThreads, 512 / kThreads)
@@ -307,6 +329,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     s_srcM[tid] = src.M;
     s_src0[tid] = fa.word0[s_proj[tid].src];
     int fed = 0;
+#pragma unroll 1
     for (int k = 0; k < src.n_out; ++k) fed |= src.out_proj[k] == p;
     s_fed[tid] = fed;
   }
@@ -325,11 +348,13 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
   /* ---- load the state the previous tick left ---- */
   const int cur0 = rp->k0 & 1, prev0 = cur0 ^ 1;
   const float prn = rp->prn;
+#pragma unroll 1
   for (int k = 0; k < n_in; ++k) {
     const ProjDev& J = s_proj[k];
     Block B = block<kQW>(sm, L, k, M, J.C);
     const size_t eoff = (size_t)J.proj_in_pop * n;
     const float kp = J.taupdt * prn;
+#pragma unroll 1
     for (int j = tid; j < M; j += kThreads) {
       const int idx = h * M + j;
       const float pj = J.pj[idx], ej = J.ej[idx];
@@ -340,6 +365,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       B.epsc[prev0 * M + j] = pop.epsc[prev0][eoff + idx];
       B.pjn[cur0 * M + j] = pj + (ej - pj) * kp;
     }
+#pragma unroll 1
     for (int s = tid; s < J.C; s += kThreads) {
       const int r = h * J.C + s, ii = J.ii[r];
       uint32_t src = 0xffffu, di = 0;
@@ -369,6 +395,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       n0 = lo;
     }
     if (tid < kQW) s_nl[k][cur0][tid] = tid == 0 ? n0 : cnt - n0;
+#pragma unroll 1
     for (int e = tid; e < cnt; e += kThreads)
       B.list[cur0 * kQW * part + (e < n0 ? e : part + e - n0)] = (uint16_t)(rows[e] - h * J.C);
   }
@@ -387,6 +414,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     const int wph = (M + 31) >> 5;
     const float pr = net->poisson_hz * net->dt;
     bool bad = false;
+#pragma unroll 1
     for (int it = 0; it < n_ticks; ++it) {
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1, prev = cur ^ 1;
       const uint32_t tag = rp->serial0 + (uint32_t)it;
@@ -401,6 +429,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       float sup = pop.lgbias + pop.igain * lg + noise;
       if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
       float wsup = 0.0f;
+#pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const Block B = block<kQW>(sm, L, k, M, s_proj[k].C);
         if (active) wsup += B.bj[j] + B.epsc[prev * M + j];
@@ -419,6 +448,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         if (it == 0) {
           float ws = 0.0f;
           int offset = 0;
+#pragma unroll 1
           for (int m = 0; m < pop.dim_proj; m++) {
             ws += __ldcg(pop.bj[prev] + offset) + __ldcg(pop.epsc[prev] + offset);
             offset += n;
@@ -436,6 +466,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         }
       }
       /* pj of the next tick (Proj.cpp:340: it takes ej and pj only); its buffer is free, the rows that read it are done */
+#pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
         const Block B = block<kQW>(sm, L, k, M, J.C);
@@ -480,6 +511,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       {
         const float4* v = (const float4*)s_act;
         float4 x = v[0];
+#pragma unroll 1
         for (int m = 4; m < M; m += 4) {
           const float4 y = v[m >> 2];
           vsum += x.x;
@@ -514,8 +546,10 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       if (spk) {
         atomicOr(&pop.spk_log[(size_t)it * pop.log_words + (idx >> 5)], 1u << (idx & 31));
         if (idx == 9)
+#pragma unroll 1
           for (int k = 0; k < n_in; ++k) atomicOr(&net->ss_log[(size_t)it * net->n_projs + s_inp[k]], 2u);
       }
+#pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
         const Block B = block<kQW>(sm, L, k, M, J.C);
@@ -536,17 +570,20 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       pop.act[idx] = act;
       pop.counter[idx] = cnt;
       pop.spike[idx] = spk ? 1 : 0;
+#pragma unroll 1
       for (int k = 0; k < pop.n_out; ++k) net->projs[pop.out_proj[k]].si[last][idx] = spk ? 1 : 0;
     }
   } else if (tid < kP + kQ) {
     /* ================= Q: spike words, delay queue ================= */
     const int qt = tid - kP, warp = qt >> 5, lane = qt & 31;
     bool bad = false;
+#pragma unroll 1
     for (int it = 0; it < n_ticks; ++it) {
       const int cur = (rp->k0 + it) & 1, prev = cur ^ 1, nxt = prev;
       if (it > 0) {
         const uint32_t tag = rp->serial0 + (uint32_t)(it - 1);
         const unsigned long long* w = fa.words + (size_t)(tag & (kWordTicks - 1)) * fa.n_words;
+#pragma unroll 1
         for (int x0 = 0; x0 < fa.n_words; x0 += 4 * kQ) {
           /* four words' loads at once; the late ones are polled */
           unsigned long long v[4];
@@ -570,6 +607,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       }
       if (kQW > 1) bar(kBarQ, kQ);
       else __syncwarp();
+#pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
         const int C = J.C;
@@ -578,6 +616,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         uint16_t* out = B.list + (nxt * kQW + warp) * part;
         const int s1 = min(C, (warp + 1) * part);
         int total = 0;
+#pragma unroll 1
         for (int s0 = warp * part; s0 < s1; s0 += 128) {
           uint32_t src[4], di[4], qv[4];
           bool on[4];
@@ -629,10 +668,12 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     /* ================= R: row traces ================= */
     const int lane = tid & 31;
     bool bad = false;
+#pragma unroll 1
     for (int it = 0; it < n_ticks; ++it) {
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1;
       if (it > 0) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err);
       if (__any_sync(0xffffffffu, bad)) break;
+#pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
         const Block B = block<kQW>(sm, L, k, M, J.C);
@@ -640,6 +681,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         const int part = queue_part(J.C, kQW);
         const uint16_t* l0 = B.list + cur * kQW * part;
         const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
+#pragma unroll 1
         for (int e = lane; e < nrow; e += 32) {
           const int r = h * J.C + (int)(e < n0 ? l0[e] : l0[part + e - n0]);
           if (r == 9) atomicOr(&net->ss_log[(size_t)it * net->n_projs + s_inp[k]], 1u);
@@ -672,6 +714,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     float* s_w = sm + L.w;
     const int rch = chunk_rows(M, kCells);
     bool bad = false;
+#pragma unroll 1
     for (int it = 0; it < n_ticks; ++it) {
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1, prev = cur ^ 1;
       if (it > 0) {
@@ -681,6 +724,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         if (bad) break;
       }
       bool traces = false;
+#pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
         const int C = J.C;
@@ -691,9 +735,12 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         const uint16_t* l0 = B.list + cur * kQW * part;
         const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
         if (nrow == 0)
+#pragma unroll 1
           for (int j = wt; j < M; j += kW) B.epsc[cur * M + j] = B.epsc[prev * M + j] * (1 - J.kepsc);
+#pragma unroll 1
         for (int base = 0; base < nrow; base += rch) {
           const int nr = min(rch, nrow - base);
+#pragma unroll 1
           for (int c = wt; c < nr * M; c += kW) {
             const int rr = c / M, j = c - rr * M, e = base + rr;
             const size_t index = (size_t)(h * C + (int)(e < n0 ? l0[e] : l0[part + e - n0])) * M + j;
@@ -724,8 +771,10 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           }
           bar(kBarW, kW);
           /* epsc in row order */
+#pragma unroll 1
           for (int j = wt; j < M; j += kW) {
             float e = base == 0 ? B.epsc[prev * M + j] * (1 - J.kepsc) : B.epsc[cur * M + j];
+#pragma unroll 1
             for (int rr = 0; rr < nr; ++rr) e += s_w[rr * M + j];
             B.epsc[cur * M + j] = e;
           }
@@ -745,6 +794,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           sp[w] = w * 32 < M ? s_spk[cur][w] : 0u;
           nspk += __popc(sp[w]);
         }
+#pragma unroll 1
         for (int k = 0; k < n_in && nspk > 0; ++k) {
           const ProjDev& J = s_proj[k];
           const int C = J.C;
@@ -752,11 +802,13 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           const TabRef& T = s_tab[k];
 #pragma unroll 1
           for (int w = 0; w < kPW; ++w)
+#pragma unroll 1
             for (uint32_t m = s_spk[cur][w]; m && w * 32 < M; m &= m - 1) {
               const int j = w * 32 + __ffs(m) - 1;
               float4* const cell = J.cell + (size_t)h * C * M + j;
               int* const tij = J.tij + (size_t)h * C * M + j;
               /* kColU cells of a thread at a time, their loads together */
+#pragma unroll 1
               for (int s0 = wt; s0 < C; s0 += kColU * kW) {
                 int pdt[kColU];
                 float4 cv[kColU], A[kColU], Bt[kColU];
@@ -801,10 +853,12 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     if (s_cols) atomicAdd(&net->counters[1], s_cols);
   }
   const int last = (rp->k0 + n_ticks - 1) & 1, next = last ^ 1;
+#pragma unroll 1
   for (int k = 0; k < n_in; ++k) {
     const ProjDev& J = s_proj[k];
     const Block B = block<kQW>(sm, L, k, M, J.C);
     const size_t eoff = (size_t)J.proj_in_pop * n;
+#pragma unroll 1
     for (int j = tid; j < M; j += kThreads) {
       const int idx = h * M + j;
       J.pj[idx] = B.pj[j];
@@ -813,11 +867,13 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       pop.epsc[last][eoff + idx] = B.epsc[last * M + j];
       pop.bj[last][eoff + idx] = B.bj[j];
     }
+#pragma unroll 1
     for (int s = tid; s < J.C; s += kThreads)
       if (B.src[s] != 0xffffu) J.qi[h * J.C + s] = (int)B.qi[s];
     const int part = queue_part(J.C, kQW), n0 = s_nl[k][next][0];
     const int cnt = kQW > 1 ? n0 + s_nl[k][next][kQW - 1] : n0;
     const uint16_t* l = B.list + next * kQW * part;
+#pragma unroll 1
     for (int e = tid; e < cnt; e += kThreads) J.list[h * J.C + e] = h * J.C + (int)(e < n0 ? l[e] : l[part + e - n0]);
     if (tid == 0) J.list_cnt[h] = cnt;
   }
