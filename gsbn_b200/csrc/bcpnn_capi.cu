@@ -137,6 +137,10 @@ struct bcpnn_net {
   const void* flow_fn = nullptr;  /* the dataflow kernel (bcpnn_flow.cuh), where the network fits it */
   size_t flow_smem = 0;
   flow::Args flow_args{};
+  /* bcpnn_reset: the fills of every state vector (fill_segments_kernel) */
+  FillSeg* d_fills = nullptr;
+  uint2* d_fill_at = nullptr;
+  unsigned int fill_blocks = 0;
   unsigned int* bar = nullptr; /* persistent kernel: [0] grid barrier arrivals, [1..2] column units by
                                   tick parity, [4 + cta] column units done for each CTA */
   int4* col_ring = nullptr;    /* deferred column units (NetDev::col_ring) */
@@ -300,48 +304,139 @@ int dzero(bcpnn_net* net, void* p, size_t bytes) {
   return BCPNN_OK;
 }
 
-/* gsbn's initial values (Pop.cpp:59-65, Proj.cpp:88-105) for every state
-   vector; connectivity (ii, di), stimulus and replay tables are kept. */
-int reset_state(bcpnn_net* net) {
-  int rc;
+uint32_t f32_bits(float v) {
+  uint32_t u;
+  std::memcpy(&u, &v, 4);
+  return u;
+}
+
+/* the fills of gsbn's initial values (Pop.cpp:59-65, Proj.cpp:88-105) for every
+   state vector; connectivity (ii, di), stimulus and replay tables are kept */
+int make_fills(bcpnn_net* net) {
+  std::vector<FillSeg> segs;
+  auto add = [&](void* p, size_t bytes, uint4 pattern) {
+    if (p && bytes) segs.push_back(FillSeg{(uint4*)p, (unsigned long long)bytes, pattern});
+  };
+  auto zero = [&](void* p, size_t bytes) { add(p, bytes, make_uint4(0u, 0u, 0u, 0u)); };
+  auto value = [&](float* p, size_t n, float v) {
+    const uint32_t u = f32_bits(v);
+    add(p, n * sizeof(float), make_uint4(u, u, u, u));
+  };
   for (size_t p = 0; p < net->pops.size(); ++p) {
     const PopHost& P = net->pops[p];
     PopDev& D = net->hp[p];
-    size_t n = P.n, ne = n * std::max(1, P.dim_proj);
+    const size_t n = P.n, ne = n * std::max(1, P.dim_proj);
     for (int b = 0; b < 2; ++b) {
-      if ((rc = dset(net, D.dsup[b], n, (float)bx_log_d(1.0 / P.M)))) return rc;   /* log(1.0/M), Pop.cpp:59 */
-      if ((rc = dzero(net, D.epsc[b], ne * sizeof(float)))) return rc;
-      if ((rc = dzero(net, D.bj[b], ne * sizeof(float)))) return rc;
+      value(D.dsup[b], n, (float)bx_log_d(1.0 / P.M)); /* log(1.0/M), Pop.cpp:59 */
+      zero(D.epsc[b], ne * sizeof(float));
+      zero(D.bj[b], ne * sizeof(float));
     }
-    if ((rc = dset(net, D.act, n, (float)(1.0 / P.M)))) return rc;                 /* Pop.cpp:60 */
-    if ((rc = dzero(net, D.spike, n))) return rc;
-    if ((rc = dzero(net, D.counter, n * sizeof(int)))) return rc;
-    if (D.ada && (rc = dzero(net, D.ada, n * sizeof(float)))) return rc;
-    if (D.ring && (rc = dzero(net, D.ring, n * (size_t)D.ring_len))) return rc;
+    value(D.act, n, (float)(1.0 / P.M)); /* Pop.cpp:60 */
+    zero(D.spike, n);
+    zero(D.counter, n * sizeof(int));
+    zero(D.ada, D.ada ? n * sizeof(float) : 0);
+    zero(D.ring, D.ring ? n * (size_t)D.ring_len : 0);
   }
   for (size_t q = 0; q < net->projs.size(); ++q) {
     const ProjHost& J = net->projs[q];
     ProjDev& D = net->hq[q];
-    size_t R = (size_t)J.H * J.C, HM = (size_t)J.H * J.M, cells = R * J.M;
-    if ((rc = dzero(net, D.qi, R * sizeof(int)))) return rc;
-    if ((rc = dset(net, D.pi, R, (float)(1.0 / J.C)))) return rc;                  /* Proj.cpp:91 */
-    if ((rc = dzero(net, D.ei, R * sizeof(float)))) return rc;
-    if ((rc = dzero(net, D.zi, R * sizeof(float)))) return rc;
-    if ((rc = dzero(net, D.ti, R * sizeof(int)))) return rc;
-    if ((rc = dset(net, D.pj, HM, (float)(1.0 / J.M)))) return rc;                 /* Proj.cpp:96 */
-    if ((rc = dzero(net, D.ej, HM * sizeof(float)))) return rc;
-    if ((rc = dzero(net, D.zj, HM * sizeof(float)))) return rc;
-    float pij0 = (float)(1.0 / J.C / J.M);                                         /* Proj.cpp:99 */
-    if ((rc = dset(net, D.cell, cells, make_float4(pij0, 0.0f, 0.0f, 0.0f)))) return rc;
-    if ((rc = dzero(net, D.tij, cells * sizeof(int)))) return rc;
-    if ((rc = dzero(net, D.wij, cells * sizeof(float)))) return rc;
-    if ((rc = dzero(net, D.si[0], 4 * (size_t)J.Ns))) return rc;
-    if ((rc = dzero(net, D.list_cnt, (size_t)J.H * sizeof(int)))) return rc;
+    const size_t R = (size_t)J.H * J.C, HM = (size_t)J.H * J.M, cells = R * J.M;
+    zero(D.qi, R * sizeof(int));
+    value(D.pi, R, (float)(1.0 / J.C)); /* Proj.cpp:91 */
+    zero(D.ei, R * sizeof(float));
+    zero(D.zi, R * sizeof(float));
+    zero(D.ti, R * sizeof(int));
+    value(D.pj, HM, (float)(1.0 / J.M)); /* Proj.cpp:96 */
+    zero(D.ej, HM * sizeof(float));
+    zero(D.zj, HM * sizeof(float));
+    add(D.cell, cells * sizeof(float4), make_uint4(f32_bits((float)(1.0 / J.C / J.M)), 0u, 0u, 0u)); /* Proj.cpp:99 */
+    zero(D.tij, cells * sizeof(int));
+    zero(D.wij, cells * sizeof(float));
+    zero(D.si[0], 4 * (size_t)J.Ns);
+    zero(D.list_cnt, (size_t)J.H * sizeof(int));
   }
+  std::vector<uint2> at;
+  for (size_t k = 0; k < segs.size(); ++k)
+    for (unsigned long long o = 0; o < segs[k].bytes; o += kFillBlock)
+      at.push_back(make_uint2((unsigned int)k, (unsigned int)(o / kFillBlock)));
+  int rc;
+  if ((rc = dalloc(net, &net->d_fills, segs.size())) || (rc = dalloc(net, &net->d_fill_at, at.size()))) return rc;
+  CU(cudaMemcpy(net->d_fills, segs.data(), segs.size() * sizeof(FillSeg), cudaMemcpyHostToDevice));
+  CU(cudaMemcpy(net->d_fill_at, at.data(), at.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  net->fill_blocks = (unsigned int)at.size();
+  return BCPNN_OK;
+}
+
+/* gsbn's initial state, in one launch */
+int reset_state(bcpnn_net* net) {
+  int rc;
+  if (!net->fill_blocks && (rc = make_fills(net))) return rc;
+  fill_segments_kernel<<<net->fill_blocks, 256, 0, net->stream>>>(net->d_fills, net->d_fill_at);
+  CU(cudaGetLastError());
+  net->launches++;
   for (size_t q = 0; q < net->check_cnt.size(); ++q)
     if (net->check_cnt[q] && (rc = dzero(net, net->check_cnt[q], (size_t)net->pops[q].H * net->pops[q].M * sizeof(int32_t))))
       return rc;
   net->k_total = 0;
+  return BCPNN_OK;
+}
+
+/* A run begins with one launch that sets its parameters and table references,
+   passed by value, and zeroes its records and the barrier words: two copies
+   and up to four memsets less, 7 us of a run's 30 (10 x 10, one tick).  For at
+   most kBeginProjs projections and kBeginPops populations; else copies and
+   memsets. */
+constexpr int kBeginProjs = 8, kBeginPops = 8;
+struct RunBegin {
+  RunParams rp;
+  TabRef tabs[kBeginProjs];
+  uint32_t* zero[kBeginPops + 2];
+  unsigned int words[kBeginPops + 2];
+  int n_zero, n_tabs;
+};
+
+__global__ void __launch_bounds__(256) run_begin_kernel(const __grid_constant__ RunBegin b, RunParams* rp, TabRef* tabs) {
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) *rp = b.rp;
+    if (threadIdx.x < b.n_tabs) tabs[threadIdx.x] = b.tabs[threadIdx.x];
+  }
+  for (int k = 0; k < b.n_zero; ++k) {
+    uint32_t* p = b.zero[k];
+    for (unsigned int i = blockIdx.x * 256 + threadIdx.x; i < b.words[k]; i += gridDim.x * 256) p[i] = 0u;
+  }
+}
+
+int begin_run(bcpnn_net* net, int n_ticks) {
+  const bool bar = net->persistent || net->multi_persistent;
+  const size_t bar_words = net->multi ? 4 : 4 + (size_t)net->total_hcu, ss_words = (size_t)n_ticks * net->h.n_projs;
+  if (net->projs.size() > kBeginProjs || net->pops.size() > kBeginPops ||
+      (size_t)n_ticks * net->log_words_per_tick > (1u << 30) || ss_words > (1u << 30)) {
+    CU(cudaMemcpyAsync(net->d_tabs, net->tabs.data(), net->tabs.size() * sizeof(TabRef), cudaMemcpyHostToDevice,
+                       net->stream));
+    CU(cudaMemcpyAsync(net->d_rp, &net->rp, sizeof(RunParams), cudaMemcpyHostToDevice, net->stream));
+    int rc;
+    for (const PopHost& P : net->pops)
+      if ((rc = dzero(net, net->log_buf + P.log_offset, (size_t)n_ticks * P.log_words * sizeof(uint32_t)))) return rc;
+    if ((rc = dzero(net, net->h.ss_log, ss_words * sizeof(uint32_t)))) return rc;
+    return bar ? dzero(net, net->bar, bar_words * sizeof(unsigned int)) : BCPNN_OK;
+  }
+  RunBegin b;
+  std::memset(&b, 0, sizeof(b));
+  b.rp = net->rp;
+  for (size_t p = 0; p < net->projs.size(); ++p) b.tabs[p] = net->tabs[p];
+  b.n_tabs = (int)net->projs.size();
+  size_t most = 0;
+  auto zero = [&](uint32_t* p, size_t words) {
+    b.zero[b.n_zero] = p;
+    b.words[b.n_zero++] = (unsigned int)words;
+    most = std::max(most, words);
+  };
+  for (const PopHost& P : net->pops) zero(net->log_buf + P.log_offset, (size_t)n_ticks * P.log_words);
+  if (ss_words) zero(net->h.ss_log, ss_words);
+  if (bar) zero(net->bar, bar_words);
+  run_begin_kernel<<<grid_for(most, 1024), 256, 0, net->stream>>>(b, net->d_rp, net->d_tabs);
+  CU(cudaGetLastError());
+  net->launches++;
   return BCPNN_OK;
 }
 
@@ -355,9 +450,6 @@ bool use_flow(const bcpnn_net* net) {
 
 /* the work of one run, queued on the network's stream */
 void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
-  for (const PopHost& P : net->pops)
-    cudaMemsetAsync(net->log_buf + P.log_offset, 0, (size_t)n_ticks * P.log_words * sizeof(uint32_t), net->stream);
-  cudaMemsetAsync(net->h.ss_log, 0, (size_t)n_ticks * net->h.n_projs * sizeof(uint32_t), net->stream);
   if (with_all && !net->multi) {
     for (int p = 0; p < net->h.n_projs; ++p) {
       const ProjHost& J = net->projs[p];
@@ -375,7 +467,6 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
         multi::all_kernel<<<grid_for((size_t)J.H * J.C * 32, 256), 256, 0, net->stream>>>(net->d_net, net->d_rp, p);
       }
     if (net->multi_persistent) {
-      cudaMemsetAsync(net->bar, 0, 4 * sizeof(unsigned int), net->stream);
       int it0 = 0, n = n_ticks;
       void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&it0, (void*)&n, (void*)&net->bar};
       cudaLaunchCooperativeKernel(net->multi_resident ? (const void*)multi::res_tick_kernel
@@ -399,7 +490,6 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
     void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&net->flow_args, (void*)&n};
     cudaLaunchCooperativeKernel(net->flow_fn, dim3(net->total_hcu), dim3(net->threads), args, net->flow_smem, net->stream);
   } else if (net->persistent) {
-    cudaMemsetAsync(net->bar, 0, (4 + (size_t)net->total_hcu) * sizeof(unsigned int), net->stream);
     int it0 = 0, n = n_ticks;
     void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&it0, (void*)&n, (void*)&net->bar};
     cudaLaunchCooperativeKernel(net->tick_fn, dim3(net->total_hcu), dim3(net->threads), args, smem, net->stream);
@@ -1195,6 +1285,23 @@ __global__ void lginp_idx_kernel(const NetDev* __restrict__ net, const int32_t* 
   for (int j = threadIdx.x; j < P.M; j += blockDim.x) out[P.mcu_start + h * P.M + j] = (want == j) ? hit : miss;
 }
 
+/* the same with the rows passed by value, mask included: one launch and no
+   copy, for at most kStimHcus HCUs (10.6 -> 3 us a call) */
+constexpr int kStimHcus = 448;
+struct StimRows {
+  int32_t lgidx[kStimHcus];
+  float wmask[kStimHcus];
+};
+
+__global__ void stim_rows_kernel(const __grid_constant__ StimRows r, const NetDev* __restrict__ net, float hit, float miss,
+                                 float* __restrict__ lginp, float* __restrict__ wmask) {
+  const PopDev& P = net->pops[net->cta_pop[blockIdx.x]];
+  const int h = net->cta_hcu[blockIdx.x], x = P.hcu_start + h, want = r.lgidx[x];
+  float* o = lginp + P.mcu_start + h * P.M;
+  for (int j = threadIdx.x; j < P.M; j += blockDim.x) o[j] = (want == j) ? hit : miss;
+  if (threadIdx.x == 0) wmask[x] = r.wmask[x];
+}
+
 int bcpnn_set_stimulus_idx(bcpnn_net* net, const int32_t* lgidx_row, size_t n_hcu, float eps, const float* wmask_row,
                            size_t n_wmask) {
   if (!net) return BCPNN_ERR_INVALID;
@@ -1202,6 +1309,18 @@ int bcpnn_set_stimulus_idx(bcpnn_net* net, const int32_t* lgidx_row, size_t n_hc
   if (n_hcu != (size_t)net->total_hcu || n_wmask != (size_t)net->total_hcu)
     return fail(net, BCPNN_ERR_SIZE, "bcpnn_set_stimulus_idx: sizes must be total HCUs");
   CU(cudaSetDevice(net->device));
+  if (net->total_hcu <= kStimHcus) {
+    StimRows r;
+    std::memcpy(r.lgidx, lgidx_row, n_hcu * sizeof(int32_t));
+    std::memcpy(r.wmask, wmask_row, n_hcu * sizeof(float));
+    stim_rows_kernel<<<net->total_hcu, 64, 0, net->stream>>>(r, net->d_net, bx_extgen_logf(1 + eps), bx_extgen_logf(0 + eps),
+                                                             net->h.lginp, net->h.wmask);
+    CU(cudaGetLastError());
+    net->launches += 1;
+    net->cur_lg = net->h.lginp;
+    net->cur_wm = net->h.wmask;
+    return BCPNN_OK;
+  }
   if (!net->d_lgidx) {
     int rc = dalloc(net, &net->d_lgidx, (size_t)net->total_hcu);
     if (rc) return rc;
@@ -1413,9 +1532,10 @@ int bcpnn_run(bcpnn_net* net, int32_t first_simstep, int32_t n_ticks, float prn,
   net->rp.serial0 = net->tick_serial;
   net->tick_serial += (uint32_t)n_ticks;
   if (net->tick_serial == 0) net->tick_serial = 1; /* tag 0 is the slots' initial value */
-  CU(cudaMemcpyAsync(net->d_tabs, net->tabs.data(), net->tabs.size() * sizeof(TabRef), cudaMemcpyHostToDevice,
-                     net->stream));
-  CU(cudaMemcpyAsync(net->d_rp, &net->rp, sizeof(RunParams), cudaMemcpyHostToDevice, net->stream));
+  {
+    int rc = begin_run(net, n_ticks);
+    if (rc) return rc;
+  }
   if (net->direct || net->persistent || net->multi_persistent) {
     enqueue_run(net, n_ticks, with_all);
     CU(cudaGetLastError());

@@ -724,6 +724,32 @@ __global__ void fill_kernel(T* p, size_t n, T v) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
+/* A fill of `bytes` bytes at a 16-byte aligned address with a 16-byte pattern;
+   fill_segments_kernel does many in one launch, block b the kFillBlock bytes
+   of segment at[b].x from offset at[b].y * kFillBlock on.  Bound by the writes
+   where there are large segments; for small networks the launch, one instead
+   of one per state vector (reset of the 10 x 10 network: 75 -> 10 us, of the
+   100 x 100 network, 240 MB: 131 -> 66 us). */
+struct FillSeg {
+  uint4* p;
+  unsigned long long bytes;
+  uint4 pattern;
+};
+constexpr unsigned int kFillBlock = 65536;
+
+__global__ void __launch_bounds__(256) fill_segments_kernel(const FillSeg* __restrict__ segs, const uint2* __restrict__ at) {
+  const uint2 b = at[blockIdx.x];
+  const FillSeg s = segs[b.x];
+  const unsigned long long from = (unsigned long long)b.y * kFillBlock;
+  const unsigned int n = s.bytes - from < kFillBlock ? (unsigned int)(s.bytes - from) : kFillBlock;
+  uint4* p = s.p + from / 16;
+  for (unsigned int i = threadIdx.x; i < n / 16; i += 256) p[i] = s.pattern;
+  if (threadIdx.x < (n & 15u)) { /* the last bytes of the segment */
+    const uint32_t w = (threadIdx.x >> 2) == 0 ? s.pattern.x : (threadIdx.x >> 2) == 1 ? s.pattern.y : (threadIdx.x >> 2) == 2 ? s.pattern.z : s.pattern.w;
+    reinterpret_cast<uint8_t*>(p + n / 16)[threadIdx.x] = (uint8_t)(w >> (8 * (threadIdx.x & 3u)));
+  }
+}
+
 /* gather / scatter of one float of the (pij, eij, zi2, zj2) cells */
 __global__ void cell_gather_kernel(const float4* cell, size_t n, int field, float* out) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
