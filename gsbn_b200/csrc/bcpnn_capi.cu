@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "bcpnn.h"
+#include "host_copy.h"
 #include "bcpnn_device.cuh"
 #define BCPNN_TICK_THREADS 512
 #define BCPNN_TICK_NS t512
@@ -92,6 +93,8 @@ struct ProjHost {
 }  // namespace
 
 struct bcpnn_net {
+  host_copy::Users copies;
+  uint32_t* stage = nullptr; /* page-locked: small results and the error word (read_small) */
   int device = 0;
   cudaStream_t stream = nullptr;
   std::vector<void*> allocs;
@@ -199,10 +202,10 @@ int grid_for(size_t n, int block) {
   return (int)g;
 }
 
-int check_device_error(bcpnn_net* net) {
-  int e = 0;
-  CU(cudaMemcpyAsync(&e, net->h.err, sizeof(int), cudaMemcpyDeviceToHost, net->stream));
-  CU(cudaStreamSynchronize(net->stream));
+/* words of bcpnn_net::stage before the error word */
+constexpr size_t kStageWords = 16384 - 16;
+
+int device_error(bcpnn_net* net, int e) {
   if (e) {
     CU(cudaMemsetAsync(net->h.err, 0, sizeof(int), net->stream));
     std::string why;
@@ -213,6 +216,25 @@ int check_device_error(bcpnn_net* net) {
     return fail(net, BCPNN_ERR_DEVICE, "kernel reported error word " + std::to_string(e) + ":" + why);
   }
   return BCPNN_OK;
+}
+
+int check_device_error(bcpnn_net* net) {
+  int* e = (int*)(net->stage + kStageWords);
+  CU(cudaMemcpyAsync(e, net->h.err, sizeof(int), cudaMemcpyDeviceToHost, net->stream));
+  CU(cudaStreamSynchronize(net->stream));
+  return device_error(net, *e);
+}
+
+/* `words` words to the caller and the error word, with one wait for both */
+int read_checked(bcpnn_net* net, uint32_t* out, const uint32_t* src, size_t words) {
+  if (words > kStageWords) {
+    CU(host_copy::to_host(out, src, words * sizeof(uint32_t), net->stream));
+    return check_device_error(net);
+  }
+  if (words) CU(cudaMemcpyAsync(net->stage, src, words * sizeof(uint32_t), cudaMemcpyDeviceToHost, net->stream));
+  const int rc = check_device_error(net);
+  if (words) std::memcpy(out, net->stage, words * sizeof(uint32_t));
+  return rc;
 }
 
 /* (re)build the decay table of slot s of projection p for kp = taupdt*prn
@@ -804,6 +826,11 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
     net->err = "cudaStreamCreate failed";
     return bail(BCPNN_ERR_CUDA);
   }
+  static_assert((kStageWords + 16) * sizeof(uint32_t) == host_copy::kSmall, "the stage is one small buffer");
+  if (!(net->stage = (uint32_t*)host_copy::take_small())) {
+    net->err = "cudaHostAlloc failed";
+    return bail(BCPNN_ERR_CUDA);
+  }
   for (int k = 0; k < 2; ++k)
     if (cudaEventCreateWithFlags(&net->stage_ready[k], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&net->stage_free[k], cudaEventDisableTiming) != cudaSuccess) {
@@ -1182,6 +1209,7 @@ int bcpnn_net_destroy(bcpnn_net* net) {
       if (s.ptr) cudaFree(s.ptr);
   for (void* p : net->allocs) cudaFree(p);
   if (net->scratch) cudaFree(net->scratch);
+  host_copy::give_small(net->stage);
   if (net->stim_lg) cudaFree(net->stim_lg);
   if (net->stim_wm) cudaFree(net->stim_wm);
   if (net->d_lgidx_tab) cudaFree(net->d_lgidx_tab);
@@ -1585,9 +1613,7 @@ int bcpnn_get_spike_log(bcpnn_net* net, int32_t pop, uint32_t* out, size_t n_wor
   size_t need = (size_t)net->last_run_ticks * P.log_words;
   if (n_words != need) return fail(net, BCPNN_ERR_SIZE, "bcpnn_get_spike_log: n_words != last run ticks * words");
   CU(cudaSetDevice(net->device));
-  if (need) CU(cudaMemcpyAsync(out, net->log_buf + P.log_offset, need * sizeof(uint32_t), cudaMemcpyDeviceToHost, net->stream));
-  CU(cudaStreamSynchronize(net->stream));
-  return check_device_error(net);
+  return read_checked(net, out, net->log_buf + P.log_offset, need);
 }
 
 int bcpnn_get_spike_log_async(bcpnn_net* net, int32_t pop, uint32_t* out, size_t n_words) {
@@ -1757,13 +1783,13 @@ int bcpnn_read_state(bcpnn_net* net, const char* name, void* host, size_t bytes)
   int last = (int)((net->k_total - 1) & 1);  /* buffer written by the last tick (1 before any tick) */
   switch (r.kind) {
     case K_PLAIN:
-      CU(cudaMemcpyAsync(host, r.ptr, bytes, cudaMemcpyDeviceToHost, net->stream));
+      CU(host_copy::to_host(host, r.ptr, bytes, net->stream));
       break;
     case K_PARITY:
-      CU(cudaMemcpyAsync(host, r.par[last], bytes, cudaMemcpyDeviceToHost, net->stream));
+      CU(host_copy::to_host(host, r.par[last], bytes, net->stream));
       break;
     case K_SI:
-      CU(cudaMemcpyAsync(host, si_last(net, r), bytes, cudaMemcpyDeviceToHost, net->stream));
+      CU(host_copy::to_host(host, si_last(net, r), bytes, net->stream));
       break;
     case K_CELL: {
       int rc = ensure_scratch(net, r.count);
@@ -1771,7 +1797,7 @@ int bcpnn_read_state(bcpnn_net* net, const char* name, void* host, size_t bytes)
       cell_gather_kernel<<<grid_for(r.count, 256), 256, 0, net->stream>>>(r.cell, r.count, r.field, net->scratch);
       CU(cudaGetLastError());
       net->launches++;
-      CU(cudaMemcpyAsync(host, net->scratch, bytes, cudaMemcpyDeviceToHost, net->stream));
+      CU(host_copy::to_host(host, net->scratch, bytes, net->stream));
       break;
     }
     case K_SIQ: {
@@ -1791,7 +1817,6 @@ int bcpnn_read_state(bcpnn_net* net, const char* name, void* host, size_t bytes)
       break;
     }
   }
-  CU(cudaStreamSynchronize(net->stream));
   return BCPNN_OK;
 }
 

@@ -40,6 +40,7 @@
 
 #include "bcpnn_numerics.h"
 #include "bcpnn_recall.h"
+#include "host_copy.h"
 
 namespace bcpnn_recall_dev {
 
@@ -961,6 +962,7 @@ __global__ void broadcast_f32_kernel(float* dst, int R, int N, const float* row)
 using namespace bcpnn_recall_dev;
 
 struct bcpnn_recall {
+  host_copy::Users copies;
   bcpnn_recall_desc d;
   int N = 0;
   cudaStream_t stream = nullptr;      /* contraction + epsc; the handle's stream */
@@ -1411,19 +1413,16 @@ int bcpnn_recall_read(bcpnn_recall* r, const char* name, int32_t row0, int32_t n
   if (kind == 2) {
     /* N is a multiple of 32: whole words per row */
     std::vector<uint32_t> tmp(n / 32);
-    RCU(cudaMemcpyAsync(tmp.data(), (uint32_t*)base + (size_t)row0 * r->N / 32, n / 8, cudaMemcpyDeviceToHost, r->stream));
-    RCU(cudaStreamSynchronize(r->stream));
+    RCU(host_copy::to_host(tmp.data(), (uint32_t*)base + (size_t)row0 * r->N / 32, n / 8, r->stream));
     int8_t* o = (int8_t*)host;
     for (size_t i = 0; i < n; i++) o[i] = (int8_t)((tmp[i / 32] >> (i % 32)) & 1u);
   } else if (kind == 1) {
     std::vector<uint16_t> tmp(n);
-    RCU(cudaMemcpyAsync(tmp.data(), (uint8_t*)base + off, n * 2, cudaMemcpyDeviceToHost, r->stream));
-    RCU(cudaStreamSynchronize(r->stream));
+    RCU(host_copy::to_host(tmp.data(), (uint8_t*)base + off, n * 2, r->stream));
     int8_t* o = (int8_t*)host;
     for (size_t i = 0; i < n; i++) o[i] = tmp[i] ? 1 : 0;
   } else {
-    RCU(cudaMemcpyAsync(host, (uint8_t*)base + off, n * elem, cudaMemcpyDeviceToHost, r->stream));
-    RCU(cudaStreamSynchronize(r->stream));
+    RCU(host_copy::to_host(host, (uint8_t*)base + off, n * elem, r->stream));
   }
   return BCPNN_OK;
 }
