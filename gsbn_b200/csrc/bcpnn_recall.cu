@@ -33,6 +33,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -75,6 +76,7 @@ struct Params {
   uint32_t seed_base;
   int simstep;
   int poisson;
+  uint32_t pr_count; /* a 24-bit uniform k 2^-24 is below pr for k < pr_count */
   int* err;
 };
 
@@ -192,28 +194,85 @@ __device__ __forceinline__ float dsup_mcu0(const Params& p, int row, uint32_t se
   return d + (sup - d) * p.taumdt;
 }
 
-/* Population update of tick `simstep` (Pop.cpp:229-323) for one quarter of
-   one HCU of one replicate: thread tid = (replicate * H + HCU) * 4 + q holds
-   MCUs q*Q .. q*Q+Q-1 of the HCU (Q = M/4), so four consecutive lanes hold
-   the four quarters of an HCU.  The HCU maximum is a shuffle max (exact); the
-   activity sum keeps gsbn's serial MCU order by passing the running sum from
-   lane to lane; one Philox call per four MCUs and stream.  Its own kernel,
-   run beside the contraction on a second stream: a CTA of the contraction
-   leaves room on its SM for three of its CTAs. */
+/* two IEEE additions in one instruction, as a 64-bit register pair */
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  return (f32x2)__float_as_uint(a) | ((f32x2)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 c;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
+}
+
+/* two products, one by one: a mul.rn.f32x2, or a multiply-add of -0, before an
+   add.rn.f32x2 came out as one multiply-add with one rounding */
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { return pack2(lo2(a) * lo2(b), hi2(a) * hi2(b)); }
+
+__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f32x2 dup2(float a) { return pack2(a, a); }
+
+/* bx_expf of two values in (kExpLow, 0], where its result is normal: the same
+   operations on pairs, without its clamps and its two-step scaling (the result
+   is the polynomial's bits plus the exponent).  Same bits. */
+constexpr float kExpLow = -83.0f;
+
+__device__ __forceinline__ f32x2 exp2_near(f32x2 x) {
+  const f32x2 shift = dup2(0x1.8p23f);
+  const f32x2 t = add2(mul2(x, dup2(0x1.715476p+0f)), shift);
+  const f32x2 kf = add2(t, neg2(shift));
+  const f32x2 r = add2(add2(x, neg2(mul2(kf, dup2(0x1.62e4p-1f)))), neg2(mul2(kf, dup2(0x1.7f7d1cp-20f))));
+  f32x2 p = dup2(0x1.a01a02p-16f);
+  p = add2(mul2(p, r), dup2(0x1.a01a02p-13f));
+  p = add2(mul2(p, r), dup2(0x1.6c16c2p-10f));
+  p = add2(mul2(p, r), dup2(0x1.111112p-7f));
+  p = add2(mul2(p, r), dup2(0x1.555556p-5f));
+  p = add2(mul2(p, r), dup2(0x1.555556p-3f));
+  p = add2(mul2(p, r), dup2(0.5f));
+  p = add2(mul2(p, r), dup2(1.0f));
+  p = add2(mul2(p, r), dup2(1.0f));
+  /* t's low bits are k + 2^22 (mod 2^9 all that shifts in): k << 23 */
+  const uint32_t a = (uint32_t)p + ((uint32_t)t << 23), b = (uint32_t)(p >> 32) + ((uint32_t)(t >> 32) << 23);
+  return (f32x2)a | ((f32x2)b << 32);
+}
+
+/* Population update of tick `simstep` (Pop.cpp:229-323) for a quarter of one
+   HCU of one replicate: thread tid = (replicate * H + HCU) * 4 + q holds the
+   groups of four MCUs q, q + 4, ... of the HCU (M/16 of them), so four
+   consecutive lanes hold an HCU and read and write 64 contiguous bytes of every
+   array at a time.  The HCU maximum is a shuffle max (exact); the activity sum
+   keeps gsbn's serial MCU order by passing the running sum from lane to lane,
+   group by group; one Philox call per four MCUs and stream.  Its own kernel,
+   run beside the contraction on a second stream: a CTA of the BF16 contraction
+   leaves room on its SM for three of its CTAs.
+
+   Bound by instruction issue: two Philox4x32-10 calls of about 50 instructions
+   per four MCUs, one exp per MCU.  The additions of support and exp run on pairs of MCUs.  The division of a spike's activity by the HCU's sum is done
+   only where the uniform is below the activity times maxfq dt / sum, rounded up
+   by 2^-20: about one MCU in 500 here; the comparison decides as if every MCU
+   divided (the exact product is below that bound by more than its roundings,
+   and a uniform of 0 always takes the exact path).  The recall counters are
+   touched only where a group has a spike.  kBits: the spikes as bits, for the
+   FP32 contraction.  64 x 64, 4096 replicates: 100 us alone as one exp and one
+   division per MCU, with 16 contiguous MCUs per lane. */
 template <int M, bool kBits>
 __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
-  constexpr int Q = M / 4;
+  constexpr int G = M / 16; /* groups of four MCUs per lane */
   const int lane = threadIdx.x & 31;
   const int tid = blockIdx.x * 256 + threadIdx.x;
   const int g = tid >> 2, q = tid & 3;
   const int h = g % p.H, r = g / p.H;
   const uint32_t seed = p.seed_base + (uint32_t)r;
   const size_t row = (size_t)r * p.N;
-  const int c0 = h * M + q * Q;
+  const int c0 = h * M; /* group i of the lane: MCUs c0 + (4 i + q) * 4 .. + 3 */
   /* self-check: every vector access below is in bounds and aligned */
   {
     const size_t n = (size_t)p.R * p.N;
-    const bool bad = r >= p.R || row + c0 + Q > n || ((row + c0) & 3) != 0 || (c0 + Q) > p.N ||
+    const bool bad = r >= p.R || row + c0 + M > n || ((row + c0) & 15) != 0 || (c0 + M) > p.N ||
                      (reinterpret_cast<uintptr_t>(p.dsup_prev) & 15) || (reinterpret_cast<uintptr_t>(p.dsup_cur) & 15) ||
                      (reinterpret_cast<uintptr_t>(p.epsc_prev) & 15) || (reinterpret_cast<uintptr_t>(p.bj) & 15) ||
                      (kBits ? reinterpret_cast<uintptr_t>(p.s_bits) & 15 : reinterpret_cast<uintptr_t>(p.s_out) & 15) ||
@@ -227,100 +286,131 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
   const float seed0 = dsup_mcu0(p, r, seed);
   const int lg = p.lgidx[(size_t)r * p.H + h];
   const float wm = p.wgain * p.wmask[(size_t)r * p.H + h];
-  float d[Q];
+  const float base_hit = p.lgbias + p.igain * p.lg_hit, base_miss = p.lgbias + p.igain * p.lg_miss;
+  f32x2 d[2 * G];
 #pragma unroll
-  for (int m = 0; m < Q; m += 4) {
-    float4 dp = *reinterpret_cast<const float4*>(p.dsup_prev + row + c0 + m);
-    float4 ep = *reinterpret_cast<const float4*>(p.epsc_prev + row + c0 + m);
-    float4 bb = *reinterpret_cast<const float4*>(p.bj + c0 + m);
-    float dpv[4] = {dp.x, dp.y, dp.z, dp.w}, epv[4] = {ep.x, ep.y, ep.z, ep.w}, bjv[4] = {bb.x, bb.y, bb.z, bb.w};
+  for (int i = 0; i < G; i++) {
+    const int m = (4 * i + q) * 4;
+    const float4 dp = *reinterpret_cast<const float4*>(p.dsup_prev + row + c0 + m);
+    const float4 ep = *reinterpret_cast<const float4*>(p.epsc_prev + row + c0 + m);
+    const float4 bb = *reinterpret_cast<const float4*>(p.bj + c0 + m);
+    float sup[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      float wsup = 0.0f;
-      wsup += bjv[k] + epv[k];
-      float noise = 0.0f;
-      if (p.snoise != 0.0f) noise = p.snoise * bx_normal01(seed, 0u, (uint32_t)p.simstep, (uint32_t)(c0 + m + k));
-      float lginp = (lg == q * Q + m + k) ? p.lg_hit : p.lg_miss;
-      float sup = p.lgbias + p.igain * lginp + noise;
-      sup += wm * wsup;
-      d[m + k] = dpv[k] + (sup - dpv[k]) * p.taumdt;
+    for (int k = 0; k < 4; k++) sup[k] = lg == m + k ? base_hit : base_miss;
+    if (p.snoise != 0.0f) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) sup[k] += p.snoise * bx_normal01(seed, 0u, (uint32_t)p.simstep, (uint32_t)(c0 + m + k));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) sup[k] += 0.0f;
+    }
+    const f32x2 dv[2] = {pack2(dp.x, dp.y), pack2(dp.z, dp.w)};
+    const f32x2 wsup[2] = {add2(dup2(0.0f), add2(pack2(bb.x, bb.y), pack2(ep.x, ep.y))),
+                           add2(dup2(0.0f), add2(pack2(bb.z, bb.w), pack2(ep.z, ep.w)))};
+#pragma unroll
+    for (int v = 0; v < 2; v++) {
+      const f32x2 s2 = add2(pack2(sup[2 * v], sup[2 * v + 1]), mul2(dup2(wm), wsup[v]));
+      d[2 * i + v] = add2(dv[v], mul2(add2(s2, neg2(dv[v])), dup2(p.taumdt)));
     }
   }
   float mx = seed0; /* the new dsup of population MCU 0 (also d[0] of HCU 0's first quarter) */
 #pragma unroll
-  for (int m = 0; m < Q; m++) mx = (d[m] > mx) ? d[m] : mx;
+  for (int i = 0; i < 2 * G; i++) {
+    mx = (lo2(d[i]) > mx) ? lo2(d[i]) : mx;
+    mx = (hi2(d[i]) > mx) ? hi2(d[i]) : mx;
+  }
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
   const float maxact = bx_expf(p.wtagain * mx);
-  float a[Q];
+  f32x2 a[2 * G];
+  bool near = true;
 #pragma unroll
-  for (int m = 0; m < Q; m++) {
-    a[m] = bx_expf(p.wtagain * (d[m] - mx));
-    if (maxact < 1.0f) a[m] *= maxact;
+  for (int i = 0; i < 2 * G; i++) {
+    a[i] = mul2(dup2(p.wtagain), add2(d[i], neg2(dup2(mx))));
+    near = near & (lo2(a[i]) > kExpLow) & (hi2(a[i]) > kExpLow) & (lo2(a[i]) <= 0.0f) & (hi2(a[i]) <= 0.0f);
+  }
+  if (near) {
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++) a[i] = exp2_near(a[i]);
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < 2 * G; i++) {
+      f32x2 v = 0;
+#pragma unroll
+      for (int j = 0; j < 2 * G; j++) v = i == j ? a[j] : v;
+      v = pack2(bx_expf(lo2(v)), bx_expf(hi2(v)));
+#pragma unroll
+      for (int j = 0; j < 2 * G; j++) a[j] = i == j ? v : a[j];
+    }
+  }
+  if (maxact < 1.0f) {
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++) a[i] = mul2(a[i], dup2(maxact));
   }
   float vs = 0.0f;
 #pragma unroll
-  for (int s = 0; s < 4; s++) {
-    if (q == s) {
+  for (int i = 0; i < G; i++)
 #pragma unroll
-      for (int m = 0; m < Q; m++) vs += a[m];
+    for (int s = 0; s < 4; s++) {
+      const float v = (((vs + lo2(a[2 * i])) + hi2(a[2 * i])) + lo2(a[2 * i + 1])) + hi2(a[2 * i + 1]);
+      vs = __shfl_sync(0xffffffffu, v, (lane & ~3) | s);
     }
-    vs = __shfl_sync(0xffffffffu, vs, (lane & ~3) | s);
-  }
-  uint32_t bits = 0u;
+  /* above every product (act / vs) * maxfqdt, in units of 2^-24 */
+  const float bound = (vs > 1.0f ? p.maxfqdt / vs : p.maxfqdt) * (0x1p24f * (1.0f + 0x1p-20f));
 #pragma unroll
-  for (int m = 0; m < Q; m += 4) {
+  for (int i = 0; i < G; i++)
+    *reinterpret_cast<float4*>(p.dsup_cur + row + c0 + (4 * i + q) * 4) =
+        make_float4(lo2(d[2 * i]), hi2(d[2 * i]), lo2(d[2 * i + 1]), hi2(d[2 * i + 1]));
+  uint32_t all = 0u; /* four bits per group */
+#pragma unroll
+  for (int i = 0; i < G; i++) {
+    const int m = (4 * i + q) * 4;
     bx_u32x4 cu;
     cu.v[0] = (uint32_t)(c0 + m) >> 2;
     cu.v[1] = (uint32_t)p.simstep;
     cu.v[2] = 0u;
     cu.v[3] = 0u;
     const bx_u32x4 ou = bx_philox4x32_10(cu, seed, 0u * 16u + BX_STREAM_UNIFORM);
-    bx_u32x4 op;
-    if (p.poisson) op = bx_philox4x32_10(cu, seed, 0u * 16u + BX_STREAM_POISSON);
+    uint32_t bits = 0u;
+    const float av[4] = {lo2(a[2 * i]), hi2(a[2 * i]), lo2(a[2 * i + 1]), hi2(a[2 * i + 1])};
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      float act = a[m + k];
-      if (vs > 1.0f) act /= vs;
-      bool spk = bx_u01(ou.v[k]) < act * p.maxfqdt;
-      if (p.poisson && bx_u01(op.v[k]) < p.pr) spk = true;
-      if (spk) bits |= 1u << (m + k);
+    for (int k = 0; k < 4; k++)
+      if ((float)(ou.v[k] >> 8) <= av[k] * bound) {
+        float act = av[k];
+        if (vs > 1.0f) act /= vs;
+        if (bx_u01(ou.v[k]) < act * p.maxfqdt) bits |= 1u << k;
+      }
+    if (p.poisson) {
+      const bx_u32x4 op = bx_philox4x32_10(cu, seed, 0u * 16u + BX_STREAM_POISSON);
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if ((op.v[k] >> 8) < p.pr_count) bits |= 1u << k;
     }
-  }
-#pragma unroll
-  for (int m = 0; m < Q; m += 4)
-    *reinterpret_cast<float4*>(p.dsup_cur + row + c0 + m) = make_float4(d[m], d[m + 1], d[m + 2], d[m + 3]);
-  if (kBits) {
-    /* row + c0 is a multiple of Q, so a quarter's bits are whole bytes, or
-       half a byte at Q = 4, where two lanes share one */
-    uint8_t* o = reinterpret_cast<uint8_t*>(p.s_bits) + ((row + c0) >> 3);
-    if (Q == 16) {
-      *reinterpret_cast<uint16_t*>(o) = (uint16_t)bits;
-    } else if (Q == 8) {
-      *o = (uint8_t)bits;
-    } else {
-      const uint32_t hi = __shfl_down_sync(0xffffffffu, bits, 1);
-      if ((q & 1) == 0) *o = (uint8_t)(bits | (hi << 4));
-    }
-  } else {
-    /* BF16 1.0 = 0x3F80; four MCUs per 8-byte store (Q is a multiple of 4) */
-#pragma unroll
-    for (int m = 0; m < Q; m += 4) {
+    if (!kBits) {
+      /* BF16 1.0 = 0x3F80 */
       uint32_t w[2];
 #pragma unroll
       for (int k = 0; k < 2; k++)
-        w[k] = (((bits >> (m + 2 * k)) & 1u) ? 0x3F80u : 0u) | ((((bits >> (m + 2 * k + 1)) & 1u) ? 0x3F80u : 0u) << 16);
+        w[k] = (((bits >> (2 * k)) & 1u) ? 0x3F80u : 0u) | ((((bits >> (2 * k + 1)) & 1u) ? 0x3F80u : 0u) << 16);
       *reinterpret_cast<uint2*>(p.s_out + row + c0 + m) = make_uint2(w[0], w[1]);
     }
-  }
-  if (p.count_on) {
-#pragma unroll
-    for (int m = 0; m < Q; m += 4) {
+    if (p.count_on && bits) {
       uint32_t* c = reinterpret_cast<uint32_t*>(p.counts + row + c0 + m);
       uint32_t add = 0;
 #pragma unroll
-      for (int k = 0; k < 4; k++) add |= ((bits >> (m + k)) & 1u) << (8 * k);
+      for (int k = 0; k < 4; k++) add |= ((bits >> k) & 1u) << (8 * k);
       *c = *c + add; /* no carry between bytes: at most 255 counted ticks between clears */
+    }
+    all |= bits << (4 * i);
+  }
+  if (kBits) {
+    /* 16 spikes of the HCU per group index, the lane's four at 4 q */
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+      uint32_t v = ((all >> (4 * i)) & 15u) << (4 * q);
+      v |= __shfl_xor_sync(0xffffffffu, v, 1);
+      v |= __shfl_xor_sync(0xffffffffu, v, 2);
+      if (q == 0) reinterpret_cast<uint16_t*>(p.s_bits)[(row + c0) / 16 + i] = (uint16_t)v;
     }
   }
 }
@@ -644,13 +734,6 @@ static_assert(kEvSmemBytes <= 232448, "shared memory of one CTA");
    of a 16-bit list entry; lane8 = 8 * lane is the low byte */
 __device__ __forceinline__ uint32_t ev_row0(uint32_t two, uint32_t lane8) { return __byte_perm(two, lane8, 0x7104); }
 __device__ __forceinline__ uint32_t ev_row1(uint32_t two, uint32_t lane8) { return __byte_perm(two, lane8, 0x7324); }
-
-/* two IEEE additions in one instruction, as a 64-bit register pair */
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long c;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
-  return c;
-}
 
 __device__ __forceinline__ unsigned long long lds64(uint32_t a) {
   unsigned long long v;
@@ -1281,6 +1364,7 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   p.one_m_kepsc = 1.0f - d.kepsc;
   p.pr = d.poisson_noise_hz * d.dt;
   p.poisson = d.poisson_noise_hz > 0.f;
+  p.pr_count = !p.poisson ? 0u : p.pr >= 1.0f ? 1u << 24 : (uint32_t)std::ceil((double)p.pr * 0x1p24);
   p.seed_base = d.seed_base;
   p.err = r->err;
   const int n_tiles = (r->N / kTileN) * (d.replicates / kTileM);
