@@ -47,6 +47,7 @@ namespace bcpnn_recall_dev {
 
 constexpr int kTileM = 128, kTileN = 256, kTileK = 64, kStages = 4, kUmmaK = 16;
 constexpr int kThreads = 192;
+constexpr int kMaxPartsLog = 3, kMaxParts = 1 << kMaxPartsLog; /* column parts of a tile, see Tiles */
 constexpr uint32_t kBytesA = kTileM * kTileK * 2; /* 16 KB */
 constexpr uint32_t kBytesB = kTileN * kTileK * 2; /* 32 KB */
 constexpr uint32_t kStageBytes = kBytesA + kBytesB;
@@ -141,16 +142,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   return d;
 }
 
-/* instruction descriptor: D F32, A BF16, B BF16, both K-major, N=256, M=128 */
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileN >> 3) << 17) |
-                            ((uint32_t)(kTileM >> 4) << 24);
+/* instruction descriptor: D F32, A BF16, B BF16, both K-major, M=128, N columns */
+__device__ __forceinline__ uint32_t umma_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+}
 
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                     uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -419,14 +422,55 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-/* Persistent contraction + epsc epilogue: one CTA per SM walks the output
-   tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (tile t = M-tile t / nN,
-   N-tile t % nN).  The stage ring runs on across tiles; two TMEM accumulators
-   of 256 columns alternate, so the epilogue of one tile overlaps the MMAs of
-   the next (acc_full: MMA -> epilogue, acc_empty: epilogue -> MMA). */
+/* The output tiles of a launch: 128 x 256, or, where these are fewer than the
+   SMs, column parts of 128, 64 or 32, as narrow as still gives every SM at most
+   one.  A single tile (256 sources, 128 replicates) takes 8 CTAs of 32 columns
+   instead of one: 24 -> 9.6 us, mostly its epilogue's loads; 32 tiles (N = R =
+   1024) take 128 CTAs: 31 -> 17 us.  Cutting the last round of more tiles too
+   makes the contraction shorter (512 tiles on 148 SMs: 158 -> 146 us in place),
+   but not the tick (176, 178): the population update beside it is then what the
+   tick waits for. */
+struct Tiles {
+  int n_n;   /* tiles across the columns */
+  int whole; /* whole tiles, 0 .. whole - 1 */
+  int parts; /* parts per tile from `whole` on */
+  int total; /* whole tiles and parts */
+  __host__ __device__ Tiles(int R, int N, int grid_max) {
+    n_n = N / kTileN;
+    const int n = n_n * (R / kTileM);
+    whole = n / grid_max * grid_max;
+    const int rest = n - whole;
+    parts = 1;
+    while (whole == 0 && parts < kMaxParts && 2 * parts * rest <= grid_max) parts *= 2;
+    total = whole + rest * parts;
+  }
+  __device__ __forceinline__ void at(int t, int& m0, int& n0, int& cols) const {
+    int tile = t, part = 0;
+    cols = kTileN;
+    if (t >= whole) {
+      tile = whole + (t - whole) / parts;
+      part = (t - whole) % parts;
+      cols = kTileN / parts;
+    }
+    m0 = tile / n_n * kTileM;
+    n0 = tile % n_n * kTileN + part * cols;
+  }
+};
+
+/* W^T boxes of a tile's columns: whole, then halves, quarters and eighths */
+struct WMaps {
+  CUtensorMap of[kMaxPartsLog + 1];
+};
+
+/* Persistent contraction + epsc epilogue: one CTA per SM walks the tiles t =
+   blockIdx.x, blockIdx.x + gridDim.x, ... (Tiles).  The stage ring runs on
+   across tiles; two TMEM accumulators of 256 columns alternate, so the epilogue
+   of one tile overlaps the MMAs of the next (acc_full: MMA -> epilogue,
+   acc_empty: epilogue -> MMA).  The epilogue's loads run one 32-column chunk
+   ahead, the first before its accumulator is there. */
 __global__ void __launch_bounds__(kThreads, 1)
-    recall_tick_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_w,
-                       Params p) {
+    recall_tick_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_constant__ WMaps map_w, Params p,
+                       int grid_max) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + kStages * kStageBytes);
@@ -437,8 +481,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nN = p.N / kTileN, nM = p.R / kTileM, n_tiles = nN * nM;
+  const Tiles tiles(p.R, p.N, grid_max);
+  const int n_tiles = tiles.total;
   const int kIters = p.N / kTileK;
+  const int part_log = tiles.parts == 1 ? 0 : tiles.parts == 2 ? 1 : tiles.parts == 4 ? 2 : 3;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -476,7 +522,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       long long it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int m0 = (t / nN) * kTileM, n0 = (t % nN) * kTileN;
+        int m0, n0, cols;
+        tiles.at(t, m0, n0, cols);
+        const CUtensorMap* w = &map_w.of[t < tiles.whole ? 0 : part_log];
         for (int k = 0; k < kIters; k++, it++) {
           const int s = (int)(it % kStages);
           if (!mbar_wait(&empty[s], (uint32_t)(((it / kStages) & 1) ^ 1), p.err)) {
@@ -484,9 +532,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           uint8_t* a = ring + s * kStageBytes;
-          mbar_expect_tx(&full[s], kStageBytes);
+          mbar_expect_tx(&full[s], kBytesA + (uint32_t)cols * kTileK * 2);
           tma_load_2d(a, &map_s, &full[s], k * kTileK, m0);
-          tma_load_2d(a + kBytesA, &map_w, &full[s], k * kTileK, n0);
+          tma_load_2d(a + kBytesA, w, &full[s], k * kTileK, n0);
         }
       }
       /* leave no copy in flight: the last use of every slot completes */
@@ -507,6 +555,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!mbar_wait(&acc_empty[j], (uint32_t)(((li >> 1) & 1) ^ 1), p.err)) break;
         tc_fence_after();
         const uint32_t acc = tmem + (uint32_t)(j * kTileN);
+        int m0, n0, cols;
+        tiles.at(t, m0, n0, cols);
+        const uint32_t idesc = umma_idesc(cols);
         for (int k = 0; k < kIters; k++, it++) {
           const int s = (int)(it % kStages);
           if (!mbar_wait(&full[s], (uint32_t)((it / kStages) & 1), p.err)) {
@@ -519,7 +570,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int kk = 0; kk < kTileK / kUmmaK; kk++) {
             /* +32 bytes along K inside the 128-byte swizzled row */
-            umma(acc, smem_desc(a + kk * 32), smem_desc(b + kk * 32), (k > 0 || kk > 0) ? 1u : 0u);
+            umma(acc, smem_desc(a + kk * 32), smem_desc(b + kk * 32), idesc, (k > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&empty[s]);
         }
@@ -532,25 +583,32 @@ __global__ void __launch_bounds__(kThreads, 1)
     int li = 0;
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, li++) {
       const int j = li & 1;
-      const int m0 = (t / nN) * kTileM, n0 = (t % nN) * kTileN;
+      int m0, n0, cols;
+      tiles.at(t, m0, n0, cols);
+      const int row = m0 + q * 32 + lane;
+      const size_t base = (size_t)row * p.N + n0;
+      float4 e[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) e[i] = *reinterpret_cast<const float4*>(p.epsc_prev + base + 4 * i);
       /* warp-uniform: tcgen05.ld is .sync.aligned */
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[j], (uint32_t)((li >> 1) & 1), p.err) ? 1 : 0) != 0;
       if (!ok) break;
       tc_fence_after();
-      const int row = m0 + q * 32 + lane;
-      const size_t base = (size_t)row * p.N + n0;
-      for (int c = 0; c < kTileN; c += 32) {
+      for (int c = 0; c < cols; c += 32) {
         float acc[32];
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(j * kTileN + c), acc);
+        if (c > 0) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          float4 e = *reinterpret_cast<const float4*>(p.epsc_prev + base + c + i);
+        for (int i = 0; i < 8; i++) e[i] = *reinterpret_cast<const float4*>(p.epsc_prev + base + c + 4 * i);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
           float4 o;
-          o.x = e.x * p.one_m_kepsc + acc[i];
-          o.y = e.y * p.one_m_kepsc + acc[i + 1];
-          o.z = e.z * p.one_m_kepsc + acc[i + 2];
-          o.w = e.w * p.one_m_kepsc + acc[i + 3];
-          *reinterpret_cast<float4*>(p.epsc_cur + base + c + i) = o;
+          o.x = e[i].x * p.one_m_kepsc + acc[4 * i];
+          o.y = e[i].y * p.one_m_kepsc + acc[4 * i + 1];
+          o.z = e[i].z * p.one_m_kepsc + acc[4 * i + 2];
+          o.w = e[i].w * p.one_m_kepsc + acc[4 * i + 3];
+          *reinterpret_cast<float4*>(p.epsc_cur + base + c + 4 * i) = o;
         }
       }
       tc_fence_before();
@@ -1067,7 +1125,8 @@ struct bcpnn_recall {
   long long kk = 0; /* ticks run since load */
   int counted = 0;   /* counted ticks since the counters were cleared */
   CUtensorMap map_s[4];
-  CUtensorMap map_w;
+  WMaps map_w;           /* BF16: boxes of a tile's columns and of its parts */
+  CUtensorMap map_wf;    /* FP32: boxes of the event kernel */
   uint4* lists[2] = {nullptr, nullptr}; /* spike lists of a tick, by tick parity (recall_lists_kernel) */
   uint8_t* list_cnt[2] = {nullptr, nullptr};
   bool finite_w = false; /* FP32 contraction: every loaded weight is finite */
@@ -1206,13 +1265,13 @@ int bcpnn_recall_create(const bcpnn_recall_desc* d, bcpnn_recall** out) {
     return bad(BCPNN_ERR_CUDA);
   if (!fp32) {
     for (int i = 0; i < 4 && !rc; i++) rc = encode_map(r, &r->map_s[i], r->s[i], R, (int)N, kTileM);
-    if (!rc) rc = encode_map(r, &r->map_w, r->wt, (int)N, (int)N, kTileN);
+    for (int i = 0; i <= kMaxPartsLog && !rc; i++) rc = encode_map(r, &r->map_w.of[i], r->wt, (int)N, (int)N, kTileN >> i);
     if (rc) return bad(rc);
     if (cudaFuncSetAttribute(recall_tick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) !=
         cudaSuccess)
       return bad(BCPNN_ERR_CUDA);
   } else {
-    if ((rc = encode_map(r, &r->map_w, r->wf, (int)N, (int)N, kEvBox, true))) return bad(rc);
+    if ((rc = encode_map(r, &r->map_wf, r->wf, (int)N, (int)N, kEvBox, true))) return bad(rc);
     for (int i = 0; i < 2; i++)
       if ((rc = dalloc(r, &r->lists[i], (size_t)R * ((N + kEvRows - 1) / kEvRows) * (kEvListWords / 4))) ||
           (rc = dalloc(r, &r->list_cnt[i], (size_t)R * ((N + kEvRows - 1) / kEvRows))))
@@ -1367,8 +1426,8 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   p.pr_count = !p.poisson ? 0u : p.pr >= 1.0f ? 1u << 24 : (uint32_t)std::ceil((double)p.pr * 0x1p24);
   p.seed_base = d.seed_base;
   p.err = r->err;
-  const int n_tiles = (r->N / kTileN) * (d.replicates / kTileM);
-  const int grid = n_tiles < r->sms ? n_tiles : r->sms;
+  const Tiles tiles(d.replicates, r->N, r->sms);
+  const int grid = tiles.total < r->sms ? tiles.total : r->sms;
   const int f32_tiles = (r->N / kF32BN) * (d.replicates / kF32BM);
   const int pop_blocks = (int)((size_t)d.replicates * d.hcu_num * 4 / 256);
   void (*pop)(Params) = nullptr;
@@ -1419,12 +1478,12 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
     RCU(cudaGetLastError());
     if (r->timing) RCU(cudaEventRecord(r->tev[2 * i], r->stream));
     if (events)
-      recall_events_kernel<<<ev_grid, kEvThreads, kEvSmemBytes, r->stream>>>(r->map_w, r->sb[mod4(kk - 3)], r->lists[cur],
+      recall_events_kernel<<<ev_grid, kEvThreads, kEvSmemBytes, r->stream>>>(r->map_wf, r->sb[mod4(kk - 3)], r->lists[cur],
                                                                            r->list_cnt[cur], p);
     else if (r->wf)
       recall_fp32_kernel<<<f32_tiles, kF32Threads, 0, r->stream>>>(r->sb[mod4(kk - 3)], r->wf, p);
     else
-      recall_tick_kernel<<<grid, kThreads, kSmemBytes, r->stream>>>(r->map_s[mod4(kk - 3)], r->map_w, p);
+      recall_tick_kernel<<<grid, kThreads, kSmemBytes, r->stream>>>(r->map_s[mod4(kk - 3)], r->map_w, p, r->sms);
     RCU(cudaGetLastError());
     if (r->timing) RCU(cudaEventRecord(r->tev[2 * i + 1], r->stream));
     /* both kernels of tick kk are queued: each stream waits for the other's
