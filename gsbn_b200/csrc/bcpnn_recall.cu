@@ -77,6 +77,7 @@ struct Params {
   uint32_t seed_base;
   int simstep;
   int poisson;
+  float one; /* 1, see add2m */
   uint32_t pr_count; /* a 24-bit uniform k 2^-24 is below pr for k < pr_count */
   int* err;
 };
@@ -197,7 +198,10 @@ __device__ __forceinline__ float dsup_mcu0(const Params& p, int row, uint32_t se
   return d + (sup - d) * p.taumdt;
 }
 
-/* two IEEE additions in one instruction, as a 64-bit register pair */
+/* two IEEE operations in one instruction, as a 64-bit register pair.  A sum
+   that may take a product is add2m, a multiply-add by a 1 that the compiler does
+   not know: a product before an add.rn.f32x2 came out as one multiply-add with
+   one rounding. */
 typedef unsigned long long f32x2;
 
 __device__ __forceinline__ f32x2 pack2(float a, float b) {
@@ -205,6 +209,7 @@ __device__ __forceinline__ f32x2 pack2(float a, float b) {
 }
 __device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 dup2(float a) { return pack2(a, a); }
 
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   f32x2 c;
@@ -212,32 +217,38 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   return c;
 }
 
-/* two products, one by one: a mul.rn.f32x2, or a multiply-add of -0, before an
-   add.rn.f32x2 came out as one multiply-add with one rounding */
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { return pack2(lo2(a) * lo2(b), hi2(a) * hi2(b)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 c;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
+}
 
-__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
-__device__ __forceinline__ f32x2 dup2(float a) { return pack2(a, a); }
+/* a * unit + b, unit = 1: a + b; unit = -1: b - a */
+__device__ __forceinline__ f32x2 add2m(f32x2 a, f32x2 b, f32x2 unit) {
+  f32x2 c;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(c) : "l"(a), "l"(unit), "l"(b));
+  return c;
+}
 
 /* bx_expf of two values in (kExpLow, 0], where its result is normal: the same
    operations on pairs, without its clamps and its two-step scaling (the result
    is the polynomial's bits plus the exponent).  Same bits. */
 constexpr float kExpLow = -83.0f;
 
-__device__ __forceinline__ f32x2 exp2_near(f32x2 x) {
+__device__ __forceinline__ f32x2 exp2_near(f32x2 x, f32x2 one, f32x2 neg) {
   const f32x2 shift = dup2(0x1.8p23f);
-  const f32x2 t = add2(mul2(x, dup2(0x1.715476p+0f)), shift);
-  const f32x2 kf = add2(t, neg2(shift));
-  const f32x2 r = add2(add2(x, neg2(mul2(kf, dup2(0x1.62e4p-1f)))), neg2(mul2(kf, dup2(0x1.7f7d1cp-20f))));
+  const f32x2 t = add2m(mul2(x, dup2(0x1.715476p+0f)), shift, one);
+  const f32x2 kf = add2m(shift, t, neg);
+  const f32x2 r = add2m(mul2(kf, dup2(0x1.7f7d1cp-20f)), add2m(mul2(kf, dup2(0x1.62e4p-1f)), x, neg), neg);
   f32x2 p = dup2(0x1.a01a02p-16f);
-  p = add2(mul2(p, r), dup2(0x1.a01a02p-13f));
-  p = add2(mul2(p, r), dup2(0x1.6c16c2p-10f));
-  p = add2(mul2(p, r), dup2(0x1.111112p-7f));
-  p = add2(mul2(p, r), dup2(0x1.555556p-5f));
-  p = add2(mul2(p, r), dup2(0x1.555556p-3f));
-  p = add2(mul2(p, r), dup2(0.5f));
-  p = add2(mul2(p, r), dup2(1.0f));
-  p = add2(mul2(p, r), dup2(1.0f));
+  p = add2m(mul2(p, r), dup2(0x1.a01a02p-13f), one);
+  p = add2m(mul2(p, r), dup2(0x1.6c16c2p-10f), one);
+  p = add2m(mul2(p, r), dup2(0x1.111112p-7f), one);
+  p = add2m(mul2(p, r), dup2(0x1.555556p-5f), one);
+  p = add2m(mul2(p, r), dup2(0x1.555556p-3f), one);
+  p = add2m(mul2(p, r), dup2(0.5f), one);
+  p = add2m(mul2(p, r), dup2(1.0f), one);
+  p = add2m(mul2(p, r), dup2(1.0f), one);
   /* t's low bits are k + 2^22 (mod 2^9 all that shifts in): k << 23 */
   const uint32_t a = (uint32_t)p + ((uint32_t)t << 23), b = (uint32_t)(p >> 32) + ((uint32_t)(t >> 32) << 23);
   return (f32x2)a | ((f32x2)b << 32);
@@ -254,11 +265,12 @@ __device__ __forceinline__ f32x2 exp2_near(f32x2 x) {
    leaves room on its SM for three of its CTAs.
 
    Bound by instruction issue: two Philox4x32-10 calls of about 50 instructions
-   per four MCUs, one exp per MCU.  The additions of support and exp run on pairs of MCUs.  The division of a spike's activity by the HCU's sum is done
+   per four MCUs, one exp per MCU.  Support and exp run on pairs of MCUs in one
+   instruction.  The division of a spike's activity by the HCU's sum is done
    only where the uniform is below the activity times maxfq dt / sum, rounded up
-   by 2^-20: about one MCU in 500 here; the comparison decides as if every MCU
-   divided (the exact product is below that bound by more than its roundings,
-   and a uniform of 0 always takes the exact path).  The recall counters are
+   by 2^-20: about one group of four in 150 here; the comparison decides as if
+   every MCU divided (the exact product is below that bound by more than its
+   roundings, and a uniform of 0 always takes the exact path).  The recall counters are
    touched only where a group has a spike.  kBits: the spikes as bits, for the
    FP32 contraction.  64 x 64, 4096 replicates: 100 us alone as one exp and one
    division per MCU, with 16 contiguous MCUs per lane. */
@@ -290,6 +302,7 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
   const int lg = p.lgidx[(size_t)r * p.H + h];
   const float wm = p.wgain * p.wmask[(size_t)r * p.H + h];
   const float base_hit = p.lgbias + p.igain * p.lg_hit, base_miss = p.lgbias + p.igain * p.lg_miss;
+  const f32x2 one = dup2(p.one), neg = dup2(-p.one);
   f32x2 d[2 * G];
 #pragma unroll
   for (int i = 0; i < G; i++) {
@@ -312,8 +325,8 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
                            add2(dup2(0.0f), add2(pack2(bb.z, bb.w), pack2(ep.z, ep.w)))};
 #pragma unroll
     for (int v = 0; v < 2; v++) {
-      const f32x2 s2 = add2(pack2(sup[2 * v], sup[2 * v + 1]), mul2(dup2(wm), wsup[v]));
-      d[2 * i + v] = add2(dv[v], mul2(add2(s2, neg2(dv[v])), dup2(p.taumdt)));
+      const f32x2 s2 = add2m(mul2(dup2(wm), wsup[v]), pack2(sup[2 * v], sup[2 * v + 1]), one);
+      d[2 * i + v] = add2m(mul2(add2m(dv[v], s2, neg), dup2(p.taumdt)), dv[v], one);
     }
   }
   float mx = seed0; /* the new dsup of population MCU 0 (also d[0] of HCU 0's first quarter) */
@@ -329,12 +342,12 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
   bool near = true;
 #pragma unroll
   for (int i = 0; i < 2 * G; i++) {
-    a[i] = mul2(dup2(p.wtagain), add2(d[i], neg2(dup2(mx))));
+    a[i] = mul2(dup2(p.wtagain), add2m(dup2(mx), d[i], neg));
     near = near & (lo2(a[i]) > kExpLow) & (hi2(a[i]) > kExpLow) & (lo2(a[i]) <= 0.0f) & (hi2(a[i]) <= 0.0f);
   }
   if (near) {
 #pragma unroll
-    for (int i = 0; i < 2 * G; i++) a[i] = exp2_near(a[i]);
+    for (int i = 0; i < 2 * G; i++) a[i] = exp2_near(a[i], one, neg);
   } else {
 #pragma unroll 1
     for (int i = 0; i < 2 * G; i++) {
@@ -358,8 +371,8 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
       const float v = (((vs + lo2(a[2 * i])) + hi2(a[2 * i])) + lo2(a[2 * i + 1])) + hi2(a[2 * i + 1]);
       vs = __shfl_sync(0xffffffffu, v, (lane & ~3) | s);
     }
-  /* above every product (act / vs) * maxfqdt, in units of 2^-24 */
-  const float bound = (vs > 1.0f ? p.maxfqdt / vs : p.maxfqdt) * (0x1p24f * (1.0f + 0x1p-20f));
+  /* above every product (act / vs) * maxfqdt, in units of 2^-32 */
+  const float bound = (vs > 1.0f ? p.maxfqdt / vs : p.maxfqdt) * (0x1p32f * (1.0f + 0x1p-20f));
 #pragma unroll
   for (int i = 0; i < G; i++)
     *reinterpret_cast<float4*>(p.dsup_cur + row + c0 + (4 * i + q) * 4) =
@@ -373,28 +386,33 @@ __global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
     cu.v[1] = (uint32_t)p.simstep;
     cu.v[2] = 0u;
     cu.v[3] = 0u;
-    const bx_u32x4 ou = bx_philox4x32_10(cu, seed, 0u * 16u + BX_STREAM_UNIFORM);
     uint32_t bits = 0u;
-    const float av[4] = {lo2(a[2 * i]), hi2(a[2 * i]), lo2(a[2 * i + 1]), hi2(a[2 * i + 1])};
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if ((float)(ou.v[k] >> 8) <= av[k] * bound) {
-        float act = av[k];
-        if (vs > 1.0f) act /= vs;
-        if (bx_u01(ou.v[k]) < act * p.maxfqdt) bits |= 1u << k;
-      }
     if (p.poisson) {
       const bx_u32x4 op = bx_philox4x32_10(cu, seed, 0u * 16u + BX_STREAM_POISSON);
 #pragma unroll
       for (int k = 0; k < 4; k++)
         if ((op.v[k] >> 8) < p.pr_count) bits |= 1u << k;
     }
+    const bx_u32x4 ou = bx_philox4x32_10(cu, seed, 0u * 16u + BX_STREAM_UNIFORM);
+    const float av[4] = {lo2(a[2 * i]), hi2(a[2 * i]), lo2(a[2 * i + 1]), hi2(a[2 * i + 1])};
+    /* the uniform is x >> 8: x itself against the bound plus the low byte */
+    bool near_spike = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) near_spike |= (float)ou.v[k] <= av[k] * bound + 257.0f;
+    if (near_spike) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        float act = av[k];
+        if (vs > 1.0f) act /= vs;
+        if (bx_u01(ou.v[k]) < act * p.maxfqdt) bits |= 1u << k;
+      }
+    }
     if (!kBits) {
       /* BF16 1.0 = 0x3F80 */
       uint32_t w[2];
 #pragma unroll
       for (int k = 0; k < 2; k++)
-        w[k] = (((bits >> (2 * k)) & 1u) ? 0x3F80u : 0u) | ((((bits >> (2 * k + 1)) & 1u) ? 0x3F80u : 0u) << 16);
+        w[k] = ((bits >> (2 * k)) & 1u) * 0x3F80u + ((bits >> (2 * k + 1)) & 1u) * 0x3F800000u;
       *reinterpret_cast<uint2*>(p.s_out + row + c0 + m) = make_uint2(w[0], w[1]);
     }
     if (p.count_on && bits) {
@@ -1423,6 +1441,7 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   p.one_m_kepsc = 1.0f - d.kepsc;
   p.pr = d.poisson_noise_hz * d.dt;
   p.poisson = d.poisson_noise_hz > 0.f;
+  p.one = 1.0f;
   p.pr_count = !p.poisson ? 0u : p.pr >= 1.0f ? 1u << 24 : (uint32_t)std::ceil((double)p.pr * 0x1p24);
   p.seed_base = d.seed_base;
   p.err = r->err;
