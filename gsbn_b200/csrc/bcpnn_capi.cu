@@ -104,9 +104,10 @@ struct bcpnn_net {
   std::vector<PopDev> hp;   /* host images of the per-population descriptors */
   std::vector<ProjDev> hq;  /* host images of the per-projection descriptors */
   std::vector<TabRef> tabs; /* host image of the run's decay-table references */
+  std::vector<TabRef> tabs_old; /* ... and of its catch-up's */
   PopDev* d_pops = nullptr;
   ProjDev* d_projs = nullptr;
-  TabRef* d_tabs = nullptr;
+  TabRef* d_tabs = nullptr; /* tabs, then tabs_old */
   NetDev* d_net = nullptr;
   RunParams rp;             /* host image of the run parameters */
   RunParams* d_rp = nullptr;
@@ -411,7 +412,7 @@ int reset_state(bcpnn_net* net) {
 constexpr int kBeginProjs = 8, kBeginPops = 8;
 struct RunBegin {
   RunParams rp;
-  TabRef tabs[kBeginProjs];
+  TabRef tabs[2 * kBeginProjs]; /* tabs, tabs_old */
   uint32_t* zero[kBeginPops + 2];
   unsigned int words[kBeginPops + 2];
   int n_zero, n_tabs;
@@ -435,6 +436,8 @@ int begin_run(bcpnn_net* net, int n_ticks) {
       (size_t)n_ticks * net->log_words_per_tick > (1u << 30) || ss_words > (1u << 30)) {
     CU(cudaMemcpyAsync(net->d_tabs, net->tabs.data(), net->tabs.size() * sizeof(TabRef), cudaMemcpyHostToDevice,
                        net->stream));
+    CU(cudaMemcpyAsync(net->d_tabs + net->tabs.size(), net->tabs_old.data(), net->tabs_old.size() * sizeof(TabRef),
+                       cudaMemcpyHostToDevice, net->stream));
     CU(cudaMemcpyAsync(net->d_rp, &net->rp, sizeof(RunParams), cudaMemcpyHostToDevice, net->stream));
     int rc;
     for (const PopHost& P : net->pops)
@@ -445,8 +448,12 @@ int begin_run(bcpnn_net* net, int n_ticks) {
   RunBegin b;
   std::memset(&b, 0, sizeof(b));
   b.rp = net->rp;
-  for (size_t p = 0; p < net->projs.size(); ++p) b.tabs[p] = net->tabs[p];
-  b.n_tabs = (int)net->projs.size();
+  const size_t nt = net->tabs.size();
+  for (size_t p = 0; p < nt; ++p) {
+    b.tabs[p] = net->tabs[p];
+    b.tabs[nt + p] = net->tabs_old[p];
+  }
+  b.n_tabs = (int)(2 * nt);
   size_t most = 0;
   auto zero = [&](uint32_t* p, size_t words) {
     b.zero[b.n_zero] = p;
@@ -475,8 +482,8 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
   if (with_all && !net->multi) {
     for (int p = 0; p < net->h.n_projs; ++p) {
       const ProjHost& J = net->projs[p];
-      all_rows_kernel<<<grid_for((size_t)J.H * J.C, 256), 256, 0, net->stream>>>(net->d_net, net->d_rp, p);
-      all_cells_kernel<<<grid_for((size_t)J.H * J.C * J.M, 256), 256, 0, net->stream>>>(net->d_net, net->d_rp, p);
+      const int rows = sweep_rows(J.M), R = J.H * J.C;
+      all_cells_kernel<<<(R + rows - 1) / rows, 256, 0, net->stream>>>(net->d_net, net->d_rp, p);
     }
   }
   size_t smem = net->tick_smem;
@@ -848,6 +855,7 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
   net->hp.assign(desc->n_pops, PopDev());
   net->hq.assign(desc->n_projs, ProjDev());
   net->tabs.assign(std::max(1, desc->n_projs), TabRef());
+  net->tabs_old = net->tabs;
   for (int p = 0; p < desc->n_pops; ++p) {
     PopHost P;
     P.d = desc->pops[p];
@@ -1056,10 +1064,11 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
   if ((rc = dalloc(net, &net->d_rp, 1))) return bail(rc);
   if ((rc = dalloc(net, &net->d_pops, net->hp.size()))) return bail(rc);
   if ((rc = dalloc(net, &net->d_projs, std::max<size_t>(1, net->hq.size())))) return bail(rc);
-  if ((rc = dalloc(net, &net->d_tabs, net->tabs.size()))) return bail(rc);
+  if ((rc = dalloc(net, &net->d_tabs, 2 * net->tabs.size()))) return bail(rc);
   H.pops = net->d_pops;
   H.projs = net->d_projs;
   net->rp.tabs = net->d_tabs;
+  net->rp.tabs_old = net->d_tabs + net->tabs.size();
   if (cudaMemcpy(net->d_pops, net->hp.data(), net->hp.size() * sizeof(PopDev), cudaMemcpyHostToDevice) != cudaSuccess ||
       (!net->hq.empty() &&
        cudaMemcpy(net->d_projs, net->hq.data(), net->hq.size() * sizeof(ProjDev), cudaMemcpyHostToDevice) != cudaSuccess) ||
@@ -1543,11 +1552,12 @@ int bcpnn_run(bcpnn_net* net, int32_t first_simstep, int32_t n_ticks, float prn,
     net->tabs[p].k = make_coef(net->hq[p].taupdt * prn, net->hq[p].ke, net->hq[p].kzi, net->hq[p].kzj, net->hq[p].fp64);
     net->tabs[p].len = J.slot[s].len;
     if (with_all) {
-      net->tabs[p].tab_old = J.slot[so].ptr;
-      net->tabs[p].old_len = J.slot[so].len;
-    } else {
-      net->tabs[p].tab_old = nullptr;
-      net->tabs[p].old_len = 0;
+      TabRef& O = net->tabs_old[p];
+      O.tab = J.slot[so].ptr;
+      O.rtab = J.slot[so].rptr;
+      O.len = J.slot[so].len;
+      O.rk = rcoef(net->hq[p], old_prn);
+      O.k = make_coef(net->hq[p].taupdt * old_prn, net->hq[p].ke, net->hq[p].kzi, net->hq[p].kzj, net->hq[p].fp64);
     }
   }
   net->rp.simstep0 = first_simstep;
@@ -1584,7 +1594,7 @@ int bcpnn_run(bcpnn_net* net, int32_t first_simstep, int32_t n_ticks, float prn,
     net->launches += (net->multi_persistent ? 1u : (uint64_t)n_ticks * (1 + net->projs.size())) +
                      (with_all ? net->projs.size() : 0u);
   else
-    net->launches += (uint64_t)(net->persistent ? 1 : n_ticks) + (with_all ? 2u * net->projs.size() : 0u);
+    net->launches += (uint64_t)(net->persistent ? 1 : n_ticks) + (with_all ? net->projs.size() : 0u);
   if (with_all)
     for (const ProjHost& J : net->projs) net->all_cells += (uint64_t)J.H * J.C * J.M;
   net->k_total += n_ticks;

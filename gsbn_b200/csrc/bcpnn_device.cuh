@@ -22,9 +22,9 @@
  *   - Values read across CTAs inside a tick (the population's MCU-0 support
  *     that seeds every HCU's softmax max, Pop.cpp:270; si) are double
  *     buffered by tick parity: a tick reads buffer prev and writes buffer cur.
- *   - all_rows_kernel / all_cells_kernel: the all-cells catch-up at a change
- *     of prn (Proj.cpp:209-308, 538-588), a streaming pass over every row and
- *     every cell.
+ *   - all_cells_kernel: the all-cells catch-up at a change of prn
+ *     (Proj.cpp:209-308, 538-588), a streaming pass over every row and every
+ *     cell.
  *   - The closed-form decay factors depend on the elapsed ticks pdt only; they
  *     are tabulated per projection and per kp by build_table_kernel with the
  *     same float expressions the reference evaluates inline, so a table
@@ -161,7 +161,8 @@ struct RunParams {
   float prn, old_prn;
   const float* lginp;   /* stimulus of the run: [total MCUs] */
   const float* wmask;   /* [total HCUs] */
-  const struct TabRef* tabs;  /* [n_projs] decay tables of the run */
+  const struct TabRef* tabs;  /* [n_projs] decay tables of the run, kp = taupdt*prn */
+  const struct TabRef* tabs_old; /* [n_projs] of its catch-up, kp = taupdt*old_prn (set when they differ) */
   unsigned int serial0; /* tag of the run's first tick (never repeats between consecutive ticks, see seed64) */
 };
 
@@ -191,14 +192,13 @@ struct RCoef {
   double Dekp, D2, D3, Dpzi, Dezi;
 };
 
-/* decay tables of one projection for a run */
+/* decay tables of one projection for a run, for one kp */
 struct TabRef {
-  const float4* tab;      /* kp = taupdt*prn     */
-  const float4* tab_old;  /* kp = taupdt*old_prn */
-  const double2* rtab;    /* kp = taupdt*prn: reciprocals of the divisor entries, see build_table_kernel */
-  int len, old_len;
-  Coef k;                 /* kp = taupdt*prn */
-  RCoef rk;               /* kp = taupdt*prn */
+  const float4* tab;
+  const double2* rtab;    /* reciprocals of the divisor entries, see build_table_kernel */
+  int len;
+  Coef k;
+  RCoef rk;
 };
 
 
@@ -610,62 +610,108 @@ __global__ void build_table_kernel(float4* tab, double2* rtab, int len, float kp
   }
 }
 
-/* All-cells catch-up, row part (Proj.cpp:234-254): every row with
-   pdt = simstep-1-ti > 0. */
-__global__ void all_rows_kernel(const NetDev* __restrict__ net, const RunParams* __restrict__ rp, int p) {
-  const ProjDev& J = net->projs[p];
-  int simstep = rp->simstep0 - 1;
-  float kp = J.taupdt * rp->old_prn;
-  Coef k = make_coef(kp, J.ke, J.kzi, J.kzj, J.fp64);
-  const float4* tab = rp->tabs[p].tab_old;
-  int len = rp->tabs[p].old_len;
-  int R = J.H * J.C;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    int pdt = simstep - J.ti[r];
-    if (pdt > 0) {
-      float pi = J.pi[r], ei = J.ei[r], zi = J.zi[r];
-      float4 A, B;
-      load_entry(tab, len, k, pdt, 2, A, B);
-      row_decay(pi, ei, zi, k, A, B);
-      J.pi[r] = pi;
-      J.ei[r] = ei;
-      J.zi[r] = zi;
-      J.ti[r] = simstep;
-    }
+/* one decay of a cell (row traces) on the float closed-form path, in line; the
+   exact fallback and the FP64-built propagators out of line */
+__device__ __forceinline__ float4 cell_step(float4 c, const TabRef& T, float4 A, float4 B, double2 R0, double2 R1) {
+  float4 f = c;
+  if (!T.k.fp64 && cell_decay_fast(f, T.k, T.rk, A, B, R0, R1)) return f;
+  return cell_step_nl(c, &T, A, B, R0, R1);
+}
+
+__device__ __forceinline__ float4 row_step(float4 r, const TabRef& T, float4 A, float4 B, double2 R0, double2 R1) {
+  float4 f = r;
+  if (!T.k.fp64 && row_decay_fast(f, T.k, T.rk, A, B, R0, R1)) return f;
+  return row_step_nl(r, &T, A, B, R0, R1);
+}
+
+/* an entry beyond the table, computed; out of line, it is never needed while
+   the tables cover a run */
+struct Entry {
+  float4 A, B;
+  double2 R0, R1;
+};
+
+__device__ __noinline__ Entry entry_beyond(const TabRef& T, int pdt, int part) {
+  Entry e;
+  load_entry(T.tab, T.len, T.k, pdt, part, e.A, e.B);
+  recip_part(e.A, e.B, part, e.R0, e.R1);
+  return e;
+}
+
+/* part 0 (cells) or 2 (rows) of the table entry of pdt > 0 elapsed ticks */
+__device__ __forceinline__ void entry(const TabRef& T, int pdt, int part, float4& A, float4& B, double2& R0, double2& R1) {
+  if (pdt < T.len) {
+    A = T.tab[(size_t)pdt * 4 + part];
+    B = T.tab[(size_t)pdt * 4 + part + 1];
+    R0 = T.rtab[(size_t)pdt * 4 + part];
+    R1 = T.rtab[(size_t)pdt * 4 + part + 1];
+  } else {
+    const Entry e = entry_beyond(T, pdt, part);
+    A = e.A;
+    B = e.B;
+    R0 = e.R0;
+    R1 = e.R1;
   }
 }
 
-/* All-cells catch-up, cell part (Proj.cpp:256-307).  Runs after
-   all_rows_kernel so w_ij sees the updated pi. */
-__global__ void all_cells_kernel(const NetDev* __restrict__ net, const RunParams* __restrict__ rp, int p) {
-  const ProjDev& J = net->projs[p];
-  int simstep = rp->simstep0 - 1;
-  float kp = J.taupdt * rp->old_prn;
-  Coef k = make_coef(kp, J.ke, J.kzi, J.kzj, J.fp64);
-  const float4* tab = rp->tabs[p].tab_old;
-  int len = rp->tabs[p].old_len;
-  size_t ncell = (size_t)J.H * J.C * J.M;
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += (size_t)gridDim.x * blockDim.x) {
-    int pdt = simstep - J.tij[c];
-    if (pdt <= 0) {
-      J.tij[c] = simstep;
-    } else {
-      float4 q = J.cell[c];
-      float4 A, B;
-      load_entry(tab, len, k, pdt, 0, A, B);
-      cell_decay(q.x, q.y, q.z, q.w, k, A, B);
-      J.cell[c] = q;
-      J.tij[c] = simstep;
-      if (kp != 0.0f) {
-        int r = (int)(c / J.M);
-        int j = (int)(c - (size_t)r * J.M);
-        int h = r / J.C;
-        float pi = J.pi[r];
-        float pj = J.pj[h * J.M + j];
-        J.wij[c] = J.wgain * dev_logf((q.x + J.eps2) / ((pi + J.eps) * (pj + J.eps)));
-      }
+/* Rows of one block of the all-cells catch-up: about kSweepCells cells. */
+constexpr int kSweepCells = 2048;
+__host__ __device__ inline int sweep_rows(int M) { return kSweepCells / M < 1 ? 1 : kSweepCells / M; }
+
+/* All-cells catch-up (Proj.cpp:209-308, 538-588) of rows [row0, row0 + nr) of
+   one projection to tick simstep, by one block: the row traces (Proj.cpp:234-254)
+   of every row with simstep - ti > 0, then its cells (Proj.cpp:256-307), whose
+   weights see the new pi.  J: a ProjDev or a batch member.  By reciprocals, as
+   the tick's decays; bound by instruction issue (a decay, a division and a log
+   per cell), 44 bytes a cell would take 0.07 ms for 1e7 cells.  0.40 -> 0.23 ms
+   there against a launch for the rows, one for the cells with exact division and
+   two 64-bit divisions of every index. */
+template <class J>
+__device__ __forceinline__ void sweep_block(const J& B, const TabRef& T, int row0, int nr, int simstep, float kp, float wgain) {
+  for (int t = threadIdx.x; t < nr; t += blockDim.x) {
+    const int r = row0 + t, pdt = simstep - B.ti[r];
+    if (pdt > 0) {
+      float4 A, Bt;
+      double2 R0, R1;
+      entry(T, pdt, 2, A, Bt, R0, R1);
+      const float4 rt = row_step(make_float4(B.pi[r], B.ei[r], B.zi[r], 0.0f), T, A, Bt, R0, R1);
+      B.pi[r] = rt.x;
+      B.ei[r] = rt.y;
+      B.zi[r] = rt.z;
+      B.ti[r] = simstep;
     }
   }
+  __syncthreads();
+  const int M = B.M, C = B.C, h0 = row0 / C, s0 = row0 - h0 * C;
+  for (int c = threadIdx.x; c < nr * M; c += blockDim.x) {
+    const size_t x = (size_t)row0 * M + c;
+    const int pdt = simstep - B.tij[x];
+    if (pdt > 0) {
+      float4 A, Bt;
+      double2 R0, R1;
+      entry(T, pdt, 0, A, Bt, R0, R1);
+      const float4 q = cell_step(B.cell[x], T, A, Bt, R0, R1);
+      B.cell[x] = q;
+      if (kp != 0.0f) {
+        const int rr = c / M, j = c - rr * M;
+        const int s = s0 + rr, h = s < C ? h0 : h0 + s / C;
+        B.wij[x] = wgain * bx_logf((q.x + B.eps2) / ((B.pi[row0 + rr] + B.eps) * (B.pj[h * M + j] + B.eps)));
+      }
+    }
+    B.tij[x] = simstep;
+  }
+}
+
+__global__ void __launch_bounds__(256) all_cells_kernel(const NetDev* __restrict__ net, const RunParams* __restrict__ rp, int p) {
+  __shared__ ProjDev J;
+  __shared__ TabRef T;
+  if (threadIdx.x == 0) {
+    J = net->projs[p];
+    T = rp->tabs_old[p];
+  }
+  __syncthreads();
+  const int rows = sweep_rows(J.M), row0 = blockIdx.x * rows;
+  sweep_block(J, T, row0, min(rows, J.H * J.C - row0), rp->simstep0 - 1, J.taupdt * rp->old_prn, J.wgain);
 }
 
 /* ------------------------------------------------------------------------ */

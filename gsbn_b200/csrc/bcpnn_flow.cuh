@@ -164,50 +164,6 @@ __device__ __forceinline__ bool bar_any(int id, int n, bool flag) {
   return r != 0;
 }
 
-/* one decay of a cell (row traces) on the float closed-form path, in line; the
-   exact fallback and the FP64-built propagators out of line */
-__device__ __forceinline__ float4 cell_step(float4 c, const TabRef& T, float4 A, float4 B, double2 R0, double2 R1) {
-  float4 f = c;
-  if (!T.k.fp64 && cell_decay_fast(f, T.k, T.rk, A, B, R0, R1)) return f;
-  return cell_step_nl(c, &T, A, B, R0, R1);
-}
-
-__device__ __forceinline__ float4 row_step(float4 r, const TabRef& T, float4 A, float4 B, double2 R0, double2 R1) {
-  float4 f = r;
-  if (!T.k.fp64 && row_decay_fast(f, T.k, T.rk, A, B, R0, R1)) return f;
-  return row_step_nl(r, &T, A, B, R0, R1);
-}
-
-/* an entry beyond the table, computed; out of line, it is never needed while
-   the tables cover a run */
-struct Entry {
-  float4 A, B;
-  double2 R0, R1;
-};
-
-__device__ __noinline__ Entry entry_beyond(const TabRef& T, int pdt, int part) {
-  Entry e;
-  load_entry(T.tab, T.len, T.k, pdt, part, e.A, e.B);
-  recip_part(e.A, e.B, part, e.R0, e.R1);
-  return e;
-}
-
-/* part 0 (cells) or 2 (rows) of the table entry of pdt > 0 elapsed ticks */
-__device__ __forceinline__ void entry(const TabRef& T, int pdt, int part, float4& A, float4& B, double2& R0, double2& R1) {
-  if (pdt < T.len) {
-    A = T.tab[(size_t)pdt * 4 + part];
-    B = T.tab[(size_t)pdt * 4 + part + 1];
-    R0 = T.rtab[(size_t)pdt * 4 + part];
-    R1 = T.rtab[(size_t)pdt * 4 + part + 1];
-  } else {
-    const Entry e = entry_beyond(T, pdt, part);
-    A = e.A;
-    B = e.B;
-    R0 = e.R0;
-    R1 = e.R1;
-  }
-}
-
 /* shared-memory layout of a CTA, in 4-byte words */
 struct Layout {
   int act;                 /* [M rounded up to 4] */

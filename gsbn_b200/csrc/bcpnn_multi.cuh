@@ -1313,41 +1313,106 @@ __device__ __forceinline__ void res_tick_loop(const NetDev* __restrict__ net, co
 
 /* update_all_cpu (Proj.cpp:490-555) for projection p at a change of prn:
    every row and its cells caught up to simstep0-1 with kp = taupdt*old_prn,
-   replaying the ring up to and including that tick.  One warp per row. */
-__global__ void all_kernel(const NetDev* __restrict__ net, const RunParams* __restrict__ rp, int p) {
-  const ProjDev& J = net->projs[p];
+   replaying the ring up to and including that tick.  One warp per row, a run of
+   consecutive rows per warp: a lane's MCUs stay the same within an HCU, so their
+   ring, as a mask of the last ticks (bit b: tick simstep - b), is read once per
+   HCU and not once per cell.  For rings of at most 32 ticks and 128 MCUs, by
+   reciprocals as the tick's decays; else replay_cell.  1e7 cells, ring of 25:
+   1.45 ms with a walk over the ring and exact division per cell, 0.46 ms. */
+constexpr int kAllMasks = 4;
+
+__global__ void __launch_bounds__(256) all_kernel(const NetDev* __restrict__ net, const RunParams* __restrict__ rp, int p) {
+  __shared__ ProjDev J;
+  __shared__ TabRef T;
+  if (threadIdx.x == 0) {
+    J = net->projs[p];
+    T = rp->tabs_old[p];
+  }
+  __syncthreads();
   const PopDev& pop = net->pops[J.dest];
   const int M = J.M, C = J.C, n = pop.n, B = pop.ring_len;
   const int simstep = rp->simstep0 - 1;
   const float kp = J.taupdt * rp->old_prn;
-  const Coef k = make_coef(kp, J.ke, J.kzi, J.kzj);
-  const float4* tab = rp->tabs[p].tab_old;
-  const int tlen = rp->tabs[p].old_len;
   const int lane = threadIdx.x & 31;
   const int R = J.H * C;
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&net->counters[2], (unsigned long long)R * M);
-  for (int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < R; r += (gridDim.x * blockDim.x) >> 5) {
+  const int warps = (int)((gridDim.x * blockDim.x) >> 5), w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int per = (R + warps - 1) / warps;
+  const bool masks = B <= 32 && M <= 32 * kAllMasks;
+  uint32_t hist[kAllMasks] = {0u, 0u, 0u, 0u};
+  int h_of = -1;
+  for (int r = w * per; r < min(R, (w + 1) * per); ++r) {
     const int ti = J.ti[r];
     const float zi = J.zi[r];
     const int h = r / C;
     const int pdt = simstep - ti;
     float4 rA = make_float4(0, 0, 0, 0), rB = rA;
-    if (pdt > 0) entry(tab, tlen, k, pdt, 2, rA, rB);
+    double2 R0 = make_double2(0, 0), R1 = R0;
+    if (pdt > 0) bcpnn::entry(T, pdt, 2, rA, rB, R0, R1);
     if (lane == 0 && pdt > 0) {
-      float pi = J.pi[r], ei = J.ei[r], z = zi;
-      row_decay(pi, ei, z, k, rA, rB);
-      J.pi[r] = pi;
-      J.ei[r] = ei;
+      const float4 rt = row_step(make_float4(J.pi[r], J.ei[r], zi, 0.0f), T, rA, rB, R0, R1);
+      J.pi[r] = rt.x;
+      J.ei[r] = rt.y;
     }
     __syncwarp();
     const float pi_new = J.pi[r];
-    for (int j = lane; j < M; j += 32) {
-      const size_t index = (size_t)r * M + j;
-      float4 c4 = J.cell[index];
-      replay_cell(c4, ti, zi, simstep, 0, pop.ring, B, n, h * M + j, k, tab, tlen, nullptr, J.kftj, false);
+    if (masks && h != h_of) {
+      h_of = h;
+#pragma unroll
+      for (int v = 0; v < kAllMasks; ++v) {
+        const int j = lane + 32 * v;
+        uint32_t m = 0u;
+        if (j < M)
+          for (int b = 0; b < B && b <= simstep; ++b)
+            m |= (pop.ring[(size_t)((simstep - b) % B) * n + h * M + j] > 0 ? 1u : 0u) << b;
+        hist[v] = m;
+      }
+    }
+    auto finish = [&](int j, size_t index, const float4& c4) {
       J.cell[index] = c4;
       if (kp != 0.0f)
         J.wij[index] = J.wgain * bx_logf((c4.x + J.eps2) / ((pi_new + J.eps) * (J.pj[h * M + j] + J.eps)));
+    };
+    if (masks) {
+      /* ticks after max(ti, simstep - B + 1) up to simstep, ascending, as replay_cell visits them */
+      const int span = pdt >= B ? B - 1 : pdt;
+      const uint32_t window = span > 0 ? 0xffffffffu >> (32 - span) : 0u;
+#pragma unroll
+      for (int v = 0; v < kAllMasks; ++v) {
+        const int j = lane + 32 * v;
+        if (j >= M) continue;
+        const size_t index = (size_t)r * M + j;
+        float4 c4 = J.cell[index];
+        c4.z = zi;
+        int tij = ti;
+        uint32_t m = hist[v] & window;
+        while (m || simstep > tij) {
+          const int b = m ? 31 - __clz(m) : 0;
+          const bool spike = m != 0u;
+          m &= ~(1u << b);
+          const int d = simstep - b - tij;
+          float4 A, Bt;
+          double2 Q0, Q1;
+          bcpnn::entry(T, d, 0, A, Bt, Q0, Q1);
+          const float4 q = cell_step(c4, T, A, Bt, Q0, Q1);
+          c4.x = q.x;
+          c4.y = q.y;
+          c4.w = q.w;
+          if (spike) {
+            c4.z = q.z;
+            c4.w = c4.w + J.kftj;
+          }
+          tij = simstep - b;
+        }
+        finish(j, index, c4);
+      }
+    } else {
+      for (int j = lane; j < M; j += 32) {
+        const size_t index = (size_t)r * M + j;
+        float4 c4 = J.cell[index];
+        replay_cell(c4, ti, zi, simstep, 0, pop.ring, B, n, h * M + j, T.k, T.tab, T.len, nullptr, J.kftj, false);
+        finish(j, index, c4);
+      }
     }
     __syncwarp();
     if (lane == 0) {
