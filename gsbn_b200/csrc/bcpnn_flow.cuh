@@ -12,8 +12,8 @@
  *         pj(t), and the columns of t-1 (same cells); it gives epsc(t).  It
  *         does not need the spikes of t: zj alone takes them (Proj.cpp:349);
  *         columns  Proj.cpp:481-536, 722-760: the spikes of t, after its rows;
- *   Q(t)  delay queue  Proj.cpp:621-630, 645-664: the spikes of t-1 of every
- *         source HCU; it lists the active rows of t+1.
+ *   Q(t)  delay queue  Proj.cpp:621-630, 645-664: it lists the active rows of
+ *         t+1, then puts the spikes of t-1 of every source HCU into the queue.
  * The row traces (Proj.cpp:397-416) belong to the rows alone, so a warp of its
  * own, R(t), does those of the listed rows beside the decays of their cells.
  * The four groups run side by side and meet at shared-memory mbarriers: E(t) (W
@@ -27,18 +27,27 @@
  * Between CTAs a spike word carries its own flag: 32 spikes and the tick's tag
  * in 64 bits, one relaxed store, polled by every CTA's Q.  Q waits for the
  * words of all HCUs of the network, its sources or not, which bounds how far
- * CTAs run apart: P(t) needs Q(t-2), so a CTA that publishes t has seen every
- * word of t-3, and a CTA that published t-3 has read the words of t-6 and the
- * seed of t-3.  Words are kept for 8 ticks and seeds for 4.
+ * CTAs run apart: P(t) needs the list of Q(t-2), which comes after all of
+ * Q(t-3), so a CTA that publishes t has seen every word of t-4, and a CTA that
+ * published t-4 has read the words of t-8 and the seed of t-4.  Words are kept
+ * for 8 ticks and seeds for 4.
  *
  * Bound by the longest cycle of dependences: P(t) -> columns(t) -> rows(t+1) ->
  * P(t+2) takes two ticks, E(t-1) -> P(t) one.  Per tick, against tick_kernel with
  * its grid barrier and its columns spread over the grid: 10 x 10 2.2 us (7.4),
- * 50 x 50 2.9 (8.8), 100 x 100 with C = 1000 4.5 (9.9), 256 x 50 with C = 1000
- * 7.4 (13.8), 296 x 20 with C = 400 3.8 (11.3).  With the row traces in W and two
- * more barriers before the sum, decays as calls: 2.8, 3.7, 6.0, 9.7 and 5.7.  The decays and their exact
+ * 50 x 50 2.6 (8.8), 100 x 100 with C = 1000 4.0 (9.9), 256 x 50 with C = 1000
+ * 6.3 (13.8), 296 x 20 with C = 400 3.6 (11.3).  With the row traces in W and two
+ * more barriers before the sum, decays as calls, and a queue word of every slot
+ * shifted every tick: 2.8, 3.7, 6.0, 9.7 and 5.7.  The decays and their exact
  * division are those of bcpnn_device.cuh, so every value is bit-identical to
  * tick_kernel's and to the oracle's.
+ *
+ * The delay queue is kept by bit planes, a ring of 32 over the ticks: the rows
+ * due are the set bits of one plane, 32 slots a word, and a spike sets one bit of
+ * the plane its delay names.  Shifting every slot's own word took a warp 900
+ * cycles per 128 slots, on the path from one tick's rows to the next (100 x 100
+ * 4.4 -> 4.0 us per tick, 256 x 50 7.4 -> 6.3, 20 x 20 2.6 -> 2.2); and the list
+ * of the due rows no longer waits for the other HCUs' spikes.
  *
  * Every wait is bounded (kBarrierNs): it sets kErrBarrier and the CTA's abort
  * flag, the groups leave their tick loops together, and the state is not
@@ -54,7 +63,7 @@ namespace flow {
 
 constexpr int kMaxM = 128;        /* one MCU per thread of up to four warps */
 constexpr int kWordTicks = 8, kSeedTicks = 4;
-constexpr int kMaxWords = 2047;   /* word and bit of a source MCU in 16 bits, 0xffff: none */
+constexpr int kMaxWords = 2047;   /* word and bit of a source MCU in 16 bits; word n_words: none */
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
 struct Args {
@@ -167,19 +176,20 @@ __device__ __forceinline__ bool bar_any(int id, int n, bool flag) {
 /* shared-memory layout of a CTA, in 4-byte words */
 struct Layout {
   int act;                 /* [M rounded up to 4] */
-  int bits;                /* [n_words] the previous tick's spikes of the network */
+  int bits;                /* [n_words] the previous tick's spikes of the network, and a word of 0 */
   int w;                   /* [chunk cells] weights to add */
   int q[kMaxIn];           /* blocks of the incoming projections */
   int total;
 };
 
-/* slots per queue warp, a multiple of 32 */
-__host__ __device__ inline int queue_part(int C, int qw) { return ((C + qw - 1) / qw + 31) & ~31; }
+/* slots per queue warp, a multiple of 64 */
+__host__ __device__ inline int queue_part(int C, int qw) { return ((C + qw - 1) / qw + 63) & ~63; }
 
-/* a projection's block: pj ej zj bj [M], epsc [2][M], pjn [2][M]; qi [C], pi [2][C] (by list entry); then 16-bit list
-   [2][qw * part], src [C]; bytes di [C] */
+/* a projection's block: pj ej zj bj [M], epsc [2][M], pjn [2][M]; pi [2][C] (by list entry); then, of the n = qw * part
+   slots: bit planes of the delay queue [32][n / 32], 16-bit list [2][n] and src [n], bytes di [n] */
 __host__ __device__ inline int block_words(int M, int C, int qw) {
-  return 8 * M + 3 * C + (2 * qw * queue_part(C, qw) + C + 1) / 2 + (C + 3) / 4;
+  const int n = qw * queue_part(C, qw);
+  return 8 * M + 2 * C + n + n + n / 2 + n / 4;
 }
 
 __host__ __device__ inline int chunk_rows(int M, int cells) { return cells / M < 1 ? 1 : cells / M; }
@@ -187,7 +197,7 @@ __host__ __device__ inline int chunk_rows(int M, int cells) { return cells / M <
 __host__ __device__ inline void layout(int M, int n_in, const int* C, int n_words, int cells, int qw, Layout& L) {
   int o = 0;
   L.act = o; o += (M + 3) & ~3;
-  L.bits = o; o += (n_words + 3) & ~3;
+  L.bits = o; o += (n_words + 4) & ~3;
   const int rows = chunk_rows(M, cells);
   const int n = rows * M > cells ? rows * M : cells;
   L.w = o; o += n;
@@ -200,7 +210,7 @@ __host__ __device__ inline void layout(int M, int n_in, const int* C, int n_word
 
 struct Block {
   float *pj, *ej, *zj, *bj, *epsc, *pjn, *pi;
-  uint32_t* qi;
+  uint32_t* plane;
   uint16_t *list, *src;
   uint8_t* di;
 };
@@ -215,11 +225,12 @@ __device__ __forceinline__ Block block(float* sm, const Layout& L, int k, int M,
   b.bj = f + 3 * M;
   b.epsc = f + 4 * M;
   b.pjn = f + 6 * M;
-  b.qi = (uint32_t*)(f + 8 * M);
-  b.pi = f + 8 * M + C;
-  b.list = (uint16_t*)(b.pi + 2 * C);
-  b.src = b.list + 2 * kQW * queue_part(C, kQW);
-  b.di = (uint8_t*)((uint32_t*)b.list + (2 * kQW * queue_part(C, kQW) + C + 1) / 2);
+  const int n = kQW * queue_part(C, kQW);
+  b.pi = f + 8 * M;
+  b.plane = (uint32_t*)(b.pi + 2 * C);
+  b.list = (uint16_t*)(b.plane + n);
+  b.src = b.list + 2 * n;
+  b.di = (uint8_t*)(b.src + n);
   return b;
 }
 
@@ -262,7 +273,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     s_rp = *rp_g;
     s_abort = 0;
     s_rows = s_cols = 0;
-    mb_init(s_E, kW / 32);
+    mb_init(s_E, kW / 32 + 1);
     mb_init(s_S, 1);
     mb_init(s_Lst, 1);
     mb_init(s_T, 1);
@@ -304,6 +315,8 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
   /* ---- load the state the previous tick left ---- */
   const int cur0 = rp->k0 & 1, prev0 = cur0 ^ 1;
   const float prn = rp->prn;
+  const uint32_t none = (uint32_t)fa.n_words << 5; /* the source of an empty slot: a word that is always 0 */
+  if (tid == 0) s_bits[fa.n_words] = 0u;
 #pragma unroll 1
   for (int k = 0; k < n_in; ++k) {
     const ProjDev& J = s_proj[k];
@@ -321,12 +334,15 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       B.epsc[prev0 * M + j] = pop.epsc[prev0][eoff + idx];
       B.pjn[cur0 * M + j] = pj + (ej - pj) * kp;
     }
+    /* a queue entry's bit b, due in b ticks, is bit `slot` of plane b; whole warps, a word of slots each */
+    const int part = queue_part(J.C, kQW), slots = kQW * part;
 #pragma unroll 1
-    for (int s = tid; s < J.C; s += kThreads) {
-      const int r = h * J.C + s, ii = J.ii[r];
-      uint32_t src = 0xffffu, di = 0;
+    for (int s = tid; s < slots; s += kThreads) {
+      const int r = h * J.C + s, ii = s < J.C ? J.ii[r] : -1;
+      uint32_t src = none, di = 0, qi = 0;
       if (ii >= J.Ns) atomicOr(net->err, kErrIndex);
       if (ii >= 0 && ii < J.Ns) {
+        qi = (uint32_t)J.qi[r];
         const int hs = ii / s_srcM[k], ms = ii - hs * s_srcM[k];
         src = (uint32_t)(s_src0[k] + hs * ((s_srcM[k] + 31) >> 5) + (ms >> 5)) << 5 | (uint32_t)(ms & 31);
         di = (uint32_t)J.di[r] & 31u;
@@ -335,10 +351,14 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       }
       B.src[s] = (uint16_t)src;
       B.di[s] = (uint8_t)di;
-      B.qi[s] = (uint32_t)J.qi[r];
+#pragma unroll 1
+      for (int b = 0; b < 32; ++b) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (qi >> b) & 1u);
+        if ((tid & 31) == b) B.plane[b * (slots >> 5) + (s >> 5)] = m;
+      }
     }
     /* the listed rows, ascending, by queue warp: the first part's are the first n0 */
-    const int part = queue_part(J.C, kQW), cnt = J.list_cnt[h];
+    const int cnt = J.list_cnt[h];
     const int* rows = J.list + h * J.C;
     int n0 = cnt;
     if (kQW > 1) {
@@ -530,12 +550,58 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       for (int k = 0; k < pop.n_out; ++k) net->projs[pop.out_proj[k]].si[last][idx] = spk ? 1 : 0;
     }
   } else if (tid < kP + kQ) {
-    /* ================= Q: spike words, delay queue ================= */
+    /* ================= Q: delay queue, spike words ================= */
     const int qt = tid - kP, warp = qt >> 5, lane = qt & 31;
     bool bad = false;
 #pragma unroll 1
     for (int it = 0; it < n_ticks; ++it) {
-      const int cur = (rp->k0 + it) & 1, prev = cur ^ 1, nxt = prev;
+      const int prev = (rp->k0 + it + 1) & 1, nxt = prev;
+      /* the lists written below were read by the rows of it - 1 */
+      if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
+      if (kQW > 1) bar(kBarQ, kQ);
+      else __syncwarp();
+      /* the slots due, from plane `it`, a word of 32 per lane; then the planes are one tick further: what was plane 0 is
+         the last one, and takes what was the last (the queue word is shifted with its sign, Proj.cpp:621) */
+#pragma unroll 1
+      for (int k = 0; k < n_in; ++k) {
+        const int C = s_proj[k].C;
+        const Block B = block<kQW>(sm, L, k, M, C);
+        const int part = queue_part(C, kQW), words = kQW * part >> 5;
+        uint32_t* const due = B.plane + (it & 31) * words;
+        const uint32_t* const last = B.plane + ((it + 31) & 31) * words;
+        uint16_t* out = B.list + (nxt * kQW + warp) * part;
+        int total = 0;
+#pragma unroll 1
+        for (int x0 = warp * (part >> 5); x0 < (warp + 1) * (part >> 5); x0 += 32) {
+          const int x = x0 + lane;
+          uint32_t m = 0;
+          if (x < (warp + 1) * (part >> 5)) {
+            m = due[x];
+            due[x] = last[x];
+          }
+          const int c = __popc(m);
+          int at = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += v;
+          }
+          const int sum = __shfl_sync(0xffffffffu, at, 31);
+          at += total - c;
+#pragma unroll 1
+          for (; m; m &= m - 1) out[at++] = (uint16_t)(x * 32 + __ffs(m) - 1);
+          total += sum;
+        }
+        if (lane == 0) s_nl[k][nxt][warp] = total;
+      }
+      if (kQW > 1) {
+        bad = bar_any(kBarQ, kQ, bad);
+      } else {
+        bad = __any_sync(0xffffffffu, bad);
+        __syncwarp();
+      }
+      if (qt == 0) mb_arrive(s_Lst, it);
+      if (bad) break;
       if (it > 0) {
         const uint32_t tag = rp->serial0 + (uint32_t)(it - 1);
         const unsigned long long* w = fa.words + (size_t)(tag & (kWordTicks - 1)) * fa.n_words;
@@ -558,66 +624,40 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
             }
           }
         }
-        /* the lists written below were read by the rows of it - 1 */
-        if (!bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
+        __syncwarp();
+        if (kQW > 1) bar(kBarQ, kQ);
       }
-      if (kQW > 1) bar(kBarQ, kQ);
-      else __syncwarp();
+      /* the slots whose source has spiked: most have not, so eight are looked at together */
 #pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
-        const ProjDev& J = s_proj[k];
-        const int C = J.C;
+        const int C = s_proj[k].C;
         const Block B = block<kQW>(sm, L, k, M, C);
-        const int part = queue_part(C, kQW);
-        uint16_t* out = B.list + (nxt * kQW + warp) * part;
-        const int s1 = min(C, (warp + 1) * part);
-        int total = 0;
+        const int part = queue_part(C, kQW), words = kQW * part >> 5;
+        const bool words_tell = it > 0 && s_fed[k];
 #pragma unroll 1
-        for (int s0 = warp * part; s0 < s1; s0 += 128) {
-          uint32_t src[4], di[4], qv[4];
-          bool on[4];
-#pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            const int s = s0 + y * 32 + lane;
-            src[y] = 0xffffu;
-            if (s < s1) {
-              src[y] = B.src[s];
-              di[y] = B.di[s];
-              qv[y] = B.qi[s];
+        for (int s0 = warp * part; s0 < (warp + 1) * part; s0 += 64) {
+          const int s = s0 + 2 * lane;
+          const uint32_t src = *(const uint32_t*)(B.src + s);
+          uint32_t hit;
+          if (words_tell) {
+            hit = (s_bits[(src & 0xffffu) >> 5] >> (src & 31u)) & 1u;
+            hit |= ((s_bits[src >> 21] >> ((src >> 16) & 31u)) & 1u) << 1;
+          } else {
+            hit = 0;
+#pragma unroll 1
+            for (int y = 0; y < 2; ++y) {
+              const uint32_t di = B.di[s + y];
+              hit |= ((di >> (di & kUnfed ? 6 + prev : 6)) & 1u) << y;
             }
           }
-#pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            const int s = s0 + y * 32 + lane;
-            on[y] = false;
-            if (src[y] != 0xffffu) {
-              bool sp;
-              if (di[y] & kUnfed) sp = (di[y] >> (6 + prev)) & 1u;
-              else if (it == 0) sp = (di[y] >> 6) & 1u;
-              else sp = (s_bits[src[y] >> 5] >> (src[y] & 31u)) & 1u;
-              on[y] = qv[y] & 1u;
-              uint32_t q = (uint32_t)((int)qv[y] >> 1);
-              if (sp) q |= 1u << ((di[y] & 31u) - 1u);
-              B.qi[s] = q;
-            }
-          }
-#pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            const unsigned m = __ballot_sync(0xffffffffu, on[y]);
-            if (on[y]) out[total + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(s0 + y * 32 + lane);
-            total += __popc(m);
+#pragma unroll 1
+          for (; hit; hit &= hit - 1) {
+            const int e = s + __ffs(hit) - 1;
+            /* due in di - 1 ticks, seen from the next one */
+            atomicOr(B.plane + ((it + (B.di[e] & 31)) & 31) * words + (e >> 5), 1u << (e & 31));
           }
         }
-        if (lane == 0) s_nl[k][nxt][warp] = total;
       }
-      if (kQW > 1) {
-        bad = bar_any(kBarQ, kQ, bad);
-      } else {
-        bad = __any_sync(0xffffffffu, bad);
-        __syncwarp();
-      }
-      if (qt == 0) mb_arrive(s_Lst, it);
-      if (bad) break;
     }
     bar(0, kThreads);
   } else if (tid < kP + kQ + 32) {
@@ -661,7 +701,10 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         }
       }
       __syncwarp();
-      if (lane == 0) mb_arrive(s_T, it);
+      if (lane == 0) {
+        mb_arrive(s_T, it);
+        mb_arrive(s_E, it); /* the rows wait for T only where a weight needs it */
+      }
     }
     bar(0, kThreads);
   } else {
@@ -773,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
                 for (int u = 0; u < kColU; ++u) {
                   const int s = s0 + u * kW;
                   pdt[u] = -1;
-                  if (s < C && B.src[s] != 0xffffu) {
+                  if (s < C && B.src[s] != none) {
                     pdt[u] = max(simstep - tij[(size_t)s * M], 0);
                     cv[u] = cell[(size_t)s * M];
                   }
@@ -823,10 +866,15 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       pop.epsc[last][eoff + idx] = B.epsc[last * M + j];
       pop.bj[last][eoff + idx] = B.bj[j];
     }
+    const int part = queue_part(J.C, kQW), n0 = s_nl[k][next][0], words = kQW * part >> 5;
 #pragma unroll 1
-    for (int s = tid; s < J.C; s += kThreads)
-      if (B.src[s] != 0xffffu) J.qi[h * J.C + s] = (int)B.qi[s];
-    const int part = queue_part(J.C, kQW), n0 = s_nl[k][next][0];
+    for (int s = tid; s < J.C; s += kThreads) {
+      if (B.src[s] == none) continue;
+      uint32_t q = 0;
+#pragma unroll 4
+      for (int b = 0; b < 32; ++b) q |= ((B.plane[((n_ticks + b) & 31) * words + (s >> 5)] >> (s & 31)) & 1u) << b;
+      J.qi[h * J.C + s] = (int)q;
+    }
     const int cnt = kQW > 1 ? n0 + s_nl[k][next][kQW - 1] : n0;
     const uint16_t* l = B.list + next * kQW * part;
 #pragma unroll 1
