@@ -138,6 +138,7 @@ struct bcpnn_net {
   int ring_len = 1;         /* its spike buffer size */
   const void* tick_fn = nullptr;  /* the tick kernel variant of the persistent launch */
   const void* tick_fn0 = nullptr; /* the same size and decay form with in-CTA columns */
+  int flow_threads = 0;
   const void* flow_fn = nullptr;  /* the dataflow kernel (bcpnn_flow.cuh), where the network fits it */
   size_t flow_smem = 0;
   flow::Args flow_args{};
@@ -469,12 +470,17 @@ int begin_run(bcpnn_net* net, int n_ticks) {
   return BCPNN_OK;
 }
 
-/* external spike replay is tick_kernel's */
+/* external spike replay is tick_kernel's and, of ProcUpdMulti, the other launches' */
 bool use_flow(const bcpnn_net* net) {
   if (!net->flow_fn) return false;
   for (const PopDev& D : net->hp)
     if (D.ext) return false;
   return true;
+}
+
+void launch_flow(bcpnn_net* net, int n_ticks) {
+  void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&net->flow_args, (void*)&n_ticks};
+  cudaLaunchCooperativeKernel(net->flow_fn, dim3(net->total_hcu), dim3(net->flow_threads), args, net->flow_smem, net->stream);
 }
 
 /* the work of one run, queued on the network's stream */
@@ -495,6 +501,10 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
         const ProjHost& J = net->projs[p];
         multi::all_kernel<<<grid_for((size_t)J.H * J.C * 32, 256), 256, 0, net->stream>>>(net->d_net, net->d_rp, p);
       }
+    if (use_flow(net)) {
+      launch_flow(net, n_ticks);
+      return;
+    }
     if (net->multi_persistent) {
       int it0 = 0, n = n_ticks;
       void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&it0, (void*)&n, (void*)&net->bar};
@@ -515,9 +525,7 @@ void enqueue_run(bcpnn_net* net, int n_ticks, bool with_all) {
     return;
   }
   if (use_flow(net)) {
-    int n = n_ticks;
-    void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&net->flow_args, (void*)&n};
-    cudaLaunchCooperativeKernel(net->flow_fn, dim3(net->total_hcu), dim3(net->threads), args, net->flow_smem, net->stream);
+    launch_flow(net, n_ticks);
   } else if (net->persistent) {
     int it0 = 0, n = n_ticks;
     void* args[] = {(void*)&net->d_net, (void*)&net->d_rp, (void*)&it0, (void*)&n, (void*)&net->bar};
@@ -594,15 +602,17 @@ bool raise_smem(const TickForm& f, bool fp64, int dev, size_t smem) {
    (one MCU per thread), the fewest that hold the network's largest HCU. */
 struct FlowForm {
   int threads, pop_warps, queue_warps;
-  const void* fn;
+  const void* fn[2]; /* ProcUpdLazy, ProcUpdMulti */
 };
-#define FLOW_FORM(T, P, Q) {T, P, Q, (const void*)flow::flow_kernel<T, P, Q>}
+#define FLOW_FORM(T, P, Q) \
+  {T, P, Q, {(const void*)flow::flow_kernel<T, P, Q, false>, (const void*)flow::flow_kernel<T, P, Q, true>}}
 const FlowForm kFlowForms[] = {FLOW_FORM(512, 1, 2), FLOW_FORM(512, 2, 2), FLOW_FORM(512, 4, 2),
                                FLOW_FORM(256, 1, 1), FLOW_FORM(256, 2, 1), FLOW_FORM(256, 4, 1)};
 #undef FLOW_FORM
 
-/* choose the dataflow kernel for a persistent network; leaves flow_fn null
-   where the network does not fit it */
+/* choose the dataflow kernel: for a persistent network of ProcUpdLazy with its
+   CTA size, for one of ProcUpdMulti with the first that holds it; leaves
+   flow_fn null where the network does not fit */
 int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
 #ifndef BCPNN_PHASE_PROBE /* the probe build measures tick_kernel */
   if (net->max_m > flow::kMaxM) return BCPNN_OK;
@@ -614,29 +624,33 @@ int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
     if (n_words > flow::kMaxWords) return BCPNN_OK;
   }
   for (const FlowForm& f : kFlowForms) {
-    if (f.threads != net->threads || f.pop_warps * 32 < net->max_m) continue;
+    if ((!net->multi && f.threads != net->threads) || f.pop_warps * 32 < net->max_m) continue;
     size_t smem = 0;
     for (const PopHost& P : net->pops) {
       int C[kMaxIn] = {0};
       for (size_t q = 0; q < P.in_proj.size(); ++q) C[q] = net->projs[P.in_proj[q]].C;
       for (int c : C)
         if (c > 0xfffe) return BCPNN_OK; /* slot numbers in 16 bits */
-      smem = std::max(smem, flow::smem_bytes(P.M, (int)P.in_proj.size(), C, n_words, f.threads, f.queue_warps));
+      smem = std::max(smem, flow::smem_bytes(P.M, (int)P.in_proj.size(), C, n_words, f.threads, f.queue_warps, net->multi));
     }
     if (smem + 8192 > smem_max) return BCPNN_OK;
     static std::mutex mu;
-    static size_t raised[sizeof(kFlowForms) / sizeof(kFlowForms[0])][kMaxDevices] = {{0}};
+    static size_t raised[2][sizeof(kFlowForms) / sizeof(kFlowForms[0])][kMaxDevices] = {{{0}}};
+    const void* const fn = f.fn[net->multi];
     {
       std::lock_guard<std::mutex> lock(mu);
-      size_t& r = raised[&f - kFlowForms][net->device];
+      size_t& r = raised[net->multi][&f - kFlowForms][net->device];
       if (smem > r) {
-        CU(cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         r = smem;
       }
     }
     int per_sm = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f.fn, f.threads, smem));
-    if ((long long)per_sm * sms < net->total_hcu) return BCPNN_OK;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, f.threads, smem));
+    if ((long long)per_sm * sms < net->total_hcu) {
+      if (net->multi) continue;
+      return BCPNN_OK;
+    }
     int rc;
     int* d_word0 = nullptr;
     unsigned long long *words = nullptr, *seeds = nullptr;
@@ -651,8 +665,10 @@ int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
     net->flow_args.seeds = seeds;
     net->flow_args.word0 = d_word0;
     net->flow_args.n_words = n_words;
+    net->flow_args.si_mask = net->multi_persistent && net->multi_resident ? 3 : 1;
     net->flow_smem = smem;
-    net->flow_fn = f.fn;
+    net->flow_threads = f.threads;
+    net->flow_fn = fn;
     return BCPNN_OK;
   }
 #endif
@@ -1174,6 +1190,16 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
     const char* e = std::getenv("GSBN_PER_TICK");
     const bool forced = e && e[0] == '1';
     net->multi_persistent = !forced && coop && (long long)per_sm * sms >= net->total_hcu;
+    /* the dataflow kernel replays from 32-bit masks, as the resident launch, and takes every source's spikes from
+       the words of the run */
+    bool fed = true;
+    for (const ProjHost& J : net->projs) {
+      const std::vector<int>& o = net->pops[J.d.src_pop].out_proj;
+      fed = fed && std::find(o.begin(), o.end(), (int)(&J - net->projs.data())) != o.end();
+    }
+    if (!forced && coop && fed && !(er && er[0] == '0') && net->ring_len <= 32 &&
+        (rc = setup_flow(net, sms, (size_t)smem_max)))
+      return bail(rc);
   }
   /* deferred columns of the persistent launch: ring halves sized for every
      MCU of every HCU spiking in one tick (units of kColUnit slots) */
@@ -1574,7 +1600,7 @@ int bcpnn_run(bcpnn_net* net, int32_t first_simstep, int32_t n_ticks, float prn,
     int rc = begin_run(net, n_ticks);
     if (rc) return rc;
   }
-  if (net->direct || net->persistent || net->multi_persistent) {
+  if (net->direct || net->persistent || net->multi_persistent || use_flow(net)) {
     enqueue_run(net, n_ticks, with_all);
     CU(cudaGetLastError());
   } else {
@@ -1591,7 +1617,7 @@ int bcpnn_run(bcpnn_net* net, int32_t first_simstep, int32_t n_ticks, float prn,
     CU(cudaGraphLaunch(ge, net->stream));
   }
   if (net->multi)
-    net->launches += (net->multi_persistent ? 1u : (uint64_t)n_ticks * (1 + net->projs.size())) +
+    net->launches += (net->multi_persistent || use_flow(net) ? 1u : (uint64_t)n_ticks * (1 + net->projs.size())) +
                      (with_all ? net->projs.size() : 0u);
   else
     net->launches += (uint64_t)(net->persistent ? 1 : n_ticks) + (with_all ? net->projs.size() : 0u);

@@ -1,8 +1,9 @@
 /*
- * bcpnn_flow.cuh -- the tick of the plain FP32 path as a dataflow inside and
- * between CTAs: one CTA per (population, destination HCU), persistent over a
- * run, without a grid-wide barrier.  HCUs of at most 128 MCUs; the others, and
- * external spike replay, take tick_kernel (bcpnn_tick.cuh).
+ * bcpnn_flow.cuh -- the tick of the plain FP32 path, and of its variant
+ * ProcUpdMulti, as a dataflow inside and between CTAs: one CTA per (population,
+ * destination HCU), persistent over a run, without a grid-wide barrier.  HCUs of
+ * at most 128 MCUs; the others, and external spike replay, take tick_kernel
+ * (bcpnn_tick.cuh) and the kernels of bcpnn_multi.cuh.
  *
  * What a tick t of HCU h needs (ProcUpdLazy.cpp:88-124):
  *   P(t)  population update  Pop.cpp:229-323: epsc(t-1), bj(t-1), and the
@@ -71,6 +72,7 @@ struct Args {
   unsigned long long* seeds; /* [n_pops][kSeedTicks]: tag << 32 | float bits */
   const int* word0;          /* [n_pops] first word of a population */
   int n_words;
+  int si_mask; /* source-spike buffers by tick & si_mask: 1, or 3 (the block of four of ProcUpdMulti's resident launch) */
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -173,6 +175,14 @@ __device__ __forceinline__ bool bar_any(int id, int n, bool flag) {
   return r != 0;
 }
 
+/* a cell's table entry for fewer than no ticks */
+__device__ __noinline__ Entry entry_before(const TabRef& T, int pdt) {
+  Entry e;
+  table_pair(T.k.kp, T.k.ke, T.k.kzi, T.k.kzj, pdt, 0, e.A, e.B, T.k.fp64);
+  recip_part(e.A, e.B, 0, e.R0, e.R1);
+  return e;
+}
+
 /* shared-memory layout of a CTA, in 4-byte words */
 struct Layout {
   int act;                 /* [M rounded up to 4] */
@@ -186,15 +196,16 @@ struct Layout {
 __host__ __device__ inline int queue_part(int C, int qw) { return ((C + qw - 1) / qw + 63) & ~63; }
 
 /* a projection's block: pj ej zj bj [M], epsc [2][M], pjn [2][M]; pi [2][C] (by list entry); then, of the n = qw * part
-   slots: bit planes of the delay queue [32][n / 32], 16-bit list [2][n] and src [n], bytes di [n] */
-__host__ __device__ inline int block_words(int M, int C, int qw) {
+   slots: bit planes of the delay queue [32][n / 32], 16-bit list [2][n] and src [n], bytes di [n].  ProcUpdMulti: then
+   the ti and zi that a tick's rows start from, [2][C] by list entry */
+__host__ __device__ inline int block_words(int M, int C, int qw, bool multi) {
   const int n = qw * queue_part(C, qw);
-  return 8 * M + 2 * C + n + n + n / 2 + n / 4;
+  return 8 * M + (multi ? 6 : 2) * C + n + n + n / 2 + n / 4;
 }
 
 __host__ __device__ inline int chunk_rows(int M, int cells) { return cells / M < 1 ? 1 : cells / M; }
 
-__host__ __device__ inline void layout(int M, int n_in, const int* C, int n_words, int cells, int qw, Layout& L) {
+__host__ __device__ inline void layout(int M, int n_in, const int* C, int n_words, int cells, int qw, bool multi, Layout& L) {
   int o = 0;
   L.act = o; o += (M + 3) & ~3;
   L.bits = o; o += (n_words + 4) & ~3;
@@ -203,7 +214,7 @@ __host__ __device__ inline void layout(int M, int n_in, const int* C, int n_word
   L.w = o; o += n;
   for (int k = 0; k < kMaxIn; ++k) {
     L.q[k] = o;
-    if (k < n_in) o += block_words(M, C[k], qw);
+    if (k < n_in) o += block_words(M, C[k], qw, multi);
   }
   L.total = o;
 }
@@ -213,6 +224,8 @@ struct Block {
   uint32_t* plane;
   uint16_t *list, *src;
   uint8_t* di;
+  int* ti0;
+  float* zi0;
 };
 
 template <int kQW>
@@ -231,6 +244,8 @@ __device__ __forceinline__ Block block(float* sm, const Layout& L, int k, int M,
   b.list = (uint16_t*)(b.plane + n);
   b.src = b.list + 2 * n;
   b.di = (uint8_t*)(b.src + n);
+  b.ti0 = (int*)(b.di + n); /* ProcUpdMulti alone has these */
+  b.zi0 = (float*)(b.ti0 + 2 * C);
   return b;
 }
 
@@ -245,8 +260,20 @@ constexpr int kUnfed = 32;
    4.7 -> 3.8 us per tick, 10 x 10: 2.4 -> 2.2).
 
    kThreads: 512 (one CTA per SM) or 256 (two); kPW warps of population update (M <= 32 kPW), kQW of delay queue, one of
-   row traces, the others rows and columns */
-template <int kThreads, int kPW, int kQW>
+   row traces, the others rows and columns.
+
+   kMulti: ProcUpdMulti (Pop.cpp:222-311, 403-421, Proj.cpp:409-488, 557-706 of
+   that variant).  The softmax is seeded by the HCU's own MCU 0; there are no
+   columns: a row's cells start from the ti and zi that the row had before this
+   tick (R puts them beside the list first, event O), replay the HCU's spikes
+   since, which s_hist holds as a mask per MCU (bit b: b ticks before the tick
+   after), and take a spike of this tick last, with the rows done and epsc given.
+   Only then are the lists free (event F, for Q).  Bound by the longer of P and W:
+   both start from E and S of the tick before.  us per tick with a ring of 25,
+   against the launch with a grid barrier (res_tick_loop) or, for 256 x 50, two
+   launches per tick: 10 x 10 5.8 -> 2.3, 50 x 50 6.3 -> 2.6, 100 x 100 with
+   C = 1000 6.3 -> 3.0, 256 x 50 with C = 1000 31.3 -> 4.4. */
+template <int kThreads, int kPW, int kQW, bool kMulti>
 __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     flow_kernel(const NetDev* __restrict__ net_g, const RunParams* __restrict__ rp_g, Args fa, int n_ticks) {
   constexpr int kP = kPW * 32, kQ = kQW * 32, kW = kThreads - kP - kQ - 32;
@@ -260,6 +287,8 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
   __shared__ int s_inp[kMaxIn], s_srcM[kMaxIn], s_src0[kMaxIn], s_fed[kMaxIn];
   __shared__ Layout s_L;
   __shared__ unsigned long long s_E[kEventTicks], s_S[kEventTicks], s_Lst[kEventTicks], s_T[kEventTicks];
+  __shared__ unsigned long long s_O[kEventTicks], s_F[kEventTicks];
+  __shared__ uint32_t s_hist[2][kMulti ? kP : 1]; /* by tick parity */
   __shared__ int s_abort;
   __shared__ int s_nl[kMaxIn][2][kQW]; /* list lengths by tick parity */
   __shared__ uint32_t s_spk[2][kPW];   /* spikes of this HCU by tick parity */
@@ -277,6 +306,8 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     mb_init(s_S, 1);
     mb_init(s_Lst, 1);
     mb_init(s_T, 1);
+    mb_init(s_O, 1);
+    mb_init(s_F, kW / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -305,7 +336,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     int c[kMaxIn];
 #pragma unroll
     for (int k = 0; k < kMaxIn; ++k) c[k] = k < n_in ? s_proj[k].C : 0;
-    layout(M, n_in, c, fa.n_words, kCells, kQW, s_L);
+    layout(M, n_in, c, fa.n_words, kCells, kQW, kMulti, s_L);
   }
   __syncthreads();
   const Layout& L = s_L;
@@ -346,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         const int hs = ii / s_srcM[k], ms = ii - hs * s_srcM[k];
         src = (uint32_t)(s_src0[k] + hs * ((s_srcM[k] + 31) >> 5) + (ms >> 5)) << 5 | (uint32_t)(ms & 31);
         di = (uint32_t)J.di[r] & 31u;
-        if (s_fed[k]) di |= J.si[prev0][ii] > 0 ? 64u : 0u;
+        if (s_fed[k]) di |= J.si[0][(size_t)((rp->k0 + fa.si_mask) & fa.si_mask) * J.Ns + ii] > 0 ? 64u : 0u;
         else di |= kUnfed | (J.si[0][ii] > 0 ? 64u : 0u) | (J.si[1][ii] > 0 ? 128u : 0u);
       }
       B.src[s] = (uint16_t)src;
@@ -376,6 +407,18 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       B.list[cur0 * kQW * part + (e < n0 ? e : part + e - n0)] = (uint16_t)(rows[e] - h * J.C);
   }
   if (tid < ((M + 3) & ~3) - M) s_act[M + tid] = 0.0f; /* read by the serial sum */
+  if (kMulti)
+#pragma unroll 1
+    for (int j = tid; j < M; j += kThreads) {
+      /* bit b: the ring's entry for tick simstep0 - 1 - b (at most 32 ticks) */
+      uint32_t m = 0;
+#pragma unroll 1
+      for (int b = 0; b < pop.ring_len - 1; ++b) {
+        const int t = rp->simstep0 - 1 - b;
+        if (t >= 0 && pop.ring[(size_t)(t % pop.ring_len) * n + h * M + j] > 0) m |= 1u << b;
+      }
+      s_hist[prev0][j] = m;
+    }
   __syncthreads();
 
   if (tid < kP) {
@@ -385,6 +428,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     const int idx = h * M + (active ? j : 0);
     float dsup = pop.dsup[prev0][idx], act = pop.act[idx];
     int cnt = pop.counter[idx];
+    float ada = kMulti ? pop.ada[idx] : 0.0f;
     bool spk = false;
     const float lg = rp->lginp[pop.mcu_start + idx], wm = rp->wmask[pop.hcu_start + h];
     const int wph = (M + 31) >> 5;
@@ -411,13 +455,18 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         if (active) wsup += B.bj[j] + B.epsc[prev * M + j];
       }
       sup += (pop.wgain * wm) * wsup;
+      if (kMulti) {
+        sup -= wm * ada;
+        sup = (float)((double)sup + 6.9 * (double)wm); /* a double constant in gsbn */
+      }
       const float d = dsup + (sup - dsup) * pop.taumdt;
       /* the softmax seed (Pop.cpp:270) */
       unsigned long long* const slot = fa.seeds + P * kSeedTicks + (tag & (kSeedTicks - 1));
       float seed = 0.0f;
-      if (h == 0) {
+      const bool own_seed = kMulti || h == 0;
+      if (own_seed) {
         if (tid == 0) {
-          st_word(slot, tag, __float_as_uint(d));
+          if (!kMulti) st_word(slot, tag, __float_as_uint(d));
           s_seed = d;
         }
       } else if (lane == 0) {
@@ -467,13 +516,13 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       if (kPW > 1) {
         if (lane == 0) s_red[warp] = mx;
         bar(kBarP, kP);
-        if (h == 0) seed = s_seed;
+        if (own_seed) seed = s_seed;
         float m = seed;
 #pragma unroll
         for (int w = 0; w < kPW; ++w) m = (s_red[w] > m) ? s_red[w] : m;
         mx = m;
       } else {
-        if (h == 0) seed = __shfl_sync(0xffffffffu, d, 0);
+        if (own_seed) seed = __shfl_sync(0xffffffffu, d, 0);
         mx = (mx > seed) ? mx : seed;
       }
       const float maxact = bx_expf(pop.wtagain * mx);
@@ -508,6 +557,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         st_word(fa.words + (size_t)(tag & (kWordTicks - 1)) * fa.n_words + fa.word0[P] + h * wph + warp, tag, word);
         s_spk[cur][warp] = word;
       }
+      if (kMulti) s_hist[cur][j] = (s_hist[prev][j] << 1) | (spk ? 1u : 0u);
       if (kPW > 1) {
         bad = bar_any(kBarP, kP, bad);
       } else {
@@ -519,6 +569,11 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       dsup = d;
       act = a;
       cnt += spk ? 1 : 0;
+      if (kMulti) {
+        ada += (pop.adgain * a - ada) * pop.tauadt;
+        /* the ring holds the last ticks: what this run would overwrite itself is not written */
+        if (active && n_ticks - it <= pop.ring_len) pop.ring[(size_t)(simstep % pop.ring_len) * n + idx] = spk ? 1 : 0;
+      }
       if (spk) {
         atomicOr(&pop.spk_log[(size_t)it * pop.log_words + (idx >> 5)], 1u << (idx & 31));
         if (idx == 9)
@@ -546,8 +601,10 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       pop.act[idx] = act;
       pop.counter[idx] = cnt;
       pop.spike[idx] = spk ? 1 : 0;
+      if (kMulti) pop.ada[idx] = ada;
+      const size_t si_last = (size_t)((rp->k0 + n_ticks - 1) & fa.si_mask) * n;
 #pragma unroll 1
-      for (int k = 0; k < pop.n_out; ++k) net->projs[pop.out_proj[k]].si[last][idx] = spk ? 1 : 0;
+      for (int k = 0; k < pop.n_out; ++k) net->projs[pop.out_proj[k]].si[0][si_last + idx] = spk ? 1 : 0;
     }
   } else if (tid < kP + kQ) {
     /* ================= Q: delay queue, spike words ================= */
@@ -558,6 +615,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       const int prev = (rp->k0 + it + 1) & 1, nxt = prev;
       /* the lists written below were read by the rows of it - 1 */
       if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
+      if (kMulti && it > 0 && !bad) bad = !mb_wait(s_F, it - 1, &s_abort, net->err);
       if (kQW > 1) bar(kBarQ, kQ);
       else __syncwarp();
       /* the slots due, from plane `it`, a word of 32 per lane; then the planes are one tick further: what was plane 0 is
@@ -669,6 +727,24 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1;
       if (it > 0) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err);
       if (__any_sync(0xffffffffu, bad)) break;
+      if (kMulti) {
+#pragma unroll 1
+        for (int k = 0; k < n_in; ++k) {
+          const ProjDev& J = s_proj[k];
+          const Block B = block<kQW>(sm, L, k, M, J.C);
+          const int part = queue_part(J.C, kQW);
+          const uint16_t* l0 = B.list + cur * kQW * part;
+          const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
+#pragma unroll 1
+          for (int e = lane; e < nrow; e += 32) {
+            const int r = h * J.C + (int)(e < n0 ? l0[e] : l0[part + e - n0]);
+            B.ti0[cur * J.C + e] = J.ti[r];
+            B.zi0[cur * J.C + e] = J.zi[r];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mb_arrive(s_O, it);
+      }
 #pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
@@ -685,7 +761,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           const float4 tr = make_float4(J.pi[r], J.ei[r], J.zi[r], 0.0f);
           float pi = tr.x;
           if (pdt <= 0) {
-            J.zi[r] = tr.z + J.kfti;
+            if (!kMulti) J.zi[r] = tr.z + J.kfti;
           } else {
             float4 A, Bt;
             double2 R0, R1;
@@ -722,7 +798,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
         bad = bar_any(kBarW, kW, bad);
         if (bad) break;
       }
-      bool traces = false;
+      bool traces = false, start = false;
 #pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
         const ProjDev& J = s_proj[k];
@@ -743,6 +819,57 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           for (int c = wt; c < nr * M; c += kW) {
             const int rr = c / M, j = c - rr * M, e = base + rr;
             const size_t index = (size_t)(h * C + (int)(e < n0 ? l0[e] : l0[part + e - n0])) * M + j;
+            if constexpr (kMulti) {
+              float4 q = J.cell[index];
+              if (!start) {
+                if (!mb_wait(s_O, it, &s_abort, net->err)) bad = true;
+                start = true;
+              }
+              int tij = B.ti0[cur * C + e];
+              float zi2 = B.zi0[cur * C + e];
+              /* the spikes after max(tij, simstep - ring) and before this tick, ascending; bit b: tick simstep - b */
+              const int span = min(simstep - tij, pop.ring_len - 1);
+              uint32_t m = span > 1 ? (s_hist[prev][j] << 1) & (0xffffffffu >> (32 - span)) : 0u;
+#pragma unroll 1
+              for (;;) {
+                const int b = m ? 31 - __clz(m) : 0, pdt = simstep - b - tij;
+                float4 A, Bt;
+                double2 R0, R1;
+                if (pdt >= 0) {
+                  entry(T, pdt, 0, A, Bt, R0, R1);
+                } else { /* a row written with a later tick: gsbn's expressions all the same */
+                  const Entry x = entry_before(T, pdt);
+                  A = x.A;
+                  Bt = x.B;
+                  R0 = x.R0;
+                  R1 = x.R1;
+                }
+                const float4 d = cell_step(make_float4(q.x, q.y, zi2, q.w), T, A, Bt, R0, R1);
+                q.x = d.x;
+                q.y = d.y;
+                q.w = d.w;
+                if (m == 0) break; /* the cell keeps the zi2 of its last replay */
+                zi2 = d.z;
+                q.w += J.kftj;
+                tij = simstep - b;
+                m &= ~(1u << b);
+              }
+              q.z = zi2;
+              float w;
+              if (kp != 0.0f) {
+                if (!traces) {
+                  if (!mb_wait(s_T, it, &s_abort, net->err)) bad = true;
+                  traces = true;
+                }
+                w = J.wgain * bx_logf((q.x + J.eps2) / ((B.pi[cur * C + e] + J.eps) * (B.pjn[cur * M + j] + J.eps)));
+                J.wij[index] = w;
+              } else {
+                w = J.wij[index];
+              }
+              J.cell[index] = q;
+              s_w[c] = w;
+              continue;
+            }
             const int pdt = simstep - J.tij[index];
             float4 q = J.cell[index];
             float w = kp == 0.0f ? J.wij[index] : 0.0f; /* without plasticity the weights stay */
@@ -804,6 +931,16 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
 #pragma unroll 1
             for (uint32_t m = s_spk[cur][w]; m && w * 32 < M; m &= m - 1) {
               const int j = w * 32 + __ffs(m) - 1;
+              if constexpr (kMulti) {
+                /* the cells of this tick's rows: written by other threads of the group, before its last barrier */
+                const int part = queue_part(C, kQW);
+                const uint16_t* l0 = B.list + cur * kQW * part;
+                const int n0 = s_nl[k][cur][0], nrow = kQW > 1 ? n0 + s_nl[k][cur][kQW - 1] : n0;
+#pragma unroll 1
+                for (int e = wt; e < nrow; e += kW)
+                  J.cell[(size_t)(h * C + (int)(e < n0 ? l0[e] : l0[part + e - n0])) * M + j].w += J.kftj;
+                continue;
+              }
               float4* const cell = J.cell + (size_t)h * C * M + j;
               int* const tij = J.tij + (size_t)h * C * M + j;
               /* kColU cells of a thread at a time, their loads together */
@@ -836,8 +973,12 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
                 }
               }
             }
-          if (wt == 0) s_cols += (unsigned long long)nspk * C;
+          if (!kMulti && wt == 0) s_cols += (unsigned long long)nspk * C;
         }
+      }
+      if (kMulti) {
+        __syncwarp();
+        if (lane == 0) mb_arrive(s_F, it);
       }
     }
     bar(0, kThreads);
@@ -884,9 +1025,9 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
 }
 
 /* dynamic shared memory, in bytes, for the network's populations; kQW queue warps, `cells` per chunk */
-inline size_t smem_bytes(int M, int n_in, const int* C, int n_words, int cells, int qw) {
+inline size_t smem_bytes(int M, int n_in, const int* C, int n_words, int cells, int qw, bool multi) {
   Layout L;
-  layout(M, n_in, C, n_words, cells, qw, L);
+  layout(M, n_in, C, n_words, cells, qw, multi, L);
   return (size_t)L.total * 4;
 }
 

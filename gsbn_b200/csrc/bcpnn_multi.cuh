@@ -16,8 +16,11 @@
  * The closed forms are gsbn's (same expressions as ProcUpdLazy), evaluated
  * with the shared decay tables and the exact division of bcpnn_device.cuh.
  *
- * Launch forms: one persistent cooperative launch per run, with each HCU's
- * state resident in shared memory (res_tick_loop) or in global memory
+ * Launch forms: the dataflow kernel (bcpnn_flow.cuh, kMulti), for HCUs of at
+ * most 128 MCUs whose sources are all published, rings of at most 32 ticks and
+ * no external spikes (3.0 us per tick at 100 x 100 with C = 1000; with the grid
+ * barrier of the next form 6.3); else one persistent cooperative launch per run,
+ * with each HCU's state resident in shared memory (res_tick_loop) or in global memory
  * (tick_loop, for spike rings longer than 32 ticks or states too large for
  * shared memory); or, when the grid cannot be co-resident, one launch of
  * pop_kernel per tick over every (population, HCU) and one of proj_kernel
