@@ -1,7 +1,8 @@
 /*
  * bcpnn_recall.cu -- replicate recall engine (include/bcpnn_recall.h).
  *
- * Two launches per tick on two streams, side by side: the population update
+ * Two launches per tick on two streams, side by side (or, of a small BF16
+ * network, one launch of CTAs of both kinds): the population update
  * of tick t (recall_pop_kernel: support from epsc(t-1), softmax/WTA, Philox
  * spikes, writing dsup(t), the BF16 spike row S(t) and the recall counters)
  * and the contraction with its epilogue epsc(t) = epsc(t-1) * (1 - kepsc) +
@@ -272,13 +273,12 @@ __device__ __forceinline__ f32x2 exp2_near(f32x2 x, f32x2 one, f32x2 neg) {
    every MCU divided (the exact product is below that bound by more than its
    roundings, and a uniform of 0 always takes the exact path).  The recall counters are
    touched only where a group has a spike.  kBits: the spikes as bits, for the
-   FP32 contraction.  64 x 64, 4096 replicates: 100 us alone as one exp and one
-   division per MCU, with 16 contiguous MCUs per lane. */
+   FP32 contraction.  64 x 64, 4096 replicates: 80 us alone; 100 as one exp and
+   one division per MCU, with 16 contiguous MCUs per lane. */
 template <int M, bool kBits>
-__global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
+__device__ __forceinline__ void recall_pop(const Params& p, int tid) {
   constexpr int G = M / 16; /* groups of four MCUs per lane */
   const int lane = threadIdx.x & 31;
-  const int tid = blockIdx.x * 256 + threadIdx.x;
   const int g = tid >> 2, q = tid & 3;
   const int h = g % p.H, r = g / p.H;
   const uint32_t seed = p.seed_base + (uint32_t)r;
@@ -440,6 +440,11 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+template <int M, bool kBits>
+__global__ void __launch_bounds__(256) recall_pop_kernel(Params p) {
+  recall_pop<M, kBits>(p, blockIdx.x * 256 + threadIdx.x);
+}
+
 /* The output tiles of a launch: 128 x 256, or, where these are fewer than the
    SMs, column parts of 128, 64 or 32, as narrow as still gives every SM at most
    one.  A single tile (256 sources, 128 replicates) takes 8 CTAs of 32 columns
@@ -481,14 +486,33 @@ struct WMaps {
 };
 
 /* Persistent contraction + epsc epilogue: one CTA per SM walks the tiles t =
-   blockIdx.x, blockIdx.x + gridDim.x, ... (Tiles).  The stage ring runs on
+   blockIdx.x, blockIdx.x + ctas, ... (Tiles).  The stage ring runs on
    across tiles; two TMEM accumulators of 256 columns alternate, so the epilogue
    of one tile overlaps the MMAs of the next (acc_full: MMA -> epilogue,
    acc_empty: epilogue -> MMA).  The epilogue's loads run one 32-column chunk
-   ahead, the first before its accumulator is there. */
+   ahead, the first before its accumulator is there.
+
+   kPopM: the HCU size, and the CTAs from `ctas` on do the population update of
+   the tick, which needs nothing of the contraction's; 0: recall_pop_kernel does
+   it, on a stream of its own.  Where all of both find an SM each, one launch per
+   tick costs less than two with the events between their streams, which the host
+   takes longer to queue than the GPU to run, and a tick's launch, its barriers and
+   its TMEM come beside the end of the tick before (programmatic launch; nothing
+   that tick writes is touched before griddepcontrol.wait): 256 sources, 128
+   replicates 9.5 -> 6.2 -> 4.2 us per tick. */
+template <int kPopM>
 __global__ void __launch_bounds__(kThreads, 1)
     recall_tick_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_constant__ WMaps map_w, Params p,
-                       int grid_max) {
+                       int grid_max, int ctas) {
+  if constexpr (kPopM > 0) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if ((int)blockIdx.x >= ctas) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      const int tid = ((int)blockIdx.x - ctas) * kThreads + threadIdx.x;
+      if (tid < p.R * p.H * 4) recall_pop<kPopM, false>(p, tid); /* whole warps: R is a multiple of 128 */
+      return;
+    }
+  }
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + kStages * kStageBytes);
@@ -525,6 +549,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  /* the set-up above ran beside the end of the tick before; all it wrote is there from here on */
+  if constexpr (kPopM > 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tmem = *s_tmem;
   /* self-check of the set-up every access below relies on: ring and barrier
      alignment, the accumulators' TMEM columns, whole tiles */
@@ -539,7 +565,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       long long it = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+      for (int t = blockIdx.x; t < n_tiles && ok; t += ctas) {
         int m0, n0, cols;
         tiles.at(t, m0, n0, cols);
         const CUtensorMap* w = &map_w.of[t < tiles.whole ? 0 : part_log];
@@ -568,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       long long it = 0;
       bool ok = true;
       int li = 0;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, li++) {
+      for (int t = blockIdx.x; t < n_tiles && ok; t += ctas, li++) {
         const int j = li & 1;
         if (!mbar_wait(&acc_empty[j], (uint32_t)(((li >> 1) & 1) ^ 1), p.err)) break;
         tc_fence_after();
@@ -599,7 +625,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     /* ---------------- epilogue: one replicate row per thread ---------------- */
     const int q = warp & 3; /* TMEM lane quarter this warp may access */
     int li = 0;
-    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, li++) {
+    for (int t = blockIdx.x; t < n_tiles; t += ctas, li++) {
       const int j = li & 1;
       int m0, n0, cols;
       tiles.at(t, m0, n0, cols);
@@ -647,6 +673,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
+
+using TickFn = void (*)(CUtensorMap, WMaps, Params, int, int);
 
 constexpr int kF32BM = 128, kF32BN = 128, kF32BK = 16, kF32Threads = 256;
 
@@ -1285,9 +1313,9 @@ int bcpnn_recall_create(const bcpnn_recall_desc* d, bcpnn_recall** out) {
     for (int i = 0; i < 4 && !rc; i++) rc = encode_map(r, &r->map_s[i], r->s[i], R, (int)N, kTileM);
     for (int i = 0; i <= kMaxPartsLog && !rc; i++) rc = encode_map(r, &r->map_w.of[i], r->wt, (int)N, (int)N, kTileN >> i);
     if (rc) return bad(rc);
-    if (cudaFuncSetAttribute(recall_tick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) !=
-        cudaSuccess)
-      return bad(BCPNN_ERR_CUDA);
+    for (TickFn f : {recall_tick_kernel<0>, recall_tick_kernel<16>, recall_tick_kernel<32>, recall_tick_kernel<64>})
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess)
+        return bad(BCPNN_ERR_CUDA);
   } else {
     if ((rc = encode_map(r, &r->map_wf, r->wf, (int)N, (int)N, kEvBox, true))) return bad(rc);
     for (int i = 0; i < 2; i++)
@@ -1461,6 +1489,11 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   const int ev_grid = (int)(ev_pairs / kEvWarps < r->sms ? ev_pairs / kEvWarps : r->sms);
   const int list_blocks =
       (int)(((long long)d.replicates * ((r->N + kEvRows - 1) / kEvRows) + 255) / 256);
+  /* BF16 in one launch per tick: tile CTAs and population CTAs with an SM each
+     (not while the contraction is timed by itself) */
+  const int pop_ctas = (int)(((long long)d.replicates * d.hcu_num * 4 + kThreads - 1) / kThreads);
+  const bool together = !r->wf && !r->timing && grid + pop_ctas <= r->sms;
+  const TickFn both = d.mcu_num == 16 ? recall_tick_kernel<16> : d.mcu_num == 32 ? recall_tick_kernel<32> : recall_tick_kernel<64>;
   /* Tick kk: the population update needs epsc(kk-1) and dsup(kk-1); the
      contraction needs S(kk-3) and epsc(kk-1).  So both wait only for tick
      kk-1 and run side by side: pop(kk) after gemm(kk-1) (it also must not
@@ -1477,8 +1510,10 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
     recall_lists_kernel<<<list_blocks, 256, 0, r->stream>>>(r->sb[mod4(r->kk - 3)], r->lists[r->kk & 1],
                                                              r->list_cnt[r->kk & 1], d.replicates, r->N);
   RCU(cudaGetLastError());
-  RCU(cudaEventRecord(r->ev_gemm, r->stream));
-  RCU(cudaStreamWaitEvent(r->pop_stream, r->ev_gemm, 0));
+  if (!together) {
+    RCU(cudaEventRecord(r->ev_gemm, r->stream));
+    RCU(cudaStreamWaitEvent(r->pop_stream, r->ev_gemm, 0));
+  }
   for (int i = 0; i < n_ticks; i++) {
     const long long kk = r->kk + i;
     const int cur = (int)(kk & 1), prev = cur ^ 1;
@@ -1490,6 +1525,20 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
     p.s_bits = r->sb[mod4(kk)];
     p.simstep = first + i;
     p.count_on = (first + i >= count_first && first + i <= count_last) ? 1 : 0;
+    if (together) {
+      cudaLaunchAttribute early = {};
+      early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      early.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(grid + pop_ctas);
+      cfg.blockDim = dim3(kThreads);
+      cfg.dynamicSmemBytes = kSmemBytes;
+      cfg.stream = r->stream;
+      cfg.attrs = &early;
+      cfg.numAttrs = 1;
+      RCU(cudaLaunchKernelEx(&cfg, both, r->map_s[mod4(kk - 3)], r->map_w, p, r->sms, grid));
+      continue;
+    }
     pop<<<pop_blocks, 256, 0, r->pop_stream>>>(p);
     if (events && i + 1 < n_ticks)
       recall_lists_kernel<<<list_blocks, 256, 0, r->pop_stream>>>(r->sb[mod4(kk - 2)], r->lists[cur ^ 1],
@@ -1502,7 +1551,7 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
     else if (r->wf)
       recall_fp32_kernel<<<f32_tiles, kF32Threads, 0, r->stream>>>(r->sb[mod4(kk - 3)], r->wf, p);
     else
-      recall_tick_kernel<<<grid, kThreads, kSmemBytes, r->stream>>>(r->map_s[mod4(kk - 3)], r->map_w, p, r->sms);
+      recall_tick_kernel<0><<<grid, kThreads, kSmemBytes, r->stream>>>(r->map_s[mod4(kk - 3)], r->map_w, p, r->sms, grid);
     RCU(cudaGetLastError());
     if (r->timing) RCU(cudaEventRecord(r->tev[2 * i + 1], r->stream));
     /* both kernels of tick kk are queued: each stream waits for the other's
@@ -1514,7 +1563,7 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   }
   r->kk += n_ticks;
   r->counted += counted;
-  r->launches += (events ? 3 : 2) * (uint64_t)n_ticks;
+  r->launches += (together ? 1 : events ? 3 : 2) * (uint64_t)n_ticks;
   int rc = check_err(r); /* synchronises the stream: every timing event has completed */
   if (rc == BCPNN_OK && r->timing) {
     for (int i = 0; i < n_ticks; i++) {
