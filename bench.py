@@ -59,8 +59,8 @@ def peaks():
 
 
 def profile_traffic():
-    """Per-launch DRAM traffic of tick_kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "tick_kernel_100x100.md")
+    """Per-launch DRAM traffic of flow_kernel from the committed ncu summary."""
+    path = os.path.join(ROOT, "profiles", "flow_kernel_100x100.md")
     try:
         with open(path) as f:
             for line in f:
@@ -315,12 +315,12 @@ def run_ours(args, rank, world, local_rank, cpu=False):
             "parity": parity,
             "recall": f"{recall[0]}/{recall[1]}",
             "gpu_launches": launches,
-            "roofline": {"bound": "hbm", "kernel": "tick_kernel", "achieved": achieved, "peak": pk["hbm_gbs"],
+            "roofline": {"bound": "hbm", "kernel": "flow_kernel", "achieved": achieved, "peak": pk["hbm_gbs"],
                          "unit": "GB/s", "frac": achieved / pk["hbm_gbs"], "peak_kind": pk_kind,
                          "traffic": traffic, "algorithmic_bytes_per_launch": bytes_per_launch,
                          "us_per_launch": launch_us, "ticks_per_launch": ticks_per_launch,
                          "us_per_tick": tick_us,
-                         "traffic_source": "profiles/tick_kernel_100x100.md (ncu dram bytes per launch)"},
+                         "traffic_source": "profiles/flow_kernel_100x100.md (ncu dram bytes per launch)"},
             "e2e": {"value": e_cells / e_s, "unit": "cell updates/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "ms_per_step": e_s * 1e3 / args.steps},
             "clocks": clk.summary(),
