@@ -35,9 +35,9 @@
  *
  * Bound by the longest cycle of dependences: P(t) -> columns(t) -> rows(t+1) ->
  * P(t+2) takes two ticks, E(t-1) -> P(t) one.  Per tick, against tick_kernel with
- * its grid barrier and its columns spread over the grid: 10 x 10 2.2 us (7.4),
- * 50 x 50 2.6 (8.8), 100 x 100 with C = 1000 4.0 (9.9), 256 x 50 with C = 1000
- * 6.3 (13.8), 296 x 20 with C = 400 3.6 (11.3).  With the row traces in W and two
+ * its grid barrier and its columns spread over the grid: 10 x 10 2.0 us (7.4),
+ * 50 x 50 2.4 (8.8), 100 x 100 with C = 1000 3.75 (9.9), 256 x 50 with C = 1000
+ * 6.0 (13.8), 296 x 20 with C = 400 3.3 (11.3).  With the row traces in W and two
  * more barriers before the sum, decays as calls, and a queue word of every slot
  * shifted every tick: 2.8, 3.7, 6.0, 9.7 and 5.7.  The decays and their exact
  * division are those of bcpnn_device.cuh, so every value is bit-identical to
@@ -943,34 +943,34 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
               }
               float4* const cell = J.cell + (size_t)h * C * M + j;
               int* const tij = J.tij + (size_t)h * C * M + j;
-              /* kColU cells of a thread at a time, their loads together */
+              /* a cell at a time, with the loads of the thread's next one in flight.  Two at a time was more code to
+                 fetch every tick and spilled: 100 x 100 4.0 -> 3.75 us per tick, 10 x 10 2.13 -> 2.02, 296 x 20 3.65 ->
+                 3.3; with the next one's table entry in flight too 4.1, 2.09 and 3.5 */
+              int pn;
+              float4 next;
+              auto load = [&](int s) {
+                pn = -1;
+                if (s < C && B.src[s] != none) {
+                  pn = max(simstep - tij[(size_t)s * M], 0);
+                  next = cell[(size_t)s * M];
+                }
+              };
+              load(wt);
 #pragma unroll 1
-              for (int s0 = wt; s0 < C; s0 += kColU * kW) {
-                int pdt[kColU];
-                float4 cv[kColU], A[kColU], Bt[kColU];
-                double2 R0[kColU], R1[kColU];
-#pragma unroll
-                for (int u = 0; u < kColU; ++u) {
-                  const int s = s0 + u * kW;
-                  pdt[u] = -1;
-                  if (s < C && B.src[s] != none) {
-                    pdt[u] = max(simstep - tij[(size_t)s * M], 0);
-                    cv[u] = cell[(size_t)s * M];
-                  }
+              for (int s = wt; s < C; s += kW) {
+                const int pdt = pn;
+                float4 q = next;
+                load(s + kW);
+                if (pdt < 0) continue;
+                if (pdt > 0) {
+                  float4 A, Bt;
+                  double2 R0, R1;
+                  entry(T, pdt, 0, A, Bt, R0, R1);
+                  q = cell_step(q, T, A, Bt, R0, R1);
                 }
-#pragma unroll
-                for (int u = 0; u < kColU; ++u)
-                  if (pdt[u] > 0) entry(T, pdt[u], 0, A[u], Bt[u], R0[u], R1[u]);
-#pragma unroll
-                for (int u = 0; u < kColU; ++u) {
-                  if (pdt[u] < 0) continue;
-                  float4 q = cv[u];
-                  if (pdt[u] > 0) q = cell_step(q, T, A[u], Bt[u], R0[u], R1[u]);
-                  q.w += J.kftj;
-                  const size_t at = (size_t)(s0 + u * kW) * M;
-                  cell[at] = q;
-                  tij[at] = simstep;
-                }
+                q.w += J.kftj;
+                cell[(size_t)s * M] = q;
+                tij[(size_t)s * M] = simstep;
               }
             }
           if (!kMulti && wt == 0) s_cols += (unsigned long long)nspk * C;
