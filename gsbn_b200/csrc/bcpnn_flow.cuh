@@ -35,7 +35,7 @@
  *
  * Bound by the longest cycle of dependences: P(t) -> columns(t) -> rows(t+1) ->
  * P(t+2) takes two ticks, E(t-1) -> P(t) one.  Per tick, against tick_kernel with
- * its grid barrier and its columns spread over the grid: 10 x 10 2.0 us (7.4),
+ * its grid barrier and its columns spread over the grid: 10 x 10 1.8 us (7.4),
  * 50 x 50 2.4 (8.8), 100 x 100 with C = 1000 3.75 (9.9), 256 x 50 with C = 1000
  * 6.0 (13.8), 296 x 20 with C = 400 3.3 (11.3).  With the row traces in W and two
  * more barriers before the sum, decays as calls, and a queue word of every slot
@@ -438,6 +438,11 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     for (int it = 0; it < n_ticks; ++it) {
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1, prev = cur ^ 1;
       const uint32_t tag = rp->serial0 + (uint32_t)it;
+      unsigned long long* const slot = fa.seeds + P * kSeedTicks + (tag & (kSeedTicks - 1));
+      const bool own_seed = kMulti || h == 0;
+      /* HCU 0, which waits for no seed, is mostly ahead: its seed is there already (10 x 10 2.07 -> 1.84 us per tick) */
+      unsigned long long early = 0;
+      if (!own_seed && lane == 0) early = ld_word(slot);
       /* what depends on tick and MCU only, before the wait */
       const float u = bx_uniform01(pop.rng_seed, pop.rng_pop, (uint32_t)simstep, (uint32_t)idx);
       bool extra = false;
@@ -461,9 +466,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       }
       const float d = dsup + (sup - dsup) * pop.taumdt;
       /* the softmax seed (Pop.cpp:270) */
-      unsigned long long* const slot = fa.seeds + P * kSeedTicks + (tag & (kSeedTicks - 1));
       float seed = 0.0f;
-      const bool own_seed = kMulti || h == 0;
       if (own_seed) {
         if (tid == 0) {
           if (!kMulti) st_word(slot, tag, __float_as_uint(d));
@@ -485,8 +488,8 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           const float d0 = __ldcg(pop.dsup[prev]);
           seed = d0 + (sp - d0) * pop.taumdt;
         } else if (!bad) {
-          uint32_t v = 0;
-          bad = !poll_word(slot, tag, v, &s_abort, net->err);
+          uint32_t v = (uint32_t)early;
+          if ((uint32_t)(early >> 32) != tag) bad = !poll_word(slot, tag, v, &s_abort, net->err);
           seed = __uint_as_float(v);
         }
       }
