@@ -599,7 +599,10 @@ bool raise_smem(const TickForm& f, bool fp64, int dev, size_t smem) {
 }
 
 /* The dataflow kernel's instances: CTA size and warps of population update
-   (one MCU per thread), the fewest that hold the network's largest HCU. */
+   (one MCU per thread), the fewest that hold the network's largest HCU.  Two
+   warps of delay queue where a CTA has an SM to itself (100 x 100 with 1000
+   slots 3.99 us per tick; with one 4.26, though 10 x 10 2.11 -> 2.08), one where
+   two CTAs share it. */
 struct FlowForm {
   int threads, pop_warps, queue_warps;
   const void* fn[2]; /* ProcUpdLazy, ProcUpdMulti */
