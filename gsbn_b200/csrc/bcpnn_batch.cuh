@@ -924,6 +924,13 @@ int bzero(bcpnn_batch* b, void* p, size_t bytes) {
   return BCPNN_OK;
 }
 
+/* a copy to the device, on the batch's stream and complete on return (not
+   cudaMemcpy: its stream is not ordered with the batch's) */
+cudaError_t upload(bcpnn_batch* b, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, b->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(b->stream) : e;
+}
+
 bool finite_pos(float x) { return x > 0.0f && x <= 3.4028234663852886e38f; }
 
 /* the fills of gsbn's initial values (Pop.cpp:59-65, Proj.cpp:88-105) of every
@@ -971,8 +978,8 @@ int make_fills(bcpnn_batch* b) {
   }
   int rc;
   if ((rc = balloc(b, &b->d_fills, segs.size())) || (rc = balloc(b, &b->d_fill_at, at.size()))) return rc;
-  BCU(cudaMemcpy(b->d_fills, segs.data(), segs.size() * sizeof(FillSeg), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy(b->d_fill_at, at.data(), at.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  BCU(upload(b, b->d_fills, segs.data(), segs.size() * sizeof(FillSeg)));
+  BCU(upload(b, b->d_fill_at, at.data(), at.size() * sizeof(uint2)));
   b->fill_blocks = (unsigned int)at.size();
   return BCPNN_OK;
 }
@@ -1074,12 +1081,12 @@ int schedule_items(bcpnn_batch* b) {
   b->d_warp_items = nullptr;
   BCU(cudaMalloc((void**)&b->d_warp_off, off.size() * sizeof(int)));
   BCU(cudaMalloc((void**)&b->d_warp_items, std::max<size_t>(1, flat.size()) * sizeof(int)));
-  BCU(cudaMemcpy(b->d_warp_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
-  if (!flat.empty()) BCU(cudaMemcpy(b->d_warp_items, flat.data(), flat.size() * sizeof(int), cudaMemcpyHostToDevice));
+  BCU(upload(b, b->d_warp_off, off.data(), off.size() * sizeof(int)));
+  if (!flat.empty()) BCU(upload(b, b->d_warp_items, flat.data(), flat.size() * sizeof(int)));
   b->h.warp_off = b->d_warp_off;
   b->h.warp_items = b->d_warp_items;
   b->h.n_warps = b->n_warps;
-  BCU(cudaMemcpy(b->d_dev, &b->h, sizeof(Dev), cudaMemcpyHostToDevice));
+  BCU(upload(b, b->d_dev, &b->h, sizeof(Dev)));
   return BCPNN_OK;
 }
 
@@ -1216,10 +1223,10 @@ int bcpnn_batch_create(const bcpnn_batch_desc* desc, bcpnn_batch** out) {
   }
   if ((rc = make_fills(b)) || (rc = reset_members(b))) return rc;
   if ((rc = balloc(b, &b->d_sweep, sweep.size()))) return rc;
-  BCU(cudaMemcpy(b->d_sweep, sweep.data(), sweep.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  BCU(upload(b, b->d_sweep, sweep.data(), sweep.size() * sizeof(uint2)));
   b->sweep_blocks = (unsigned int)sweep.size();
   if ((rc = balloc(b, &b->d_items, b->items.size()))) return rc;
-  BCU(cudaMemcpy(b->d_items, b->items.data(), b->items.size() * sizeof(int2), cudaMemcpyHostToDevice));
+  BCU(upload(b, b->d_items, b->items.data(), b->items.size() * sizeof(int2)));
   if ((rc = balloc(b, &b->d_m, (size_t)N)) || (rc = balloc(b, &b->d_dev, 1)) || (rc = balloc(b, &b->d_run, 1)) ||
       (rc = balloc(b, &b->d_tabs, 2 * (size_t)N)))
     return rc;
@@ -1279,11 +1286,11 @@ int bcpnn_batch_set_conn(bcpnn_batch* b, int32_t member, const int32_t* ii, cons
   int8_t* fo_di = nullptr;
   int rc;
   if ((rc = balloc(b, &fo_row, row.size())) || (rc = balloc(b, &fo_di, dl.size()))) return rc;
-  BCU(cudaMemcpy(fo_row, row.data(), row.size() * sizeof(int), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy(fo_di, dl.data(), dl.size(), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy((void*)B.fo_off, cnt.data(), cnt.size() * sizeof(int), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy(B.ii, ii, R * sizeof(int), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy(B.di, di, R * sizeof(int), cudaMemcpyHostToDevice));
+  BCU(upload(b, fo_row, row.data(), row.size() * sizeof(int)));
+  BCU(upload(b, fo_di, dl.data(), dl.size()));
+  BCU(upload(b, (void*)B.fo_off, cnt.data(), cnt.size() * sizeof(int)));
+  BCU(upload(b, B.ii, ii, R * sizeof(int)));
+  BCU(upload(b, B.di, di, R * sizeof(int)));
   B.fo_row = fo_row;
   B.fo_di = fo_di;
   b->members_changed = true;
@@ -1305,8 +1312,8 @@ int bcpnn_batch_upload_stimuli_idx(bcpnn_batch* b, int32_t member, int32_t n_lgi
   int rc;
   if ((rc = balloc(b, &lg, (size_t)n_lgidx_rows * B.H)) || (rc = balloc(b, &wm, (size_t)n_wmask_rows * B.H)))
     return rc;
-  BCU(cudaMemcpy(lg, lgidx_rows, (size_t)n_lgidx_rows * B.H * sizeof(int32_t), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy(wm, wmask_rows, (size_t)n_wmask_rows * B.H * sizeof(float), cudaMemcpyHostToDevice));
+  BCU(upload(b, lg, lgidx_rows, (size_t)n_lgidx_rows * B.H * sizeof(int32_t)));
+  BCU(upload(b, wm, wmask_rows, (size_t)n_wmask_rows * B.H * sizeof(float)));
   B.lgidx = lg;
   B.wmask = wm;
   b->members_changed = true;
@@ -1677,7 +1684,8 @@ int bcpnn_batch_phase_probe(bcpnn_batch* b, uint64_t* out, int32_t max_ctas, int
   if (max_ctas > 0) BCU(cudaMemcpyFromSymbol(out, g_phase_probe, (size_t)std::min(n, (int)max_ctas) * kProbeSlots * 8));
   if (reset) {
     static const uint64_t zeros[kProbeCtas * kProbeSlots] = {};
-    BCU(cudaMemcpyToSymbol(g_phase_probe, zeros, sizeof(zeros)));
+    BCU(cudaMemcpyToSymbolAsync(g_phase_probe, zeros, sizeof(zeros), 0, cudaMemcpyHostToDevice, b->stream));
+    BCU(cudaStreamSynchronize(b->stream));
   }
   return BCPNN_OK;
 #else

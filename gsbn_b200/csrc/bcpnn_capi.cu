@@ -328,6 +328,16 @@ int dzero(bcpnn_net* net, void* p, size_t bytes) {
   return BCPNN_OK;
 }
 
+/* a copy to the device, on the network's stream and complete on return.  Not
+   cudaMemcpy: that one runs on the legacy stream, which the network's
+   non-blocking stream does not wait for, and with pageable memory returns
+   before its last part has reached the device -- a kernel launched next could
+   read what was there before. */
+cudaError_t upload(bcpnn_net* net, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, net->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(net->stream) : e;
+}
+
 uint32_t f32_bits(float v) {
   uint32_t u;
   std::memcpy(&u, &v, 4);
@@ -385,8 +395,8 @@ int make_fills(bcpnn_net* net) {
       at.push_back(make_uint2((unsigned int)k, (unsigned int)(o / kFillBlock)));
   int rc;
   if ((rc = dalloc(net, &net->d_fills, segs.size())) || (rc = dalloc(net, &net->d_fill_at, at.size()))) return rc;
-  CU(cudaMemcpy(net->d_fills, segs.data(), segs.size() * sizeof(FillSeg), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(net->d_fill_at, at.data(), at.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  CU(upload(net, net->d_fills, segs.data(), segs.size() * sizeof(FillSeg)));
+  CU(upload(net, net->d_fill_at, at.data(), at.size() * sizeof(uint2)));
   net->fill_blocks = (unsigned int)at.size();
   return BCPNN_OK;
 }
@@ -1003,7 +1013,7 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
     }
     int* dl = nullptr;
     if ((rc = dalloc(net, &dl, std::max<size_t>(1, all.size())))) return bail(rc);
-    if (!all.empty() && cudaMemcpy(dl, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (!all.empty() && upload(net, dl, all.data(), all.size() * sizeof(int)) != cudaSuccess) {
       net->err = "copy of projection lists failed";
       return bail(BCPNN_ERR_CUDA);
     }
@@ -1071,8 +1081,8 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
     int* dh = nullptr;
     if ((rc = dalloc(net, &dp, cp.size()))) return bail(rc);
     if ((rc = dalloc(net, &dh, ch.size()))) return bail(rc);
-    if (cudaMemcpy(dp, cp.data(), cp.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dh, ch.data(), ch.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload(net, dp, cp.data(), cp.size() * sizeof(int)) != cudaSuccess ||
+        upload(net, dh, ch.data(), ch.size() * sizeof(int)) != cudaSuccess) {
       net->err = "copy of CTA map failed";
       return bail(BCPNN_ERR_CUDA);
     }
@@ -1088,10 +1098,10 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
   H.projs = net->d_projs;
   net->rp.tabs = net->d_tabs;
   net->rp.tabs_old = net->d_tabs + net->tabs.size();
-  if (cudaMemcpy(net->d_pops, net->hp.data(), net->hp.size() * sizeof(PopDev), cudaMemcpyHostToDevice) != cudaSuccess ||
+  if (upload(net, net->d_pops, net->hp.data(), net->hp.size() * sizeof(PopDev)) != cudaSuccess ||
       (!net->hq.empty() &&
-       cudaMemcpy(net->d_projs, net->hq.data(), net->hq.size() * sizeof(ProjDev), cudaMemcpyHostToDevice) != cudaSuccess) ||
-      cudaMemcpy(net->d_net, &net->h, sizeof(NetDev), cudaMemcpyHostToDevice) != cudaSuccess) {
+       upload(net, net->d_projs, net->hq.data(), net->hq.size() * sizeof(ProjDev)) != cudaSuccess) ||
+      upload(net, net->d_net, &net->h, sizeof(NetDev)) != cudaSuccess) {
     net->err = "copy of network descriptor failed";
     return bail(BCPNN_ERR_CUDA);
   }
@@ -1222,7 +1232,7 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
       if ((rc = dalloc(net, &net->col_ring, 2 * (size_t)cap))) return bail(rc);
       H.col_ring = net->col_ring;
       H.col_cap = (int)cap;
-      if (cudaMemcpy(net->d_net, &net->h, sizeof(NetDev), cudaMemcpyHostToDevice) != cudaSuccess) {
+      if (upload(net, net->d_net, &net->h, sizeof(NetDev)) != cudaSuccess) {
         net->err = "copy of network descriptor failed";
         return bail(BCPNN_ERR_CUDA);
       }
@@ -1309,8 +1319,8 @@ int bcpnn_upload_stimuli(bcpnn_net* net, int32_t n_lginp_rows, const float* lgin
   size_t nl = (size_t)n_lginp_rows * net->total_mcu, nw = (size_t)n_wmask_rows * net->total_hcu;
   CU(cudaMalloc((void**)&net->stim_lg, nl * sizeof(float)));
   CU(cudaMalloc((void**)&net->stim_wm, nw * sizeof(float)));
-  CU(cudaMemcpy(net->stim_lg, lginp_rows, nl * sizeof(float), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(net->stim_wm, wmask_rows, nw * sizeof(float), cudaMemcpyHostToDevice));
+  CU(upload(net, net->stim_lg, lginp_rows, nl * sizeof(float)));
+  CU(upload(net, net->stim_wm, wmask_rows, nw * sizeof(float)));
   net->stim_lg_rows = net->stim_lg_cap = n_lginp_rows;
   net->stim_wm_rows = net->stim_wm_cap = n_wmask_rows;
   net->cur_lg = net->h.lginp;
@@ -1534,8 +1544,8 @@ int bcpnn_set_ext_spikes(bcpnn_net* net, int32_t pop, int32_t n, const int32_t* 
   P.ext_idx = nullptr;
   CU(cudaMalloc((void**)&P.ext_off, off.size() * sizeof(int)));
   CU(cudaMalloc((void**)&P.ext_idx, std::max<size_t>(1, flat.size()) * sizeof(int)));
-  CU(cudaMemcpy(P.ext_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
-  if (!flat.empty()) CU(cudaMemcpy(P.ext_idx, flat.data(), flat.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CU(upload(net, P.ext_off, off.data(), off.size() * sizeof(int)));
+  if (!flat.empty()) CU(upload(net, P.ext_idx, flat.data(), flat.size() * sizeof(int)));
   net->allocs.push_back(P.ext_off);
   net->allocs.push_back(P.ext_idx);
   PopDev& D = net->hp[pop];
@@ -1544,7 +1554,7 @@ int bcpnn_set_ext_spikes(bcpnn_net* net, int32_t pop, int32_t n, const int32_t* 
   D.ext_idx = P.ext_idx;
   D.ext_t0 = t0;
   D.ext_t1 = t1;
-  CU(cudaMemcpy(net->d_pops + pop, &D, sizeof(PopDev), cudaMemcpyHostToDevice));
+  CU(upload(net, net->d_pops + pop, &D, sizeof(PopDev)));
   return BCPNN_OK;
 }
 
@@ -1556,7 +1566,7 @@ int bcpnn_set_pop_rng(bcpnn_net* net, int32_t pop, uint32_t seed, uint32_t key_p
   PopDev& D = net->hp[pop];
   D.rng_seed = seed;
   D.rng_pop = key_pop;
-  CU(cudaMemcpy(net->d_pops + pop, &D, sizeof(PopDev), cudaMemcpyHostToDevice));
+  CU(upload(net, net->d_pops + pop, &D, sizeof(PopDev)));
   return BCPNN_OK;
 }
 
@@ -2013,7 +2023,8 @@ int bcpnn_phase_probe(bcpnn_net* net, uint64_t* out, int32_t max_ctas, int32_t* 
   }
   if (reset) {
     static const uint64_t zeros[kProbeCtas * kProbeSlots] = {};
-    CU(cudaMemcpyToSymbol(g_phase_probe, zeros, sizeof(zeros)));
+    CU(cudaMemcpyToSymbolAsync(g_phase_probe, zeros, sizeof(zeros), 0, cudaMemcpyHostToDevice, net->stream));
+    CU(cudaStreamSynchronize(net->stream));
   }
   return BCPNN_OK;
 #else

@@ -1236,6 +1236,13 @@ int dalloc(bcpnn_recall* r, T** p, size_t count) {
   return BCPNN_OK;
 }
 
+/* a copy to the device, on the handle's stream and complete on return (not
+   cudaMemcpy: its stream is not ordered with the handle's) */
+cudaError_t upload(bcpnn_recall* r, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, r->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(r->stream) : e;
+}
+
 uint16_t to_bf16(float f) {
   uint32_t u;
   std::memcpy(&u, &f, 4);
@@ -1307,7 +1314,8 @@ int bcpnn_recall_create(const bcpnn_recall_desc* d, bcpnn_recall** out) {
   if (!rc) rc = dalloc(r, &r->wmask, (size_t)R * H);
   if (!rc) rc = dalloc(r, &r->err, 4);
   if (rc) return bad(rc);
-  if (cudaMemset(r->err, 0, 4 * sizeof(int)) != cudaSuccess || cudaMemset(r->counts, 0, RN) != cudaSuccess)
+  if (cudaMemsetAsync(r->err, 0, 4 * sizeof(int), r->stream) != cudaSuccess ||
+      cudaMemsetAsync(r->counts, 0, RN, r->stream) != cudaSuccess)
     return bad(BCPNN_ERR_CUDA);
   if (!fp32) {
     for (int i = 0; i < 4 && !rc; i++) rc = encode_map(r, &r->map_s[i], r->s[i], R, (int)N, kTileM);
@@ -1358,7 +1366,7 @@ int bcpnn_recall_load(bcpnn_recall* r, const float* w, const float* bj, const fl
   RCU(cudaSetDevice(r->d.device));
   if (r->wf) {
     /* FP32 contraction: W as given, [source][destination] */
-    RCU(cudaMemcpy(r->wf, w, (size_t)N * N * 4, cudaMemcpyHostToDevice));
+    RCU(upload(r, r->wf, w, (size_t)N * N * 4));
     int* flag = r->err + 2;
     int bad = 0;
     RCU(cudaMemsetAsync(flag, 0, sizeof(int), r->stream));
@@ -1373,9 +1381,9 @@ int bcpnn_recall_load(bcpnn_recall* r, const float* w, const float* bj, const fl
     std::vector<uint16_t> wt((size_t)N * N);
     for (int i = 0; i < N; i++)
       for (int j = 0; j < N; j++) wt[(size_t)j * N + i] = to_bf16(w[(size_t)i * N + j]);
-    RCU(cudaMemcpy(r->wt, wt.data(), wt.size() * 2, cudaMemcpyHostToDevice));
+    RCU(upload(r, r->wt, wt.data(), wt.size() * 2));
   }
-  RCU(cudaMemcpy(r->bj, bj, (size_t)N * 4, cudaMemcpyHostToDevice));
+  RCU(upload(r, r->bj, bj, (size_t)N * 4));
   float* row_f = nullptr;
   int8_t* row_s = nullptr;
   RCU(cudaMalloc((void**)&row_f, (size_t)N * 4));
@@ -1386,19 +1394,19 @@ int bcpnn_recall_load(bcpnn_recall* r, const float* w, const float* bj, const fl
   }
   r->kk = 0;
   const int prev = 1; /* parity buffer read by the next tick (kk = 0) */
-  e = cudaMemcpy(row_f, epsc, (size_t)N * 4, cudaMemcpyHostToDevice);
+  e = upload(r, row_f, epsc, (size_t)N * 4);
   if (e == cudaSuccess) {
     broadcast_f32_kernel<<<592, 256, 0, r->stream>>>(r->epsc[prev], R, N, row_f);
     e = cudaStreamSynchronize(r->stream);
   }
-  if (e == cudaSuccess) e = cudaMemcpy(row_f, dsup, (size_t)N * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(r, row_f, dsup, (size_t)N * 4);
   if (e == cudaSuccess) {
     broadcast_f32_kernel<<<592, 256, 0, r->stream>>>(r->dsup[prev], R, N, row_f);
     e = cudaStreamSynchronize(r->stream);
   }
-  if (e == cudaSuccess) e = cudaMemcpy(row_s, spikes_tm3, (size_t)N, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(row_s + N, spikes_tm2, (size_t)N, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(row_s + 2 * N, spikes_tm1, (size_t)N, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(r, row_s, spikes_tm3, (size_t)N);
+  if (e == cudaSuccess) e = upload(r, row_s + N, spikes_tm2, (size_t)N);
+  if (e == cudaSuccess) e = upload(r, row_s + 2 * N, spikes_tm1, (size_t)N);
   if (e == cudaSuccess) {
     for (int k = 0; k < 3; k++) {
       if (r->wf)
