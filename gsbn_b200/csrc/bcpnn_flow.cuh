@@ -250,7 +250,7 @@ __device__ __forceinline__ Block block(float* sm, const Layout& L, int k, int M,
 }
 
 constexpr int kBarP = 1, kBarW = 2, kBarQ = 3;
-/* delay byte: delay in bits 0-4; bit 5: the source population is not published, and bits 6 and 7 are its constant flags
+/* delay byte: delay (1-31, or 0 for 32) in bits 0-4; bit 5: the source population is not published, and bits 6 and 7 are its constant flags
    by tick parity; else bit 6 is the source's spike before the launch */
 constexpr int kUnfed = 32;
 
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
   /* ---- load the state the previous tick left ---- */
   const int cur0 = rp->k0 & 1, prev0 = cur0 ^ 1;
   const float prn = rp->prn;
-  const uint32_t none = (uint32_t)fa.n_words << 5; /* the source of an empty slot: a word that is always 0 */
+  const uint32_t none = (uint32_t)fa.n_words << 5; /* the source of an empty slot: a word that is always 0; none | 1: of a slot that no spike reaches */
   if (tid == 0) s_bits[fa.n_words] = 0u;
 #pragma unroll 1
   for (int k = 0; k < n_in; ++k) {
@@ -375,10 +375,15 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       if (ii >= 0 && ii < J.Ns) {
         qi = (uint32_t)J.qi[r];
         const int hs = ii / s_srcM[k], ms = ii - hs * s_srcM[k];
-        src = (uint32_t)(s_src0[k] + hs * ((s_srcM[k] + 31) >> 5) + (ms >> 5)) << 5 | (uint32_t)(ms & 31);
-        di = (uint32_t)J.di[r] & 31u;
-        if (s_fed[k]) di |= J.si[0][(size_t)((rp->k0 + fa.si_mask) & fa.si_mask) * J.Ns + ii] > 0 ? 64u : 0u;
-        else di |= kUnfed | (J.si[0][ii] > 0 ? 64u : 0u) | (J.si[1][ii] > 0 ? 128u : 0u);
+        const int delay = J.di[r];
+        if (delay >= 1 && delay <= 32) {
+          src = (uint32_t)(s_src0[k] + hs * ((s_srcM[k] + 31) >> 5) + (ms >> 5)) << 5 | (uint32_t)(ms & 31);
+          di = (uint32_t)delay & 31u;
+          if (s_fed[k]) di |= J.si[0][(size_t)((rp->k0 + fa.si_mask) & fa.si_mask) * J.Ns + ii] > 0 ? 64u : 0u;
+          else di |= kUnfed | (J.si[0][ii] > 0 ? 64u : 0u) | (J.si[1][ii] > 0 ? 128u : 0u);
+        } else { /* written into the state: bit delay - 1 is none of the word's, no spike arrives */
+          src = none | 1u;
+        }
       }
       B.src[s] = (uint16_t)src;
       B.di[s] = (uint8_t)di;
