@@ -127,7 +127,7 @@ inline cudaError_t to_host(void* dst, const void* src, size_t bytes, cudaStream_
   Shared& s = shared();
   std::unique_lock<std::mutex> use(s.use, std::try_to_lock);
   if (!use.owns_lock() || !chunks_ready(s)) return plain(dst, src, bytes, stream);
-  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr}; /* of the chunks, and of the work queued before */
   for (cudaEvent_t& x : ev)
     if (cudaEventCreateWithFlags(&x, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
@@ -160,8 +160,11 @@ inline cudaError_t to_host(void* dst, const void* src, size_t bytes, cudaStream_
       piece(k, p);
     }
   };
-  cudaError_t e = post(0);
+  cudaError_t e = cudaEventRecord(ev[2], stream);
+  if (e == cudaSuccess) e = post(0);
   if (e == cudaSuccess && n > 1) e = post(1);
+  /* the work queued before may take long: the others start after it, and spin for a chunk's copy at most */
+  if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);
   std::vector<std::thread> team;
   const int want = (int)std::min(bytes < kLarge ? 2u : 6u, std::max(1u, std::thread::hardware_concurrency()));
   try {

@@ -1,0 +1,50 @@
+/* host_copy.h on the host, over fake_cuda/cuda_runtime.h: `host_copy_check
+   <check>` prints what failed and returns the number of failures. */
+#include "host_copy.h"
+
+#include <cstdio>
+#include <ctime>
+#include <string>
+
+static int failed = 0;
+
+#define CHECK(x)                                         \
+  do {                                                   \
+    if (!(x)) {                                          \
+      std::printf("line %d: %s\n", __LINE__, #x);        \
+      failed++;                                          \
+    }                                                    \
+  } while (0)
+
+static const size_t MB = (size_t)1 << 20;
+
+/* a read of n bytes gives them */
+static void read(size_t n) {
+  std::vector<uint8_t> src(n), dst(n);
+  for (size_t i = 0; i < n; i += 997) src[i] = (uint8_t)(i / 997);
+  src[n - 1] = 77;
+  CHECK(host_copy::to_host(dst.data(), src.data(), n, 0) == cudaSuccess);
+  CHECK(src == dst);
+}
+
+/* a read queued behind half a second of work: no thread works meanwhile */
+static void waiting() {
+  host_copy::Users u;
+  read(40 * MB);
+  std::vector<uint8_t> src(40 * MB, 1), dst(40 * MB);
+  fake::busy_until = fake::clock::now() + std::chrono::milliseconds(500);
+  const std::clock_t c0 = std::clock(); /* of all threads */
+  host_copy::to_host(dst.data(), src.data(), src.size(), 0);
+  const double cpu = (double)(std::clock() - c0) / CLOCKS_PER_SEC;
+  CHECK(fake::clock::now() >= fake::busy_until);
+  CHECK(src == dst);
+  std::printf("%.3f s of CPU time\n", cpu);
+  CHECK(cpu < 0.25);
+}
+
+int main(int argc, char** argv) {
+  const std::string check = argc > 1 ? argv[1] : "";
+  if (check == "waiting") waiting();
+  else failed = 100;
+  return failed;
+}
