@@ -6,9 +6,9 @@
  * into page-locked memory.  Large reads go through two page-locked chunks
  * instead: while one is filled, a few threads copy the other out, which also
  * spreads the first touch of the destination's pages.  The chunks are shared
- * by the process, allocated at the first large read and freed with the last
- * handle (Users); a second reader at the same time, or one without memory for
- * them, takes the plain copy.
+ * by the process, allocated by a read that is worth it (kOwn) and freed with the
+ * last handle (Users); a second reader at the same time, or one without memory
+ * for them, takes the plain copy.
  */
 #ifndef GSBN_HOST_COPY_H
 #define GSBN_HOST_COPY_H
@@ -27,19 +27,28 @@
 
 namespace host_copy {
 
-/* Into fresh numpy arrays on a 16-core host, plain / this way: 4 MB 0.6 / 0.7
-   ms, 8 MB 1.2 / 0.9, 17 MB 2.3 / 1.45 (two threads, chunks of 4 MB), 40 MB 8.8
-   / 2.9 (six threads, chunks of 8 MB; two threads 4.2).  Starting threads and
-   first touches of the same huge page by several of them cost more than they
-   give below. */
+/* Plain / this way, in ms, on a 16-core host: into memory that the process has
+   touched before 6 MB 0.57 / 0.39, 12 MB 1.14 / 0.72, 24 MB 2.2 / 1.1 (two
+   threads, chunks of 4 MB); into fresh pages 32 MB 15 / 3.3, 40 MB 19 / 4.3, 64
+   MB 30 / 6.2 (six threads, chunks of 8 MB).  Starting threads and first touches
+   of the same huge page by several of them cost more than they give below. */
 constexpr size_t kLeast = (size_t)6 << 20, kLarge = (size_t)24 << 20;
 constexpr size_t kChunk = (size_t)8 << 20;
 
+/* Allocating the two chunks takes 6 to 20 ms: as much as one copy of kOwn bytes
+   gains (the first read of 32 MB 15.0 ms with the allocation, 15.1 plain; of 40
+   MB 17.0, 18.8), but ten times what one of 8 MB does (18.7 ms with it, 0.8
+   plain).  So a read of fewer bytes takes the plain copy until such reads have
+   come to kSaved bytes since the chunks were last freed, and have lost by then
+   about what the chunks cost. */
+constexpr size_t kOwn = (size_t)32 << 20, kSaved = (size_t)192 << 20;
+
 struct Shared {
   std::mutex use;   /* held during a copy */
-  std::mutex count; /* users, allocation */
+  std::mutex count; /* everything below */
   int users = 0;
   void* chunk[2] = {nullptr, nullptr};
+  size_t plain_bytes = 0;   /* large reads by the plain copy since the chunks were last freed */
   std::vector<void*> small; /* free small buffers */
 };
 
@@ -62,6 +71,7 @@ struct Users {
         if (c) cudaFreeHost(c);
         c = nullptr;
       }
+      s.plain_bytes = 0;
       for (void* p : s.small) cudaFreeHost(p);
       s.small.clear();
     }
@@ -102,8 +112,13 @@ inline void give_small(void* p) {
   cudaFreeHost(p);
 }
 
-inline bool chunks_ready(Shared& s) {
+/* the chunks, for a read of `bytes`: there, or worth allocating for it */
+inline bool chunks_ready(Shared& s, size_t bytes) {
   std::lock_guard<std::mutex> l(s.count);
+  if (!(s.chunk[0] && s.chunk[1]) && bytes < kOwn) {
+    s.plain_bytes += bytes;
+    if (s.plain_bytes <= kSaved) return false;
+  }
   for (void*& c : s.chunk)
     if (!c && cudaHostAlloc(&c, kChunk, cudaHostAllocPortable) != cudaSuccess) {
       c = nullptr;
@@ -126,7 +141,7 @@ inline cudaError_t to_host(void* dst, const void* src, size_t bytes, cudaStream_
   else if (at.type != cudaMemoryTypeUnregistered) return plain(dst, src, bytes, stream);
   Shared& s = shared();
   std::unique_lock<std::mutex> use(s.use, std::try_to_lock);
-  if (!use.owns_lock() || !chunks_ready(s)) return plain(dst, src, bytes, stream);
+  if (!use.owns_lock() || !chunks_ready(s, bytes)) return plain(dst, src, bytes, stream);
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr}; /* of the chunks, and of the work queued before */
   for (cudaEvent_t& x : ev)
     if (cudaEventCreateWithFlags(&x, cudaEventDisableTiming) != cudaSuccess) {

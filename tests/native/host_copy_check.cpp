@@ -42,9 +42,45 @@ static void waiting() {
   CHECK(cpu < 0.25);
 }
 
+/* the chunks are allocated by a read that gains what they cost, or after as
+   many smaller ones as together would have, and go with the last handle */
+static void chunks() {
+  for (int round = 0; round < 2; ++round) {
+    host_copy::Users u;
+    const int a0 = fake::allocs, f0 = fake::frees;
+    for (int k = 0; k < 24; ++k) read(8 * MB); /* 192 MB */
+    read(5 * MB);                              /* not a large read */
+    CHECK(fake::allocs == a0);
+    read(8 * MB);
+    CHECK(fake::allocs == a0 + 2);
+    read(8 * MB);
+    read(40 * MB);
+    CHECK(fake::allocs == a0 + 2);
+    CHECK(fake::frees == f0);
+  }
+  CHECK(fake::locked.empty());
+  {
+    host_copy::Users u;
+    const int a0 = fake::allocs;
+    read(31 * MB);
+    CHECK(fake::allocs == a0);
+    read(32 * MB);
+    CHECK(fake::allocs == a0 + 2);
+  }
+  CHECK(fake::locked.empty());
+  host_copy::Users u;
+  fake::refuse = true;
+  read(40 * MB);
+  CHECK(cudaGetLastError() == cudaSuccess);
+  fake::refuse = false;
+  read(40 * MB);
+  CHECK(fake::locked.size() == 2);
+}
+
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "waiting") waiting();
+  else if (check == "chunks") chunks();
   else failed = 100;
   return failed;
 }
