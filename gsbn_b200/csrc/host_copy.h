@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -48,8 +49,9 @@ struct Shared {
   std::mutex count; /* everything below */
   int users = 0;
   void* chunk[2] = {nullptr, nullptr};
-  size_t plain_bytes = 0;   /* large reads by the plain copy since the chunks were last freed */
-  std::vector<void*> small; /* free small buffers */
+  size_t plain_bytes = 0;      /* large reads by the plain copy since the chunks were last freed */
+  std::vector<void*> small;    /* free small buffers */
+  std::vector<void*> pageable; /* small buffers, in use, of ordinary memory */
 };
 
 inline Shared& shared() {
@@ -72,29 +74,55 @@ struct Users {
         c = nullptr;
       }
       s.plain_bytes = 0;
-      for (void* p : s.small) cudaFreeHost(p);
-      s.small.clear();
     }
   }
   Users(const Users&) = delete;
   Users& operator=(const Users&) = delete;
 };
 
-/* a page-locked buffer of kSmall bytes for a handle's small results (an
-   allocation takes about a millisecond, so a few stay for the next handle);
-   null without memory for it */
+/* a buffer of kSmall bytes for a handle's small results, page-locked where there
+   is memory for that.  An allocation takes 1 to 3 ms, which a program that makes
+   one network after the other would pay for each of them: so up to kSmallKept
+   buffers (512 KB) stay for the process's next handles, past the last one.  One
+   that a reset of the device has taken away is not handed out again: it is no
+   longer page-locked or, if its address is another buffer's by now, without the
+   mark it was left with. */
 constexpr size_t kSmall = 65536, kSmallKept = 8;
+
+struct Mark {
+  uint64_t words[2];
+  explicit Mark(const void* p) : words{0x6273676e5f6b6570ull, (uint64_t)(uintptr_t)p * 0x9e3779b97f4a7c15ull} {}
+};
+
+inline bool page_locked(const void* p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+
+inline bool still_ours(const void* p) {
+  const Mark m(p);
+  return page_locked(p) && std::memcmp(p, &m, sizeof(m)) == 0;
+}
 
 inline void* take_small() {
   Shared& s = shared();
   std::lock_guard<std::mutex> l(s.count);
-  if (!s.small.empty()) {
+  while (!s.small.empty()) {
     void* p = s.small.back();
     s.small.pop_back();
-    return p;
+    if (still_ours(p)) return p;
   }
   void* p = nullptr;
-  if (cudaHostAlloc(&p, kSmall, cudaHostAllocPortable) != cudaSuccess) return nullptr;
+  if (cudaHostAlloc(&p, kSmall, cudaHostAllocPortable) == cudaSuccess) return p;
+  cudaGetLastError(); /* ordinary memory serves: the copies into it are staged by the driver */
+  try {
+    s.pageable.reserve(s.pageable.size() + 1);
+  } catch (const std::bad_alloc&) {
+    return nullptr;
+  }
+  if ((p = std::malloc(kSmall))) s.pageable.push_back(p);
   return p;
 }
 
@@ -102,9 +130,18 @@ inline void give_small(void* p) {
   if (!p) return;
   Shared& s = shared();
   std::lock_guard<std::mutex> l(s.count);
+  const auto at = std::find(s.pageable.begin(), s.pageable.end(), p);
+  if (at != s.pageable.end()) {
+    s.pageable.erase(at);
+    std::free(p);
+    return;
+  }
+  if (!page_locked(p)) return; /* gone with a reset of the device */
   if (s.small.size() < kSmallKept) {
     try {
       s.small.push_back(p);
+      const Mark m(p);
+      std::memcpy(p, &m, sizeof(m));
       return;
     } catch (const std::bad_alloc&) {
     }

@@ -77,10 +77,53 @@ static void chunks() {
   CHECK(fake::locked.size() == 2);
 }
 
+/* small buffers: of a handle that is gone for the next one, a few of them; not
+   what a reset of the device took away; of ordinary memory without any other */
+static void small() {
+  void* p;
+  {
+    host_copy::Users u;
+    p = host_copy::take_small();
+    host_copy::give_small(p);
+  }
+  CHECK(fake::allocs == 1 && fake::frees == 0);
+  {
+    host_copy::Users u;
+    CHECK(host_copy::take_small() == p);
+    host_copy::give_small(p);
+    std::vector<void*> many;
+    for (int k = 0; k < 20; ++k) many.push_back(host_copy::take_small());
+    CHECK(fake::allocs == 20);
+    for (void* x : many) host_copy::give_small(x);
+  }
+  CHECK(fake::locked.size() == 8 && fake::frees == 12);
+  fake::locked.clear(); /* cudaDeviceReset, and another buffer where one of them was */
+  fake::locked.insert(p);
+  std::memset(p, 0, host_copy::kSmall);
+  host_copy::Users u;
+  p = host_copy::take_small();
+  CHECK(fake::allocs == 21 && fake::locked.size() == 2);
+  fake::refuse = true;
+  void* q = host_copy::take_small();
+  CHECK(q != nullptr && q != p && fake::locked.count(q) == 0);
+  if (q) std::memset(q, 1, host_copy::kSmall);
+  CHECK(cudaGetLastError() == cudaSuccess);
+  host_copy::give_small(q);
+  host_copy::give_small(p);
+  fake::refuse = false;
+  CHECK(host_copy::take_small() == p);
+  host_copy::give_small(p);
+  host_copy::give_small(nullptr);
+  static const int gone[4] = {0};
+  host_copy::give_small(const_cast<int*>(gone)); /* of a reset while the handle lived: not written to */
+  CHECK(cudaGetLastError() == cudaSuccess);
+}
+
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "waiting") waiting();
   else if (check == "chunks") chunks();
+  else if (check == "small") small();
   else failed = 100;
   return failed;
 }

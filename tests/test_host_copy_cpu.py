@@ -7,7 +7,7 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "gsbn_b200", "csrc")
-CHECKS = ["waiting", "chunks"]
+CHECKS = ["waiting", "chunks", "small"]
 
 
 @pytest.fixture(scope="module")
