@@ -24,7 +24,7 @@ EXPORTS = (
     "bcpnn_run", "bcpnn_sync", "bcpnn_spike_log_words", "bcpnn_get_spike_log", "bcpnn_get_spike_log_async", "bcpnn_check_count",
     "bcpnn_check_result_async", "bcpnn_get_ss_flags",
     "bcpnn_state_info", "bcpnn_read_state", "bcpnn_write_state", "bcpnn_read_state_noalloc", "bcpnn_counters", "bcpnn_kernel_launches",
-    "bcpnn_selftest_barrier_timeout", "bcpnn_selftest_division", "bcpnn_phase_probe", "bcpnn_set_pop_rng", "bcpnn_prune",
+    "bcpnn_selftest_barrier_timeout", "bcpnn_selftest_flow_timeout", "bcpnn_selftest_division", "bcpnn_phase_probe", "bcpnn_set_pop_rng", "bcpnn_prune",
     "bcpnn_last_error",
     "bcpnn_status_string",
 )
@@ -101,6 +101,7 @@ def load():
         "bcpnn_counters": (ctypes.c_int, [vp, P(ctypes.c_uint64)]),
         "bcpnn_kernel_launches": (ctypes.c_int, [vp, P(ctypes.c_uint64)]),
         "bcpnn_selftest_barrier_timeout": (ctypes.c_int, [vp, ctypes.c_int64]),
+        "bcpnn_selftest_flow_timeout": (ctypes.c_int, [vp, ctypes.c_int64]),
         "bcpnn_selftest_division": (ctypes.c_int, [vp, ctypes.c_uint64, ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64),
                                                    ctypes.POINTER(ctypes.c_uint64)]),
         "bcpnn_set_pop_rng": (ctypes.c_int, [vp, i32, ctypes.c_uint32, ctypes.c_uint32]),
@@ -322,6 +323,11 @@ class Net:
     def selftest_barrier_timeout(self, limit_ns):
         """status of the barrier self-test (BCPNN_ERR_DEVICE = -6 expected)"""
         return self._lib.bcpnn_selftest_barrier_timeout(self._h, int(limit_ns)), \
+            self._lib.bcpnn_last_error(self._h).decode()
+
+    def selftest_flow_timeout(self, limit_ns):
+        """status of the dataflow kernel's wait self-test (BCPNN_ERR_DEVICE = -6 expected); reset() afterwards"""
+        return self._lib.bcpnn_selftest_flow_timeout(self._h, int(limit_ns)), \
             self._lib.bcpnn_last_error(self._h).decode()
 
     def kernel_launches(self):

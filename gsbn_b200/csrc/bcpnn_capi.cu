@@ -212,7 +212,7 @@ int device_error(bcpnn_net* net, int e) {
     CU(cudaMemsetAsync(net->h.err, 0, sizeof(int), net->stream));
     std::string why;
     if (e & kErrIndex) why += " a slot's source MCU index is outside the source population;";
-    if (e & kErrBarrier) why += " a grid barrier of the persistent tick kernel timed out;";
+    if (e & kErrBarrier) why += " a grid barrier or another wait of the persistent tick kernel timed out;";
     if (e & kErrColumns) why += " a wait for the grid's column updates in the persistent tick kernel timed out;";
     if (e & kErrSeed) why += " a softmax seed published for the next tick carried the wrong tick tag;";
     return fail(net, BCPNN_ERR_DEVICE, "kernel reported error word " + std::to_string(e) + ":" + why);
@@ -647,6 +647,7 @@ int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
       smem = std::max(smem, flow::smem_bytes(P.M, (int)P.in_proj.size(), C, n_words, f.threads, f.queue_warps, net->multi));
     }
     if (smem + 8192 > smem_max) return BCPNN_OK;
+    smem += 16; /* the self-test's further word */
     static std::mutex mu;
     static size_t raised[2][sizeof(kFlowForms) / sizeof(kFlowForms[0])][kMaxDevices] = {{{0}}};
     const void* const fn = f.fn[net->multi];
@@ -667,7 +668,7 @@ int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
     int rc;
     int* d_word0 = nullptr;
     unsigned long long *words = nullptr, *seeds = nullptr;
-    const size_t nw = (size_t)flow::kWordTicks * n_words, ns = (size_t)flow::kSeedTicks * net->pops.size();
+    const size_t nw = (size_t)flow::kWordTicks * (n_words + 1), ns = (size_t)flow::kSeedTicks * net->pops.size();
     if ((rc = dalloc(net, &d_word0, word0.size())) || (rc = dalloc(net, &words, nw)) || (rc = dalloc(net, &seeds, ns)))
       return rc;
     CU(cudaMemcpyAsync(d_word0, word0.data(), word0.size() * sizeof(int), cudaMemcpyHostToDevice, net->stream));
@@ -678,6 +679,7 @@ int setup_flow(bcpnn_net* net, int sms, size_t smem_max) {
     net->flow_args.seeds = seeds;
     net->flow_args.word0 = d_word0;
     net->flow_args.n_words = n_words;
+    net->flow_args.wait_ns = flow::kWaitNs;
     net->flow_args.si_mask = net->multi_persistent && net->multi_resident ? 3 : 1;
     net->flow_smem = smem;
     net->flow_threads = f.threads;
@@ -2032,6 +2034,20 @@ int bcpnn_phase_probe(bcpnn_net* net, uint64_t* out, int32_t max_ctas, int32_t* 
   if (n_ctas) *n_ctas = 0;
   return fail(net, BCPNN_ERR_STATE, "bcpnn_phase_probe: this library was built without BCPNN_PHASE_PROBE");
 #endif
+}
+
+int bcpnn_selftest_flow_timeout(bcpnn_net* net, int64_t limit_ns) {
+  if (!net) return BCPNN_ERR_INVALID;
+  if (limit_ns < 100000 || limit_ns > 2000000000) return fail(net, BCPNN_ERR_INVALID, "bcpnn_selftest_flow_timeout: limit outside [1e5, 2e9] ns");
+  if (!use_flow(net) || net->flow_args.n_words >= flow::kMaxWords || net->max_ticks < 4)
+    return fail(net, BCPNN_ERR_STATE, "bcpnn_selftest_flow_timeout: the network's runs are not the dataflow kernel's");
+  /* a run that waits for one word more than the network publishes: there is room for it in the words and in shared memory */
+  const flow::Args args = net->flow_args;
+  net->flow_args.n_words++;
+  net->flow_args.wait_ns = (unsigned long long)limit_ns;
+  const int rc = bcpnn_run(net, 1, 4, 1.0f, 1.0f);
+  net->flow_args = args;
+  return rc ? rc : bcpnn_sync(net);
 }
 
 int bcpnn_selftest_division(bcpnn_net* net, uint64_t n_pairs, uint64_t seed, uint64_t* tested, uint64_t* mismatches) {

@@ -50,9 +50,12 @@
  * 4.4 -> 4.0 us per tick, 256 x 50 7.4 -> 6.3, 20 x 20 2.6 -> 2.2); and the list
  * of the due rows no longer waits for the other HCUs' spikes.
  *
- * Every wait is bounded (kBarrierNs): it sets kErrBarrier and the CTA's abort
- * flag, the groups leave their tick loops together, and the state is not
- * written back.
+ * Every wait is bounded (Args::wait_ns, kWaitNs but for the self-test): one that
+ * runs out sets kErrBarrier and the CTA's abort flag, the groups of that CTA and,
+ * at their next wait for it, the other CTAs leave their tick loops together.  The
+ * network's state is undefined then, until a reset: such a CTA does not write
+ * back what it keeps in shared memory, but its cells and row traces are in global
+ * memory already, and a CTA that had finished did write.
  */
 #ifndef BCPNN_FLOW_CUH
 #define BCPNN_FLOW_CUH
@@ -72,6 +75,7 @@ struct Args {
   unsigned long long* seeds; /* [n_pops][kSeedTicks]: tag << 32 | float bits */
   const int* word0;          /* [n_pops] first word of a population */
   int n_words;
+  unsigned long long wait_ns; /* limit of every wait */
   int si_mask; /* source-spike buffers by tick & si_mask: 1, or 3 (the block of four of ProcUpdMulti's resident launch) */
 };
 
@@ -109,15 +113,16 @@ __device__ __forceinline__ bool mb_try(unsigned long long* b, uint32_t parity) {
   return ok != 0;
 }
 
-/* wait for the event of tick k >= 0; false when another group gave up, or after kWaitNs */
-__device__ __forceinline__ bool mb_wait(unsigned long long* ev, int k, volatile int* abort_flag, int* err) {
+/* wait for the event of tick k >= 0; false when another group gave up, or after limit_ns */
+__device__ __forceinline__ bool mb_wait(unsigned long long* ev, int k, volatile int* abort_flag, int* err,
+                                        unsigned long long limit_ns) {
   unsigned long long* const b = ev + k % kEventTicks;
   const uint32_t parity = (uint32_t)(k / kEventTicks) & 1u;
   if (mb_try(b, parity)) return true;
   const unsigned long long t0 = now_ns();
   while (!mb_try(b, parity)) {
     if (*abort_flag) return false;
-    if (now_ns() - t0 > kWaitNs) {
+    if (now_ns() - t0 > limit_ns) {
       atomicOr(err, kErrBarrier);
       *abort_flag = 1;
       return false;
@@ -136,18 +141,19 @@ __device__ __forceinline__ void st_word(unsigned long long* p, uint32_t tag, uin
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)tag << 32) | v) : "memory");
 }
 
-/* poll *p for the tag; false when a group or another CTA gave up, or after kWaitNs */
+/* poll *p for the tag; false when a group or another CTA gave up a wait (no other error ends a run: a slot whose
+   index is out of range is left out of it), or after limit_ns */
 __device__ __forceinline__ bool poll_word(const unsigned long long* p, uint32_t tag, uint32_t& v, volatile int* abort_flag,
-                                          int* err) {
+                                          int* err, unsigned long long limit_ns) {
   unsigned long long w = ld_word(p);
   if ((uint32_t)(w >> 32) != tag) {
     const unsigned long long t0 = now_ns();
     do {
-      if (*abort_flag || *(volatile int*)err) {
+      if (*abort_flag || (*(volatile int*)err & kErrBarrier)) {
         *abort_flag = 1;
         return false;
       }
-      if (now_ns() - t0 > kWaitNs) {
+      if (now_ns() - t0 > limit_ns) {
         atomicOr(err, kErrBarrier);
         *abort_flag = 1;
         return false;
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       if (pop.snoise != 0.0f)
         noise = pop.snoise * dev_normal01(pop.rng_seed, pop.rng_pop, (uint32_t)simstep, (uint32_t)idx);
       float sup = pop.lgbias + pop.igain * lg + noise;
-      if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
+      if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err, fa.wait_ns);
       float wsup = 0.0f;
 #pragma unroll 1
       for (int k = 0; k < n_in; ++k) {
@@ -494,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
           seed = d0 + (sp - d0) * pop.taumdt;
         } else if (!bad) {
           uint32_t v = (uint32_t)early;
-          if ((uint32_t)(early >> 32) != tag) bad = !poll_word(slot, tag, v, &s_abort, net->err);
+          if ((uint32_t)(early >> 32) != tag) bad = !poll_word(slot, tag, v, &s_abort, net->err, fa.wait_ns);
           seed = __uint_as_float(v);
         }
       }
@@ -622,8 +628,8 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     for (int it = 0; it < n_ticks; ++it) {
       const int prev = (rp->k0 + it + 1) & 1, nxt = prev;
       /* the lists written below were read by the rows of it - 1 */
-      if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err);
-      if (kMulti && it > 0 && !bad) bad = !mb_wait(s_F, it - 1, &s_abort, net->err);
+      if (it > 0 && !bad) bad = !mb_wait(s_E, it - 1, &s_abort, net->err, fa.wait_ns);
+      if (kMulti && it > 0 && !bad) bad = !mb_wait(s_F, it - 1, &s_abort, net->err, fa.wait_ns);
       if (kQW > 1) bar(kBarQ, kQ);
       else __syncwarp();
       /* the slots due, from plane `it`, a word of 32 per lane; then the planes are one tick further: what was plane 0 is
@@ -685,7 +691,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
             const int x = x0 + y * kQ + qt;
             if (x < fa.n_words) {
               uint32_t b = (uint32_t)v[y];
-              if ((uint32_t)(v[y] >> 32) != tag && !bad) bad = !poll_word(w + x, tag, b, &s_abort, net->err);
+              if ((uint32_t)(v[y] >> 32) != tag && !bad) bad = !poll_word(w + x, tag, b, &s_abort, net->err, fa.wait_ns);
               s_bits[x] = b;
             }
           }
@@ -733,7 +739,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
 #pragma unroll 1
     for (int it = 0; it < n_ticks; ++it) {
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1;
-      if (it > 0) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err);
+      if (it > 0) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err, fa.wait_ns);
       if (__any_sync(0xffffffffu, bad)) break;
       if (kMulti) {
 #pragma unroll 1
@@ -801,7 +807,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
     for (int it = 0; it < n_ticks; ++it) {
       const int simstep = rp->simstep0 + it, cur = (rp->k0 + it) & 1, prev = cur ^ 1;
       if (it > 0) {
-        if (!bad) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err);
+        if (!bad) bad = !mb_wait(s_Lst, it - 1, &s_abort, net->err, fa.wait_ns);
         /* together: a list that is not there is not read.  Also: the columns of it - 1 are in place */
         bad = bar_any(kBarW, kW, bad);
         if (bad) break;
@@ -830,7 +836,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
             if constexpr (kMulti) {
               float4 q = J.cell[index];
               if (!start) {
-                if (!mb_wait(s_O, it, &s_abort, net->err)) bad = true;
+                if (!mb_wait(s_O, it, &s_abort, net->err, fa.wait_ns)) bad = true;
                 start = true;
               }
               int tij = B.ti0[cur * C + e];
@@ -866,7 +872,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
               float w;
               if (kp != 0.0f) {
                 if (!traces) {
-                  if (!mb_wait(s_T, it, &s_abort, net->err)) bad = true;
+                  if (!mb_wait(s_T, it, &s_abort, net->err, fa.wait_ns)) bad = true;
                   traces = true;
                 }
                 w = J.wgain * bx_logf((q.x + J.eps2) / ((B.pi[cur * C + e] + J.eps) * (B.pjn[cur * M + j] + J.eps)));
@@ -892,7 +898,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
               q.z = q.z + J.kfti;
               if (kp != 0.0f) { /* Proj.cpp:458-462 */
                 if (!traces) {
-                  if (!mb_wait(s_T, it, &s_abort, net->err)) bad = true;
+                  if (!mb_wait(s_T, it, &s_abort, net->err, fa.wait_ns)) bad = true;
                   traces = true;
                 }
                 w = J.wgain * bx_logf((q.x + J.eps2) / ((B.pi[cur * C + e] + J.eps) * (B.pjn[cur * M + j] + J.eps)));
@@ -919,7 +925,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
       __syncwarp();
       if (lane == 0) mb_arrive(s_E, it);
       /* columns of this tick's spikes */
-      if (!bad) bad = !mb_wait(s_S, it, &s_abort, net->err);
+      if (!bad) bad = !mb_wait(s_S, it, &s_abort, net->err, fa.wait_ns);
       if (!bad) {
         uint32_t sp[kPW];
         int nspk = 0;

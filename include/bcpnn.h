@@ -299,6 +299,13 @@ int bcpnn_kernel_launches(const bcpnn_net* net, uint64_t* out);
    without bound. */
 int bcpnn_selftest_barrier_timeout(bcpnn_net* net, int64_t limit_ns);
 
+/* The same for the waits of the dataflow kernel: four ticks that wait for one
+   spike word more than the network publishes.  Returns BCPNN_ERR_DEVICE as
+   above; the network's state is undefined until bcpnn_reset.  BCPNN_ERR_STATE
+   when the network's runs are another kernel's (HCUs of more than 128 MCUs,
+   external spikes, one launch per tick). */
+int bcpnn_selftest_flow_timeout(bcpnn_net* net, int64_t limit_ns);
+
 /* Numerics self-test (no counterpart in the reference): the decay closed
    forms divide by a multiplication with a correctly rounded double
    reciprocal, RN_float(a * RN_double(1/b)), and fall back to a warp-uniform
