@@ -214,7 +214,7 @@ __device__ __forceinline__ void decay_cell(float& pij, float& eij, float& zi2, f
   float4 A, Bv;
   if (T) {
     double2 R0, R1;
-    if (pdt < tlen) {
+    if ((unsigned)pdt < (unsigned)tlen) { /* a row written with a later tick decays over a negative number of them */
       A = tab[(size_t)pdt * 4];
       Bv = tab[(size_t)pdt * 4 + 1];
       R0 = T->rtab[(size_t)pdt * 4];
