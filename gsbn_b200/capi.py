@@ -15,6 +15,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("GSBN_B200_LIB") or os.path.join(_HERE, "libgsbn_b200.so")
 
 F32, I32, I8 = 0, 1, 2
+FORMS = ("per tick", "barrier", "dataflow")  # BCPNN_FORM_*
 _NP = {F32: np.float32, I32: np.int32, I8: np.int8}
 
 # every entry point declared in include/bcpnn.h
@@ -23,7 +24,7 @@ EXPORTS = (
     "bcpnn_use_stimulus", "bcpnn_set_stimulus_idx", "bcpnn_upload_stimuli_idx", "bcpnn_upload_stimuli_idx_async", "bcpnn_set_ext_spikes", "bcpnn_reset", "bcpnn_get_stream",
     "bcpnn_run", "bcpnn_sync", "bcpnn_spike_log_words", "bcpnn_get_spike_log", "bcpnn_get_spike_log_async", "bcpnn_check_count",
     "bcpnn_check_result_async", "bcpnn_get_ss_flags",
-    "bcpnn_state_info", "bcpnn_read_state", "bcpnn_write_state", "bcpnn_read_state_noalloc", "bcpnn_counters", "bcpnn_kernel_launches",
+    "bcpnn_state_info", "bcpnn_read_state", "bcpnn_write_state", "bcpnn_read_state_noalloc", "bcpnn_counters", "bcpnn_run_form", "bcpnn_kernel_launches",
     "bcpnn_selftest_barrier_timeout", "bcpnn_selftest_flow_timeout", "bcpnn_selftest_division", "bcpnn_phase_probe", "bcpnn_set_pop_rng", "bcpnn_prune",
     "bcpnn_last_error",
     "bcpnn_status_string",
@@ -99,6 +100,7 @@ def load():
         "bcpnn_write_state": (ctypes.c_int, [vp, ctypes.c_char_p, vp, sz]),
         "bcpnn_read_state_noalloc": (ctypes.c_int, [vp, ctypes.c_char_p, vp, sz]),
         "bcpnn_counters": (ctypes.c_int, [vp, P(ctypes.c_uint64)]),
+        "bcpnn_run_form": (ctypes.c_int, [vp, P(i32), P(i32)]),
         "bcpnn_kernel_launches": (ctypes.c_int, [vp, P(ctypes.c_uint64)]),
         "bcpnn_selftest_barrier_timeout": (ctypes.c_int, [vp, ctypes.c_int64]),
         "bcpnn_selftest_flow_timeout": (ctypes.c_int, [vp, ctypes.c_int64]),
@@ -329,6 +331,12 @@ class Net:
         """status of the dataflow kernel's wait self-test (BCPNN_ERR_DEVICE = -6 expected); reset() afterwards"""
         return self._lib.bcpnn_selftest_flow_timeout(self._h, int(limit_ns)), \
             self._lib.bcpnn_last_error(self._h).decode()
+
+    def run_form(self):
+        """how the next run() advances the network, one of FORMS, and the threads of a CTA"""
+        form, threads = ctypes.c_int32(), ctypes.c_int32()
+        self._check(self._lib.bcpnn_run_form(self._h, ctypes.byref(form), ctypes.byref(threads)))
+        return FORMS[form.value], threads.value
 
     def kernel_launches(self):
         out = ctypes.c_uint64()

@@ -1954,6 +1954,14 @@ int bcpnn_counters(bcpnn_net* net, uint64_t out[3]) {
   return BCPNN_OK;
 }
 
+int bcpnn_run_form(const bcpnn_net* net, int32_t* form, int32_t* threads) {
+  if (!net || !form || !threads) return BCPNN_ERR_INVALID;
+  const bool flow = use_flow(net);
+  *form = flow ? BCPNN_FORM_DATAFLOW : net->persistent || net->multi_persistent ? BCPNN_FORM_BARRIER : BCPNN_FORM_PER_TICK;
+  *threads = flow ? net->flow_threads : net->multi ? multi::kProjThreads : net->threads;
+  return BCPNN_OK;
+}
+
 int bcpnn_kernel_launches(const bcpnn_net* net, uint64_t* out) {
   if (!net || !out) return BCPNN_ERR_INVALID;
   *out = net->launches;

@@ -290,6 +290,15 @@ int bcpnn_counters(bcpnn_net* net, uint64_t out[3]);
 /* Number of kernels this library launched for the network since creation. */
 int bcpnn_kernel_launches(const bcpnn_net* net, uint64_t* out);
 
+/* How the next bcpnn_run advances the network -- the results do not depend on
+   it -- and the threads of a CTA: one launch per tick (and, of ProcUpdMulti,
+   projection); one launch per run with a barrier of the whole grid every tick;
+   or one launch per run whose CTAs wait for each other's spike words alone. */
+#define BCPNN_FORM_PER_TICK 0
+#define BCPNN_FORM_BARRIER 1
+#define BCPNN_FORM_DATAFLOW 2
+int bcpnn_run_form(const bcpnn_net* net, int32_t* form, int32_t* threads);
+
 /* Failure-detection self-test (no counterpart in the reference, whose
    errors all abort): runs the bounded grid-barrier wait of the persistent tick
    kernel on an arrival count that never completes.  Every wait gives up after
