@@ -907,7 +907,10 @@ int bfail(bcpnn_batch* b, int code, const std::string& msg) {
 #define BCU(call)                                                                              \
   do {                                                                                         \
     cudaError_t e_ = (call);                                                                   \
-    if (e_ != cudaSuccess) return bfail(b, BCPNN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                                   \
+      cudaGetLastError(); /* reported once, see CU (bcpnn_capi.cu) */                          \
+      return bfail(b, BCPNN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));     \
+    }                                                                                          \
   } while (0)
 
 template <typename T>

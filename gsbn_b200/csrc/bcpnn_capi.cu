@@ -181,11 +181,15 @@ int fail(bcpnn_net* net, int code, const std::string& msg) {
   return code;
 }
 
+/* a failed call is reported once: the runtime also keeps its error for the next
+   cudaGetLastError, which would fail a later call of this or another handle */
 #define CU(call)                                                                              \
   do {                                                                                        \
     cudaError_t e_ = (call);                                                                  \
-    if (e_ != cudaSuccess)                                                                    \
+    if (e_ != cudaSuccess) {                                                                  \
+      cudaGetLastError();                                                                     \
       return fail(net, BCPNN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));   \
+    }                                                                                         \
   } while (0)
 
 template <typename T>
@@ -857,7 +861,11 @@ int bcpnn_net_create(const bcpnn_net_desc* desc, bcpnn_net** out) {
   std::memset(&net->h, 0, sizeof(NetDev));
   std::memset(&net->rp, 0, sizeof(RunParams));
   int rc = BCPNN_OK;
-  auto bail = [&](int code) { *out = net; return code; };
+  auto bail = [&](int code) {
+    if (code == BCPNN_ERR_CUDA) cudaGetLastError(); /* reported here, see CU */
+    *out = net;
+    return code;
+  };
   if (cudaSetDevice(net->device) != cudaSuccess) { net->err = "cudaSetDevice failed"; return bail(BCPNN_ERR_CUDA); }
   if (cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&net->copy_stream, cudaStreamNonBlocking) != cudaSuccess) {

@@ -1197,8 +1197,10 @@ int fail(bcpnn_recall* r, int code, const std::string& msg) {
 #define RCU(call)                                                                             \
   do {                                                                                        \
     cudaError_t e_ = (call);                                                                  \
-    if (e_ != cudaSuccess)                                                                    \
+    if (e_ != cudaSuccess) {                                                                  \
+      cudaGetLastError(); /* reported once, see CU (bcpnn_capi.cu) */                         \
       return fail(r, BCPNN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));     \
+    }                                                                                         \
   } while (0)
 
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1285,6 +1287,7 @@ int bcpnn_recall_create(const bcpnn_recall_desc* d, bcpnn_recall** out) {
   r->d = *d;
   r->N = (int)N;
   auto bad = [&](int rc) {
+    if (rc == BCPNN_ERR_CUDA) cudaGetLastError(); /* reported here, see CU (bcpnn_capi.cu) */
     bcpnn_recall_destroy(r);
     return rc;
   };
