@@ -79,6 +79,9 @@ struct Params {
   int simstep;
   int poisson;
   float one; /* 1, see add2m */
+  /* maxfqdt in units of 2^-32, rounded up by 2^-20, as the division by an HCU's sum takes it: the quotient maxfqdt / sum
+     of a sum near the largest float is subnormal, and off by more than that margin once times an activity */
+  float bound1;
   uint32_t pr_count; /* a 24-bit uniform k 2^-24 is below pr for k < pr_count */
   int* err;
 };
@@ -372,7 +375,7 @@ __device__ __forceinline__ void recall_pop(const Params& p, int tid) {
       vs = __shfl_sync(0xffffffffu, v, (lane & ~3) | s);
     }
   /* above every product (act / vs) * maxfqdt, in units of 2^-32 */
-  const float bound = (vs > 1.0f ? p.maxfqdt / vs : p.maxfqdt) * (0x1p32f * (1.0f + 0x1p-20f));
+  const float bound = vs > 1.0f ? p.bound1 / vs : p.bound1;
 #pragma unroll
   for (int i = 0; i < G; i++)
     *reinterpret_cast<float4*>(p.dsup_cur + row + c0 + (4 * i + q) * 4) =
@@ -1481,6 +1484,7 @@ int bcpnn_recall_run(bcpnn_recall* r, int32_t first, int32_t n_ticks, int32_t co
   p.pr = d.poisson_noise_hz * d.dt;
   p.poisson = d.poisson_noise_hz > 0.f;
   p.one = 1.0f;
+  p.bound1 = p.maxfqdt * (0x1p32f * (1.0f + 0x1p-20f));
   p.pr_count = !p.poisson ? 0u : p.pr >= 1.0f ? 1u << 24 : (uint32_t)std::ceil((double)p.pr * 0x1p24);
   p.seed_base = d.seed_base;
   p.err = r->err;
