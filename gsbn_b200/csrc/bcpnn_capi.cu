@@ -616,7 +616,19 @@ bool raise_smem(const TickForm& f, bool fp64, int dev, size_t smem) {
    (one MCU per thread), the fewest that hold the network's largest HCU.  Two
    warps of delay queue where a CTA has an SM to itself (100 x 100 with 1000
    slots 3.99 us per tick; with one 4.26, though 10 x 10 2.11 -> 2.08), one where
-   two CTAs share it. */
+   two CTAs share it.
+
+   Taken wherever it fits: us per tick, with tick_kernel of the same CTA size in
+   brackets: 160 x 65 with C = 500 5.4 (11.8), 160 x 128 with C = 1000 9.4
+   (14.4), 296 x 100 with C = 1000 10.8 (16.4), 296 x 128 with C = 400 6.7 (12.6),
+   though four population warps leave two of a 256-thread CTA's to the rows and
+   columns.  A whole column stays on one CTA, and still the largest columns that
+   fit shared memory are faster than spread over the grid, at low rates too: 100 x
+   100 with C = 4000 10.1 (17.0), 8000 20.9 (32.2), 8000 with a tenth of the spikes
+   11.8 (17.8), with a fiftieth 9.1 (15.9).  There is none of 128 threads: 297 to
+   592 HCUs take tick_kernel's, 14.2 us at 297 x 20 with C = 400 against 3.4 at
+   296 x 20.  Its four groups want a warp each and more for the rows, and four
+   such CTAs would have to share an SM; not built, so not measured. */
 struct FlowForm {
   int threads, pop_warps, queue_warps;
   const void* fn[2]; /* ProcUpdLazy, ProcUpdMulti */

@@ -441,14 +441,6 @@ __device__ __forceinline__ void cell_decay(float& pij, float& eij, float& zi2, f
   zj2 = zj2 * B.w;
 }
 
-/* Out-of-line copies for the tick kernel: one body of the closed forms
-   shared by its call sites keeps the kernel's instruction footprint small
-   (each phase runs once per tick, so its code is fetched again every tick). */
-__device__ __noinline__ float4 cell_decay_nl(float4 c, const Coef k, float4 A, float4 B) {
-  cell_decay(c.x, c.y, c.z, c.w, k, A, B);
-  return c;
-}
-
 /* Closed-form decay of the row traces, Proj.cpp:409-415 (row), :241-247
    (all).  A = entry[2], B = entry[3]. */
 __device__ __forceinline__ void row_decay(float& pi, float& ei, float& zi, const Coef& k, float4 A, float4 B) {
@@ -469,11 +461,6 @@ __device__ __forceinline__ void row_decay(float& pi, float& ei, float& zi, const
   pi = pn;
   ei = en;
   zi = zi * B.w;
-}
-
-__device__ __noinline__ float4 row_decay_nl(float4 r, const Coef k, float4 A, float4 B) {
-  row_decay(r.x, r.y, r.z, k, A, B);
-  return r;
 }
 
 /* The closed forms with every division a / b evaluated as
@@ -774,8 +761,9 @@ __global__ void fill_kernel(T* p, size_t n, T v) {
    fill_segments_kernel does many in one launch, block b the kFillBlock bytes
    of segment at[b].x from offset at[b].y * kFillBlock on.  Bound by the writes
    where there are large segments; for small networks the launch, one instead
-   of one per state vector (reset of the 10 x 10 network: 75 -> 10 us, of the
-   100 x 100 network, 240 MB: 131 -> 66 us). */
+   of one per state vector (reset of the 10 x 10 network, the call and the wait
+   for it: 75 -> 31 us, 8.7 of them on the device; of the 100 x 100 network, 240
+   MB: 131 -> 65 us, 42 on the device). */
 struct FillSeg {
   uint4* p;
   unsigned long long bytes;

@@ -492,8 +492,8 @@ struct WMaps {
    blockIdx.x, blockIdx.x + ctas, ... (Tiles).  The stage ring runs on
    across tiles; two TMEM accumulators of 256 columns alternate, so the epilogue
    of one tile overlaps the MMAs of the next (acc_full: MMA -> epilogue,
-   acc_empty: epilogue -> MMA).  The epilogue's loads run one 32-column chunk
-   ahead, the first before its accumulator is there.
+   acc_empty: epilogue -> MMA).  The epilogue loads the epsc of a tile's first 32
+   columns before its accumulator is there.
 
    kPopM: the HCU size, and the CTAs from `ctas` on do the population update of
    the tick, which needs nothing of the contraction's; 0: recall_pop_kernel does
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(j * kTileN + c), acc);
         if (c > 0) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) e[i] = *reinterpret_cast<const float4*>(p.epsc_prev + base + c + 4 * i);
+          for (int i = 0; i < 8; i++) e[i] = *reinterpret_cast<const float4*>(p.epsc_prev + base + c + 4 * i);
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) {

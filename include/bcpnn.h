@@ -100,7 +100,7 @@ typedef struct bcpnn_net_desc {
                                 bit-identical to the reference */
   int32_t update_variant;    /* 0: ProcUpdLazy; 1: ProcUpdMulti (row-only updates
                                 that replay a ring of postsynaptic spikes,
-                                adaptation in the population; per-tick launches) */
+                                adaptation in the population) */
   int32_t spike_buffer_size; /* ProcUpdMulti argi "spike buffer size" (1 .. 1024;
                                 0 means 1) */
 } bcpnn_net_desc;
@@ -138,10 +138,12 @@ int bcpnn_use_stimulus(bcpnn_net* net, int32_t lginp_row, int32_t wmask_row);
 /* The same from ProcExtGen's pattern-index rows (.lgidx, one MCU index per
    HCU; any other value means no input to that HCU): the library computes
    lginp = log(1+eps) on the indexed MCU and log(0+eps) elsewhere
-   (ProcExtGen.cpp:130-144) with its own float log, on the device.  Both
-   rows are copied on the network's stream: a page-locked row is read when
-   the stream reaches the copy, so keep it unchanged until the next
-   bcpnn_sync; a pageable row is staged before the call returns. */
+   (ProcExtGen.cpp:130-144) with its own float log, on the device.  Of a
+   network of at most 448 HCUs bcpnn_set_stimulus_idx takes both rows with
+   the call; of a larger one they are copied on the network's stream: a
+   page-locked row is read when the stream reaches the copy, so keep it
+   unchanged until the next bcpnn_sync; a pageable row is staged before the
+   call returns. */
 int bcpnn_set_stimulus_idx(bcpnn_net* net, const int32_t* lgidx_row, size_t n_hcu, float eps, const float* wmask_row,
                            size_t n_wmask);
 int bcpnn_upload_stimuli_idx(bcpnn_net* net, int32_t n_lgidx_rows, const int32_t* lgidx_rows, float eps,
