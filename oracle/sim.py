@@ -50,11 +50,12 @@ def build():
 
 def reference_root():
     """The gsbn source tree ($GSBN_REFERENCE_ROOT, else oracle/Makefile's
-    REF_ROOT), or None when it is not present."""
+    REF_ROOT), or None when it is not present (an empty folder in its place is
+    not the tree)."""
     r = os.environ.get("GSBN_REFERENCE_ROOT")
     if not r:
         r = subprocess.run(["make", "-s", "-C", HERE, "ref-root"], capture_output=True, text=True).stdout.strip()
-    return r if r and os.path.isdir(r) else None
+    return r if r and os.path.isdir(r) and os.listdir(r) else None
 
 
 def ref_available():
