@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads)
   /* ---- load the state the previous tick left ---- */
   const int cur0 = rp->k0 & 1, prev0 = cur0 ^ 1;
   const float prn = rp->prn;
-  const uint32_t none = (uint32_t)fa.n_words << 5; /* the source of an empty slot: a word that is always 0; none | 1: of a slot that no spike reaches */
+  /* the source of an empty slot: a word that is always 0; none | 1: of a slot that no spike reaches */
+  const uint32_t none = (uint32_t)fa.n_words << 5;
   if (tid == 0) s_bits[fa.n_words] = 0u;
 #pragma unroll 1
   for (int k = 0; k < n_in; ++k) {
